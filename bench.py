@@ -14,9 +14,10 @@ force along x. The headline kernel is the list AA kernel
   e2e       the same metric through the reference-facing C ABI: one Kernel()
             call of the configuration's 500 steps with the PDF field uploaded
             from the pinned host mirror before and downloaded after
-  roofline  the dominant kernel (the odd, adjacency-driven step): algorithmic
-            bytes per launch / mean launch time, against the measured HBM copy
-            bandwidth in MEASURED_PEAKS.json
+  roofline  the dominant kernel (the fused even/odd step pair): the bytes a
+            pair cannot do without (every PDF read and written once, plus the
+            adjacency records) / mean launch time, against the measured HBM
+            copy bandwidth in MEASURED_PEAKS.json
   cpu_baseline  the reference's own list-aa-pv-soa (compiled from its sources
             into oracle/_ref) on this host's cores, a bounded sample of the
             same domain
@@ -297,6 +298,28 @@ def _cpu_ranges(cpus):
         out.append(str(cpus[i]) if i == j else "%d-%d" % (cpus[i], cpus[j]))
         i = j + 1
     return ",".join(out)
+
+
+def list_aa_roofline(t, nodes, pdf_bytes, adj_node, peak, names):
+    """HBM roofline entry of a list AA row from its per-launch times. One
+    launch per pair (fused even and odd step): every PDF has to be read and
+    written once per launch, plus the adjacency records; "streamed" counts both
+    steps' accesses, half of which L2 serves. Two launches: the odd one."""
+    per = t["per_launch_ms"]
+    pair_bytes = 2 * 19 * pdf_bytes + adj_node
+    if t["launches_per_pair"] == 1:
+        ms = statistics.mean(per)
+        achieved = pair_bytes * nodes / (ms / 1e3) / 1e9
+        return {"kernel": names[0], "achieved": round(achieved, 1), "frac": round(achieved / peak, 4),
+                "bytes_per_pair": round(pair_bytes, 2), "bytes_per_flup": round(pair_bytes / 2, 2),
+                "launch_ms": round(ms, 5),
+                "streamed_gbs": round((pair_bytes + 2 * 19 * pdf_bytes) * nodes / (ms / 1e3) / 1e9, 1)}
+    even_ms, odd_ms = statistics.mean(per[0::2]), statistics.mean(per[1::2])
+    achieved = pair_bytes * nodes / (odd_ms / 1e3) / 1e9
+    return {"kernel": names[1], "achieved": round(achieved, 1), "frac": round(achieved / peak, 4),
+            "bytes_per_flup": round(pair_bytes, 2), "launch_ms": round(odd_ms, 5),
+            "even_step": {"bytes_per_flup": 2 * 19 * pdf_bytes, "launch_ms": round(even_ms, 5),
+                          "achieved": round(2 * 19 * pdf_bytes * nodes / (even_ms / 1e3) / 1e9, 1)}}
 
 
 def aa_line(lbmb200, fl, args, kargs, dist, peak):
@@ -653,7 +676,6 @@ def run_ours(args, dist):
     t = time_kernel(lbmb200, "cuda-list-aa-pv-soa", lat, args.steps, max(3, args.warmup), kargs, dist, "odd")
     inst = t["inst"]
     adj_node = adjacency_bytes_per_node(lbmb200, inst, lat.n_fluid)
-    odd_bpf = B_PER_FLUP["even"] + adj_node
     try:
         # e2e: the reference-facing Kernel() call, mirror uploaded and downloaded
         cd = lbmb200.case(omega=1.0, xforce=1e-5, iterations=500)
@@ -674,28 +696,19 @@ def run_ours(args, dist):
     ms = dist.max(t["ms"])
     steps_run = t["steps_run"]
     value = nf_total * steps_run / (ms / 1e3) / 1e6
-    per = t["per_launch_ms"]
-    even = per[0::2]
-    odd = per[1::2]
-    odd_ms = statistics.mean(odd)
-    even_ms = statistics.mean(even)
-    achieved = odd_bpf * lat.n_fluid / (odd_ms / 1e3) / 1e9
-    traffic = profile_traffic("list_odd_fp64")
+    roof = list_aa_roofline(t, lat.n_fluid, 8, adj_node, peak,
+                            ("k_list_pair_fp64 (even and odd step in one launch)",
+                             "k_list_odd_fp64 (adjacency-driven odd step)"))
+    traffic = profile_traffic("list_pair_fp64" if t["launches_per_pair"] == 1 else "list_odd_fp64")
     line = {
         "metric": "MFLUP/s & % HBM roofline at 256^3", "value": round(value, 3), "unit": "MFLUP/s",
         "n_gpus": dist.world, "steps": steps_run, "warmup": max(3, args.warmup),
         "ms_per_step": round(ms / steps_run, 5), "higher_is_better": True, "scaling": "weak",
         "vs_baseline": None, "dtype": "f64", "data": "synthetic",
         "config": headline_config(args, stats, lat, n_cells, dist),
-        "roofline": {"bound": "hbm", "kernel": "k_list_odd_fp64 (adjacency-driven odd step)",
-                     "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
-                     "frac": round(achieved / peak, 4), "peak_kind": peak_kind,
-                     "bytes_per_flup": round(odd_bpf, 2),
+        "roofline": {"bound": "hbm", "peak": peak, "unit": "GB/s", "peak_kind": peak_kind,
                      "adjacency": "run-compressed: %.2f B per node (72 uncompressed)" % adj_node,
-                     "launch_ms": round(odd_ms, 5),
-                     "traffic": traffic,
-                     "even_step": {"bytes_per_flup": B_PER_FLUP["even"], "launch_ms": round(even_ms, 5),
-                                   "achieved": round(B_PER_FLUP["even"] * lat.n_fluid / (even_ms / 1e3) / 1e9, 1)}},
+                     "traffic": traffic, **roof},
         "e2e": {"value": round(nf_total * e2e_iters / e2e_s / 1e6, 3), "unit": "MFLUP/s",
                 "h2d_bytes_per_step": int(round(h2d / e2e_iters)), "d2h_bytes_per_step": int(round(d2h / e2e_iters)),
                 "h2d_bytes_per_call": int(h2d), "d2h_bytes_per_call": int(d2h), "steps_per_call": e2e_iters,
@@ -752,16 +765,11 @@ def run_ours(args, dist):
         for prec, pb in (("fp32", 4), ("fp16", 2)):
             tl = time_kernel(lbmb200, "cuda-list-aa-pv-soa", lat, min(args.steps, 200), 4,
                              kargs + ["-precision", prec], dist, "odd")
-            # mean of the even (38 s) and odd (38 s + adjacency) steps
-            bpf = 2 * 19 * pb + adjacency_bytes_per_node(lbmb200, tl["inst"], lat.n_fluid) / 2
+            adj = adjacency_bytes_per_node(lbmb200, tl["inst"], lat.n_fluid)
             tl["inst"].deinit()
-            m = statistics.mean(tl["per_launch_ms"])
             extra["cuda-list-aa-pv-soa/" + prec] = {
-                "mflups": round(lat.n_fluid / (m / 1e3) / 1e6, 1), "bytes_per_flup": round(bpf, 2),
-                "achieved_gbs": round(bpf * lat.n_fluid / (m / 1e3) / 1e9, 1),
-                "frac": round(bpf * lat.n_fluid / (m / 1e3) / 1e9 / peak, 4),
-                "even_ms": round(statistics.mean(tl["per_launch_ms"][0::2]), 5),
-                "odd_ms": round(statistics.mean(tl["per_launch_ms"][1::2]), 5)}
+                "mflups": round(lat.n_fluid * tl["steps_run"] / (tl["ms"] / 1e3) / 1e6, 1),
+                **list_aa_roofline(tl, lat.n_fluid, pb, adj, peak, ("k_list_pair_lp", "k_list_odd_lp"))}
         line["kernels"] = extra
 
     for name, fn, enabled in (("batched", section_batched, args.batched > 0 and dist.world == 1),

@@ -10,8 +10,10 @@
 //   2. exclusive prefix sum of the flags = the node index of each fluid cell;
 //   3. grid[cell] = node; then, once the grid is complete, each node's 18
 //      adjacency entries from its neighbours' node indices.
+#include <algorithm>
 #include <cstdint>
 #include <cstdio>
+#include <vector>
 
 #include <cub/device/device_scan.cuh>
 
@@ -272,6 +274,95 @@ int list_runs_device(const uint32_t* adj, int nFluid, cudaStream_t s, uint32_t**
     return (int)e;
   }
   return 0;
+}
+
+// --- fused step pairs ----------------------------------------------------------------
+
+// One block of kListTile threads per tile.
+__global__ void k_tile_reach(const uint32_t* __restrict__ adj, int nFluid, uint32_t nCells,
+                             uint32_t* __restrict__ reach) {
+  __shared__ uint32_t lo[3], hi[3];
+  if (threadIdx.x < 3) {
+    lo[threadIdx.x] = 0xffffffffu;
+    hi[threadIdx.x] = 0u;
+  }
+  __syncthreads();
+  const uint32_t n = blockIdx.x * kListTile + threadIdx.x;
+  if (n < static_cast<uint32_t>(nFluid)) {
+    uint32_t l[3] = {0xffffffffu, n, 0xffffffffu}, h[3] = {0u, n, 0u};
+#pragma unroll
+    for (int d = 0; d < QM; ++d) {
+      // the neighbour's slot in plane d, or (bounce back) the node's own in plane inv(d)
+      const uint32_t a = adj[(size_t)n * QM + d];
+      const uint32_t m = a == static_cast<uint32_t>(inv(d)) * nCells + n ? n : a - static_cast<uint32_t>(d) * nCells;
+      const int c = cx(d) + 1;
+      l[c] = min(l[c], m);
+      h[c] = max(h[c], m);
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+      if (l[c] <= h[c]) {
+        atomicMin(&lo[c], l[c] / kListTile);
+        atomicMax(&hi[c], h[c] / kListTile);
+      }
+  }
+  __syncthreads();
+  if (threadIdx.x < 3) {
+    reach[(size_t)blockIdx.x * 6 + 2 * threadIdx.x] = lo[threadIdx.x];
+    reach[(size_t)blockIdx.x * 6 + 2 * threadIdx.x + 1] = hi[threadIdx.x];
+  }
+}
+
+void list_tile_reach(const uint32_t* adj, int nFluid, long long nCells, uint32_t* reach, cudaStream_t s) {
+  const int nTiles = (nFluid + kListTile - 1) / kListTile;
+  if (nTiles > 0) k_tile_reach<<<nTiles, kListTile, 0, s>>>(adj, nFluid, static_cast<uint32_t>(nCells), reach);
+}
+
+long long pair_schedule(const uint32_t* reach, const uint32_t* runOff, int nTiles, int margin,
+                        std::vector<PairItem>& items) {
+  items.clear();
+  if (nTiles <= 0) return 0;
+  // the odd steps in the order of the last even tile they need (a counting
+  // sort; with the blocked numbering this is nearly the tile order, except
+  // for the first x plane of a periodic lattice, which needs the last one)
+  std::vector<uint32_t> need(nTiles), odd(nTiles), first(static_cast<size_t>(nTiles) + 1, 0);
+  for (int t = 0; t < nTiles; ++t) {
+    uint32_t m = static_cast<uint32_t>(t);
+    for (int c = 0; c < 3; ++c) {
+      const uint32_t lo = reach[6 * (size_t)t + 2 * c], hi = reach[6 * (size_t)t + 2 * c + 1];
+      if (lo <= hi) m = std::max(m, hi);
+    }
+    need[t] = m;
+    ++first[m + 1];
+  }
+  for (int t = 0; t < nTiles; ++t) first[t + 1] += first[t];
+  for (int t = 0; t < nTiles; ++t) odd[first[need[t]]++] = static_cast<uint32_t>(t);
+  // item k = even tile k, then odd tile odd[k - lead], for the smallest lead
+  // that keeps the margin
+  long long lead = 0;
+  for (int j = 0; j < nTiles; ++j) lead = std::max(lead, static_cast<long long>(need[odd[j]]) + margin - j);
+  lead = std::min<long long>(lead, nTiles);
+  PairItem none{};
+  none.tile = kPairNone;
+  items.assign(static_cast<size_t>(nTiles + lead), none);
+  for (int j = 0; j < nTiles; ++j) {
+    const uint32_t t = odd[j];
+    PairItem& it = items[static_cast<size_t>(j + lead)];
+    it.tile = t;
+    it.run = runOff[t];
+    it.run16 = runOff[t + 1] - runOff[t];
+    for (int c = 0; c < 3; ++c) {
+      const uint32_t lo = reach[6 * (size_t)t + 2 * c], hi = reach[6 * (size_t)t + 2 * c + 1];
+      if (lo > hi) continue;
+      it.lo[c] = lo >> kPairGroupShift;
+      it.n[c] = (hi >> kPairGroupShift) - it.lo[c] + 1;
+    }
+  }
+  for (size_t k = 0; k + kPairAhead < items.size(); ++k) {
+    items[k].aheadRun = items[k + kPairAhead].run;
+    items[k].aheadRun16 = items[k + kPairAhead].run16;
+  }
+  return lead;
 }
 
 }  // namespace lbm

@@ -101,6 +101,11 @@ struct Gpu {
   int nFluid, nCells;
   int cur;  // pull: index of the current grid (0 = dF, 1 = dG)
 
+  // fused step pairs of a list AA instance (null: one launch per step)
+  lbm::PairItem* dPairItems;
+  uint32_t* dPairCount;
+  uint32_t pairItems, pairGroups, pairEpoch;
+
   double* dMomOut;  // 4 doubles for lbm_b200_instance_moments (allocated on first use)
   double* dMomPartials;  // its per-block partial sums for reduced storage (first use)
 
@@ -350,6 +355,18 @@ lbm::ListArgsLp list_args_lp(Gpu* g) {
   return a;
 }
 
+// The arguments of the instance's next fused pair launch.
+lbm::PairArgs pair_args(Gpu* g) {
+  lbm::PairArgs p;
+  p.items = g->dPairItems;
+  p.count = g->dPairCount;
+  p.nItems = g->pairItems;
+  p.nTiles = static_cast<uint32_t>((g->nFluid + lbm::kListTile - 1) / lbm::kListTile);
+  p.epoch = ++g->pairEpoch;
+  p.prefetch = list_prefetch_enabled();
+  return p;
+}
+
 double* current_grid(Gpu* g) { return (two_grid(g->kind) && g->cur == 1) ? g->dG : g->dF; }
 
 // Enqueues n time steps (AA kernels: rounded up to whole even/odd pairs, as
@@ -378,6 +395,16 @@ long enqueue_steps(Gpu* g, const lbm::Trt<double>& t, int n, cudaEvent_t* ev = n
         lbm::aa_odd_face_fp64(a, t, g->stream);
         ++k;
       }
+      g->iteration = it + 1;
+    }
+  } else if (g->kind == kListAa && g->dPairItems) {
+    for (int it = 0; it < n; it += 2) {
+      mark();
+      if (g->storage == lbm::kStoreF64)
+        lbm::list_pair_fp64(list_args(g), pair_args(g), t, g->stream);
+      else
+        lbm::list_pair_lp(list_args_lp(g), pair_args(g), to_trtw(t), g->storage, g->stream);
+      ++k;
       g->iteration = it + 1;
     }
   } else if (g->kind == kListAa && g->storage != lbm::kStoreF64) {
@@ -434,7 +461,7 @@ long enqueue_steps(Gpu* g, const lbm::Trt<double>& t, int n, cudaEvent_t* ev = n
 
 long launches_for(Gpu* g, int n) {
   if (two_grid(g->kind)) return n;
-  long perPair = 2;
+  long perPair = g->dPairItems ? 1 : 2;
   if (g->kind == kAa) {
     const lbm::AaArgs a = aa_args(g);
     perPair = 1 + (g->nOddItems > 0) + (lbm::aa_shell_needed(a) ? 1 : 0);
@@ -505,6 +532,11 @@ void raw_to_mirror(Gpu* g) {
 void clear_lost(Gpu* g) {
   if (!g->stateLost) return;
   LBM_CK(cudaMemsetAsync(g->dErr, 0, sizeof(int), g->stream));
+  if (g->dPairCount) {
+    // fused pairs count from zero again, whatever the lost launch left
+    LBM_CK(cudaMemsetAsync(g->dPairCount, 0, sizeof(uint32_t) * g->pairGroups, g->stream));
+    g->pairEpoch = 0;
+  }
   g->stateLost = false;
 }
 
@@ -613,6 +645,54 @@ void cb_kernel(LatticeDesc* ld, KernelData* kd, CaseData* cd) {
   check_device_error(g);
   download(g);
   if (cd->VtkOutput) vtk_or_exit(ld, kd, cd, cd->MaxIterations);
+}
+
+// Schedules the instance's fused step pairs (lbm_pair.cuh) from its adjacency
+// and run records, or leaves it on two launches per pair.
+//
+// Margin (items between an odd step and the last even tile it needs): shorter,
+// and blocks wait; longer, and the PDFs leave L2 before the odd step. FP64,
+// 256^3 packing, 444 resident blocks: 0.280 ms per step at 350, 0.275 at 444,
+// 0.276 at 520, 0.281 at 600. Reduced storage takes half the room or less:
+// FP32, 740 resident: 0.172 at 740, 0.165 at 1100, 0.171 at 1500.
+//
+// Where the pair pays: the PDFs of the lead (about two x planes and the
+// margin) have to stay in L2. Up to 2/5 of L2 (50 MB) it is faster (FP64,
+// 256^3 packing: 25 MB 0.275 ms per step, 50 MB 0.328, two launches 0.342);
+// beyond (large cross-sections, numberings that put neighbours far apart) the
+// two launches stay. FP16 storage: the two launches' even step, staged for two
+// nodes per thread, is worth more than the traffic saved, so the pair is for
+// domains of at most 2048 tiles, where it is the launch that counts (96^3
+// packing, 1382 tiles: 0.0097 ms per step against 0.0104; 128^3, 3274 tiles:
+// 0.0185 both; 256^3: 0.145 against 0.125).
+constexpr int kPairF16Tiles = 2048;
+
+void schedule_pairs(Gpu* g) {
+  const int nTiles = (g->nFluid + lbm::kListTile - 1) / lbm::kListTile;
+  if (nTiles == 0 || (g->storage == lbm::kStoreF16 && nTiles > kPairF16Tiles)) return;
+  uint32_t* dReach = nullptr;
+  std::vector<uint32_t> reach(6 * (size_t)nTiles), off((size_t)nTiles + 1);
+  LBM_CK(cudaMallocAsync(&dReach, sizeof(uint32_t) * reach.size(), g->stream));
+  lbm::list_tile_reach(g->dAdj, g->nFluid, g->nCells, dReach, g->stream);
+  LBM_CK(cudaGetLastError());
+  LBM_CK(cudaMemcpyAsync(reach.data(), dReach, sizeof(uint32_t) * reach.size(), cudaMemcpyDeviceToHost, g->stream));
+  LBM_CK(cudaMemcpyAsync(off.data(), g->dRunOff, sizeof(uint32_t) * off.size(), cudaMemcpyDeviceToHost, g->stream));
+  LBM_CK(cudaFreeAsync(dReach, g->stream));
+  LBM_CK(cudaStreamSynchronize(g->stream));
+  const int resident = lbm::list_pair_resident(g->storage);
+  const int margin = g->storage == lbm::kStoreF64 ? resident : resident * 3 / 2;
+  std::vector<lbm::PairItem> items;
+  const long long lead = lbm::pair_schedule(reach.data(), off.data(), nTiles, margin, items);
+  int dev = 0, l2 = 0;
+  LBM_CK(cudaGetDevice(&dev));
+  LBM_CK(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev));
+  if (lead * lbm::kListTile * Q * (long long)g->elemBytes > (long long)l2 * 2 / 5) return;
+  g->pairGroups = static_cast<uint32_t>((nTiles + (1 << lbm::kPairGroupShift) - 1) >> lbm::kPairGroupShift);
+  LBM_CK(cudaMalloc(&g->dPairCount, sizeof(uint32_t) * g->pairGroups));
+  LBM_CK(cudaMemset(g->dPairCount, 0, sizeof(uint32_t) * g->pairGroups));
+  LBM_CK(cudaMalloc(&g->dPairItems, sizeof(lbm::PairItem) * items.size()));
+  LBM_CK(cudaMemcpy(g->dPairItems, items.data(), sizeof(lbm::PairItem) * items.size(), cudaMemcpyHostToDevice));
+  g->pairItems = static_cast<uint32_t>(items.size());
 }
 
 // --- Init / Deinit ----------------------------------------------------------------
@@ -794,6 +874,7 @@ Gpu* gpu_new(Kind kind, LatticeDesc* ld, Parameters* params, const SlabSpec* sla
         std::exit(1);
       }
     }
+    if (kind == kListAa && !g->listSlab) schedule_pairs(g);
     g->mirrorElems = (size_t)Q * nCells;
     LBM_CK(cudaMalloc(&g->dF, g->elemBytes * g->mirrorElems));
     LBM_CK(cudaMemset(g->dF, 0, g->elemBytes * g->mirrorElems));
@@ -841,6 +922,8 @@ void gpu_free(KernelData** kernelData) {
   cudaFree(g->dAdj);
   cudaFree(g->dRuns);
   cudaFree(g->dRunOff);
+  cudaFree(g->dPairItems);
+  cudaFree(g->dPairCount);
   for (int side = 0; side < 2; ++side)
     for (int list = 0; list < 2; ++list) cudaFree(g->dHalo[side][list]);
   cudaFree(g->dErr);

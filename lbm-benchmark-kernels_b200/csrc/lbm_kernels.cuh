@@ -158,6 +158,49 @@ void slot_scatter(void* f, const uint32_t* idx, long long n, const void* buf, in
 int list_runs_device(const uint32_t* adj, int nFluid, cudaStream_t s, uint32_t** runs, uint32_t** runOff,
                      size_t* runBytes);
 
+// Fused list AA step pairs (lbm_pair.cuh): one launch runs the even and the
+// odd step. Item k: the even step of tile k (k < nTiles), then the odd step
+// of the tile that the record names, once the groups of 2^kPairGroupShift even
+// tiles that its links reach are complete: up to three ranges [lo, lo + n) of
+// groups (links with c_x = -1, 0, +1).
+constexpr int kPairGroupShift = 3;
+struct PairItem {
+  uint32_t tile;   // tile of the odd step, or kPairNone
+  uint32_t run;    // its run record, 16-byte units into the records
+  uint32_t run16;  // its size, 16-byte units
+  uint32_t lo[3], n[3];
+  uint32_t aheadRun, aheadRun16;  // run record of the item kPairAhead later (0: none)
+  uint32_t pad;
+};
+constexpr uint32_t kPairNone = 0xffffffffu;
+constexpr uint32_t kPairAhead = 512;  // about a wave of resident blocks
+constexpr int kPairItemWords = static_cast<int>(sizeof(PairItem) / 4);
+static_assert(sizeof(PairItem) == 48, "item records are loaded as 12 words");
+
+struct PairArgs {
+  const PairItem* items;  // nItems records
+  uint32_t* count;        // even tiles done per group, summed over all launches
+  uint32_t nItems;        // blocks of the launch
+  uint32_t nTiles;
+  uint32_t epoch;         // launches including this one (counter targets)
+  int prefetch;           // as ListArgs::prefetch (0: none)
+};
+
+// Tiles that each tile's links reach (device; 6 words per tile: the lowest
+// and highest tile reached by links with c_x = -1, 0, +1; lowest > highest:
+// none), for the nFluid nodes of adj.
+void list_tile_reach(const uint32_t* adj, int nFluid, long long nCells, uint32_t* reach, cudaStream_t s);
+// Host: the item records of a fused pair from the tiles' reach and the run
+// records' offsets (nTiles + 1). Every odd step comes at least `margin` items
+// after the last even tile it needs, or after all of them. Returns the items
+// between a tile's even and its odd step (the lead of the even steps).
+long long pair_schedule(const uint32_t* reach, const uint32_t* runOff, int nTiles, int margin,
+                        std::vector<PairItem>& items);
+// Blocks of a fused kernel that run at once on the current device.
+int list_pair_resident(int storage);
+void list_pair_fp64(const ListArgs& a, const PairArgs& p, const Trt<double>& t, cudaStream_t s);
+void list_pair_lp(const ListArgsLp& a, const PairArgs& p, const TrtW& t, int storage, cudaStream_t s);
+
 // Launchers (stream-ordered, no synchronisation).
 void list_even_lp(const ListArgsLp& a, const TrtW& t, int storage, cudaStream_t s);
 void list_odd_lp(const ListArgsLp& a, const TrtW& t, int storage, cudaStream_t s);

@@ -27,6 +27,7 @@
 
 #include "lbm_bulk.cuh"
 #include "lbm_kernels.cuh"
+#include "lbm_pair.cuh"
 
 namespace lbm {
 
@@ -676,6 +677,51 @@ __global__ void __launch_bounds__(kListTile, 3) k_list_odd_fp64(const ListArgs a
   trt_update(t, load, store);
 }
 
+// The fused pair (lbm_pair.cuh): the arithmetic of the two kernels above. The
+// parameters are read in place (__grid_constant__), which leaves room for
+// both steps under the 72 registers of 3 blocks of 288 threads per SM. What
+// bounds it: L2 and the fabric between its halves (the odd step's gathers and
+// scatters touch 1.2-1.5 sectors per sector of payload; without any waiting
+// the 256^3 packing would take 0.247 ms per step), then the waits.
+__global__ void __launch_bounds__(kPairThreads, 3)
+    k_list_pair_fp64(const __grid_constant__ ListArgs a, const __grid_constant__ PairArgs p,
+                     const __grid_constant__ Trt<double> t) {
+  __shared__ PairShared sh;
+  pair_init(&sh);
+  const uint32_t k = blockIdx.x;
+  if (threadIdx.x >= kListTile) {
+    pair_service(&sh, p, a.runs, a.err, k);
+    return;
+  }
+  const long long S = a.nCells;
+  if (k < p.nTiles) {
+    const int n = static_cast<int>(k) * kListTile + threadIdx.x;
+    if (n < a.nFluid) {
+      const double* const f = a.f + n;
+      double* const fs = launder(a.f + n);
+      const uint64_t keep = l2_keep_policy();
+      trt_update(t, [&](int d) { return __ldcs(f + d * S); },
+                 [&](int d, double v) { st_keep(fs + inv(d) * S, v, keep); });
+    }
+    pair_even_done(&sh);
+  }
+  if (!pair_odd_turn(&sh, a.err)) return;
+  const int n = static_cast<int>(sh.item.tile) * kListTile + threadIdx.x;
+  if (n >= a.nFluid) return;
+  uint32_t off;
+  const uint32_t* e = run_row(sh.run, threadIdx.x, off);
+  double* const f = a.f;
+  auto load = [&](int d) -> double { return (d == DC ? f[DC * S + n] : f[e[inv(d)] + off]) + t.force[d]; };
+  auto store = [&](int d, double v) {
+    if (d == DC) { __stcs(f + DC * S + n, v + t.force[DC]); return; }
+    const uint32_t dst = reinterpret_cast<const volatile uint32_t*>(e)[d] + off;
+    const int j = inv(d);
+    const bool bounce = dst == static_cast<uint32_t>(j * S + n);
+    __stcs(f + dst, v + (bounce ? t.force[j] : t.force[d]));
+  };
+  trt_update(t, load, store);
+}
+
 __global__ void __launch_bounds__(kListTile) k_list_pull_fp64(const ListArgs a, const Trt<double> t) {
   __shared__ alignas(128) uint32_t srun[kRunTileWords];
   __shared__ alignas(8) uint64_t bar;
@@ -803,6 +849,13 @@ void list_odd_fp64_tiles(const ListArgs& a, const Trt<double>& t, int t0, int t1
   b.tileBase = t0;
   b.prefetch = prefetch_distance(g_oddAhead, k_list_odd_fp64, kListTile, a.prefetch != 0);
   k_list_odd_fp64<<<(unsigned)(t1 - t0), kListTile, 0, s>>>(b, t);
+}
+void list_pair_fp64(const ListArgs& a, const PairArgs& p, const Trt<double>& t, cudaStream_t s) {
+  if (p.nItems > 0) k_list_pair_fp64<<<p.nItems, kPairThreads, 0, s>>>(a, p, t);
+}
+int list_pair_resident_fp64() {
+  static std::atomic<int> n{0};
+  return prefetch_distance(n, k_list_pair_fp64, kPairThreads, true);
 }
 void list_pull_fp64(const ListArgs& a, const Trt<double>& t, cudaStream_t s) {
   // no adjacency prefetch: with the full adjacency it slowed this kernel by

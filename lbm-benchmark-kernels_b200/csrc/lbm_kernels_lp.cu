@@ -7,6 +7,7 @@
 
 #include "lbm_bulk.cuh"
 #include "lbm_kernels.cuh"
+#include "lbm_pair.cuh"
 #include "lbm_store.cuh"
 
 namespace lbm {
@@ -127,6 +128,53 @@ __global__ void __launch_bounds__(kListTile, LBM_LP_ODD_BLOCKS) k_list_odd_lp(co
   uint32_t off;
   const uint32_t* e = run_row(srun, threadIdx.x, off);  // link d = e[d] + off (run-compressed adjacency)
   lp_odd_node<St>(static_cast<typename St::T*>(a.f), static_cast<uint32_t>(a.nCells), n, e, off, TrtDev<St>(w));
+}
+
+// The fused pair (lbm_pair.cuh): the arithmetic of the per-node even kernel
+// and of the odd kernel above. 5 blocks of 288 threads per SM (40 registers);
+// 4 blocks measured the same, 3 slower (FP32, 256^3 packing: 0.165, 0.166 and
+// 0.173 ms per step; two launches 0.185).
+template <class St>
+__global__ void __launch_bounds__(kPairThreads, 5)
+    k_list_pair_lp(const __grid_constant__ ListArgsLp a, const __grid_constant__ PairArgs p,
+                   const __grid_constant__ TrtW w) {
+  __shared__ PairShared sh;
+  pair_init(&sh);
+  const uint32_t k = blockIdx.x;
+  if (threadIdx.x >= kListTile) {
+    pair_service(&sh, p, a.runs, a.err, k);
+    return;
+  }
+  using T = typename St::T;
+  const TrtDev<St> t(w);
+  if (k < p.nTiles) {
+    const int n = static_cast<int>(k) * kListTile + threadIdx.x;
+    if (n < a.nFluid) lp_even_node<St, true, PairAccess>(static_cast<T*>(a.f), a.nCells, n, t);
+    pair_even_done(&sh);
+  }
+  if (!pair_odd_turn(&sh, a.err)) return;
+  const int n = static_cast<int>(sh.item.tile) * kListTile + threadIdx.x;
+  if (n >= a.nFluid) return;
+  uint32_t off;
+  const uint32_t* e = run_row(sh.run, threadIdx.x, off);
+  lp_odd_node<St, true, PairAccess>(static_cast<T*>(a.f), static_cast<uint32_t>(a.nCells), n, e, off, t);
+}
+
+void list_pair_lp(const ListArgsLp& a, const PairArgs& p, const TrtW& t, int storage, cudaStream_t s) {
+  if (p.nItems == 0) return;
+  if (storage == kStoreF16)
+    k_list_pair_lp<StoreF16><<<p.nItems, kPairThreads, 0, s>>>(a, p, t);
+  else
+    k_list_pair_lp<StoreF32><<<p.nItems, kPairThreads, 0, s>>>(a, p, t);
+}
+
+int list_pair_resident_fp64();
+
+int list_pair_resident(int storage) {
+  static std::atomic<int> n32{0}, n16{0};
+  if (storage == kStoreF16) return prefetch_distance(n16, k_list_pair_lp<StoreF16>, kPairThreads, true);
+  if (storage == kStoreF32) return prefetch_distance(n32, k_list_pair_lp<StoreF32>, kPairThreads, true);
+  return list_pair_resident_fp64();
 }
 
 static unsigned lp_blocks(const ListArgsLp& a) { return (a.nFluid + kListTile - 1) / kListTile; }

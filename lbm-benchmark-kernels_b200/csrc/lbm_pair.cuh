@@ -1,0 +1,153 @@
+// lbm_pair.cuh -- the even and the odd step of a list AA pair in one launch,
+// the odd step trailing the even one closely enough that it finds the PDFs in
+// L2 (shared by the FP64, the reduced-storage and the batched kernels).
+//
+// What bounds the two-launch pair: each step streams all PDFs through HBM
+// (304 B per FP64 node and step). The odd step of a tile needs the even step
+// of the tiles its links reach and of no others: with the blocked x-y-z
+// numbering these lie within one x plane on either side. So block k of the
+// fused launch runs the even step of tile k and then the odd step of a tile
+// about two planes back, whose PDFs the even step wrote a few microseconds
+// earlier: HBM is read once and written once per pair.
+//
+// Order and waiting. Even steps wait for nothing. An odd step waits until the
+// groups of even tiles its links reach are complete (counters in device
+// memory, release/acquire at GPU scope). The hardware starts the blocks of a
+// one-dimensional grid in index order, and item k only depends on the even
+// tiles of blocks at least `margin` below k, so the blocks that a waiting one
+// depends on have always started and, waiting for nothing before their even
+// tile is counted, always finish it. The wait is bounded all the same: it
+// gives up after kPairSpinLimit polls, or as soon as another block has, and
+// sets the error word.
+//
+// Work split of a block: 8 compute warps (one thread per node) and one
+// service warp that fetches the item and the tile's run record, polls the
+// counters while the compute warps run the even step, and counts the even
+// tile once they are done. The release then costs the compute warps nothing
+// (waiting for a tile's stores to reach L2 takes 3-6 us under load; done by
+// a compute warp the 256^3 packing's pair was slower by 7 %), and there is no
+// block-wide barrier between the two steps.
+#pragma once
+#include <cstdint>
+
+#include "lbm_bulk.cuh"
+#include "lbm_kernels.cuh"
+
+namespace lbm {
+
+constexpr int kPairThreads = kListTile + 32;
+constexpr uint32_t kPairSpinLimit = 1u << 20;  // polls before giving up
+
+// Cache hints. A slot written by the even step is read back by the odd step
+// soon, one written by the odd step not before the next pair: even loads and
+// odd stores stream (evict first), so that finished tiles do not push waiting
+// ones out of L2, and FP64 even stores ask to be kept (256^3 packing, FP64:
+// 0.298 -> 0.275 ms per step; the reduced storage takes a third or less of the
+// room and does without the policy's registers).
+__device__ __forceinline__ uint64_t l2_keep_policy() {
+  uint64_t p;
+  asm("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(p));
+  return p;
+}
+__device__ __forceinline__ void st_keep(double* a, double v, uint64_t pol) {
+  asm volatile("st.global.L2::cache_hint.f64 [%0], %1, %2;" ::"l"(a), "d"(v), "l"(pol) : "memory");
+}
+__device__ __forceinline__ uint32_t ld_acquire(const uint32_t* p) {
+  uint32_t v;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void red_release(uint32_t* p, uint32_t v) {
+  asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
+  asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+}
+
+// What a block shares: the odd tile's run record, its item, and the two
+// hand-overs between the service warp and the compute warps.
+struct PairShared {
+  alignas(128) uint32_t run[kRunTileWords];
+  alignas(16) PairItem item;
+  alignas(8) uint64_t go;    // the odd step may start: dependencies met, run record here
+  alignas(8) uint64_t even;  // every compute warp has stored its even nodes
+};
+
+__device__ __forceinline__ void pair_init(PairShared* sh) {
+  if (threadIdx.x == kListTile) {
+    mbar_init(&sh->go, 1);
+    mbar_init(&sh->even, kListTile / 32);
+  }
+  __syncthreads();
+}
+
+// One look (by the whole warp) at the even groups the item depends on:
+// whether all are complete. Counters and targets are compared modulo 2^32.
+__device__ __forceinline__ bool pair_ready(const PairItem& it, const PairArgs& p) {
+  const uint32_t n0 = it.n[0], n01 = n0 + it.n[1], all = n01 + it.n[2];
+  bool good = true;
+  for (uint32_t i = threadIdx.x & 31; i < all; i += 32) {
+    const uint32_t g = i < n0 ? it.lo[0] + i : (i < n01 ? it.lo[1] + (i - n0) : it.lo[2] + (i - n01));
+    const uint32_t size = min(p.nTiles - (g << kPairGroupShift), 1u << kPairGroupShift);
+    good = good && static_cast<int32_t>(ld_acquire(p.count + g) - p.epoch * size) >= 0;
+  }
+  return __all_sync(0xffffffffu, good);
+}
+
+// The service warp of block k (see above).
+__device__ __forceinline__ void pair_service(PairShared* sh, const PairArgs& p, const uint32_t* runs, int* err,
+                                             uint32_t k) {
+  const int lane = threadIdx.x - kListTile;
+  const bool even = k < p.nTiles;
+  if (lane < kPairItemWords)
+    reinterpret_cast<uint32_t*>(&sh->item)[lane] = __ldg(reinterpret_cast<const uint32_t*>(p.items + k) + lane);
+  __syncwarp();
+  const PairItem& it = sh->item;
+  if (lane == 0) {
+    if (it.tile != kPairNone) {
+      mbar_expect_tx(&sh->go, it.run16 * 16u);
+      bulk_g2s(sh->run, runs + static_cast<size_t>(it.run) * 4, it.run16 * 16u, &sh->go);
+    }
+    if (p.prefetch) {
+      // the record and the item of blocks that have not started yet, into L2
+      if (it.aheadRun16) bulk_prefetch_l2(runs + static_cast<size_t>(it.aheadRun) * 4, it.aheadRun16 * 16u);
+      if (k + 2 * kPairAhead < p.nItems) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.items + k + 2 * kPairAhead));
+    }
+  }
+  const bool ready = it.tile == kPairNone || pair_ready(it, p);
+  if (ready && lane == 0) mbar_arrive(&sh->go);
+  if (even) {
+    if (!mbar_wait_bounded(&sh->even, 0)) atomicOr(err, 1);
+    if (lane == 0) red_release(p.count + (k >> kPairGroupShift), 1u);
+  }
+  if (!ready) {
+    for (uint32_t spin = 0; !pair_ready(it, p); ++spin) {
+      const bool stop = spin >= kPairSpinLimit || ((spin & 255u) == 255u && *reinterpret_cast<volatile int*>(err) != 0);
+      if (__any_sync(0xffffffffu, stop)) {
+        if (lane == 0) atomicOr(err, 1);
+        break;
+      }
+    }
+    if (lane == 0) mbar_arrive(&sh->go);
+  }
+}
+
+// Compute warps: their even nodes are stored.
+__device__ __forceinline__ void pair_even_done(PairShared* sh) {
+  __syncwarp();
+  if ((threadIdx.x & 31) == 0) mbar_arrive(&sh->even);
+}
+
+// Compute warps: waits for the odd step's turn; false if there is none.
+__device__ __forceinline__ bool pair_odd_turn(PairShared* sh, int* err) {
+  if (!mbar_wait_bounded(&sh->go, 0)) {
+    atomicOr(err, 1);
+    return false;
+  }
+  return sh->item.tile != kPairNone;
+}
+
+}  // namespace lbm

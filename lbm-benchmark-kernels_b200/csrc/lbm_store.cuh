@@ -160,15 +160,31 @@ __device__ __forceinline__ void trt_collide_dev(const TrtDev<St>& t, const float
   }
 }
 
+// How a node update accesses its PDFs (L2 cache hints): as they come, or for
+// the fused pair, where even loads and odd stores stream past what waits in L2
+// between the two steps (lbm_pair.cuh).
+struct PlainAccess {
+  template <class T>
+  __device__ static T even_load(const T* p) { return *p; }
+  template <class T>
+  __device__ static void odd_store(T* p, T v) { *p = v; }
+};
+struct PairAccess {
+  template <class T>
+  __device__ static T even_load(const T* p) { return __ldcs(p); }
+  template <class T>
+  __device__ static void odd_store(T* p, T v) { __stcs(p, v); }
+};
+
 // Even step of node n (local collide, swapped store): f[d * S + n].
-template <class St, bool kPacked = true>
+template <class St, bool kPacked = true, class Access = PlainAccess>
 __device__ __forceinline__ void lp_even_node(typename St::T* f, long long S, int n, const TrtDev<St>& t) {
   using T = typename St::T;
   const T* const src = f + n;
   T* const dst = launder(f + n);
   float x[Q], o[Q];
 #pragma unroll
-  for (int d = 0; d < Q; ++d) x[d] = St::in(src[d * S], d);
+  for (int d = 0; d < Q; ++d) x[d] = St::in(Access::even_load(src + d * S), d);
   trt_collide_dev<St, kPacked>(t, x, o);
 #pragma unroll
   for (int d = 0; d < Q; ++d) dst[inv(d) * S] = St::out(o[d], inv(d));
@@ -183,7 +199,7 @@ __device__ __forceinline__ void lp_even_node(typename St::T* f, long long S, int
 // link's plane (one compare against a constant per direction). Addresses
 // are formed from f + off, so a link costs one index on top of its
 // shared-memory read.
-template <class St, bool kPacked = true>
+template <class St, bool kPacked = true, class Access = PlainAccess>
 __device__ __forceinline__ void lp_odd_node(typename St::T* f, uint32_t S, uint32_t n, const uint32_t* e,
                                             uint32_t off, const TrtDev<St>& t) {
   using T = typename St::T;
@@ -201,7 +217,7 @@ __device__ __forceinline__ void lp_odd_node(typename St::T* f, uint32_t S, uint3
   }
   trt_collide_dev<St, kPacked>(t, x, o);
   T* const fs = launder(fo);
-  fs[DC * S + head] = St::out(o[DC], DC);
+  Access::odd_store(fs + (DC * S + head), St::out(o[DC], DC));
 #pragma unroll
   for (int d = 0; d < QM; ++d) {
     // re-read from shared memory: keeps no links live across the collision
@@ -212,7 +228,7 @@ __device__ __forceinline__ void lp_odd_node(typename St::T* f, uint32_t S, uint3
       const bool bounce = inv(d) < d ? ed < static_cast<uint32_t>(d) * S : ed >= static_cast<uint32_t>(d + 1) * S;
       v += bounce ? t.force(inv(d)) : t.force(d);
     }
-    fs[ed] = St::out(v, d);  // the scale is equal for d and inv(d)
+    Access::odd_store(fs + ed, St::out(v, d));  // the scale is equal for d and inv(d)
   }
 }
 

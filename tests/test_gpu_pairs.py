@@ -1,0 +1,52 @@
+"""The fused even/odd launch of the list AA rows (csrc/lbm_pair.cuh) where it
+has to wait: lattices with more tiles than the lead of the even steps, so that
+blocks run the even step of one tile and the odd step of another while the
+steps they depend on are still under way. Small lattices, whose odd steps all
+follow the even ones, are in test_gpu_parity.py. The reference is the same
+lattice as two x-slabs, which take one launch per step; the arithmetic is the
+same, so the fields agree bit for bit in every storage."""
+import numpy as np
+import pytest
+
+import lbmb200
+from lbm_cases import random_pdfs
+from test_gpu_slabs import _run_slabs
+
+pytestmark = pytest.mark.gpu
+
+
+def _spheres(dims, porosity):
+    return lbmb200.spheres(dims, 42, porosity, 3.0, 6.0, 4000)[0]
+
+
+CASES = [
+    # periodic rings: the first x plane's odd step needs the last plane's even step
+    (lambda: _spheres((160, 61, 60), 0.6), ["-precision", "fp64"]),
+    (lambda: _spheres((160, 61, 60), 0.6), ["-precision", "fp32"]),
+    (lambda: _spheres((160, 61, 60), 0.6), ["-precision", "fp16"]),
+    (lambda: lbmb200.geometry("fluid", (131, 41, 43), (1, 1, 1)), ["-pad", "no"]),
+    # numberings whose neighbours lie further apart, and closed x ends
+    (lambda: _spheres((150, 48, 50), 0.6), ["-blk", "24"]),
+    (lambda: lbmb200.geometry("box", (120, 44, 45), (0, 1, 1)), ["-blk-z", "16"]),
+    # planes of less than one tile
+    (lambda: lbmb200.geometry("fluid", (2500, 9, 11), (1, 1, 1)), ["-pad", "no"]),
+]
+
+
+@pytest.mark.parametrize("make,kargs", CASES)
+def test_fused_pairs_equal_separate_steps(make, kargs):
+    lat = make()
+    init = random_pdfs(lat.mask.size, 53)
+    cd = lbmb200.case(omega=1.2, xforce=2e-4, iterations=8)
+    kargs = ["-lambda", "3/16"] + kargs
+    inst = lbmb200.kernel("cuda-list-aa-pv-soa").init(lat, kernel_args=kargs)
+    try:
+        assert inst.launches_for(2) == 1 and lat.n_fluid > 450 * 256
+        inst.set_field(init)
+        inst.run(cd)
+        whole = inst.get_field()
+    finally:
+        inst.deinit()
+    got = _run_slabs(lat, 2, init, cd, 4, layout="list", kargs=kargs)
+    m = lat.mask != 0
+    assert np.array_equal(got[m], whole[m])
