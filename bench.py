@@ -323,23 +323,18 @@ def list_aa_roofline(t, nodes, pdf_bytes, adj_node, peak, names):
 
 
 def aa_line(lbmb200, fl, args, kargs, dist, peak):
-    """Device-timed cuda-aa-soa steps on lattice `fl`: MFLUP/s, HBM fraction,
-    per-launch split of each even/odd pair, and the reference's fastest
-    full-array CPU kernel (aa-vec-soa) on the same lattice beside it."""
+    """Device-timed cuda-aa-soa steps on lattice `fl`: MFLUP/s and HBM fraction
+    of the fused even/odd launches, and the reference's fastest full-array CPU
+    kernel (aa-vec-soa) on the same lattice beside it."""
     ta = time_kernel(lbmb200, "cuda-aa-soa", fl, min(args.steps, 200), 4, kargs, dist, "aa")
     ta["inst"].deinit()
-    per, lpp = ta["per_launch_ms"], ta["launches_per_pair"]
-    # per pair: even step, then the odd step's launches (interior blocks without
-    # and with reversed links, face shell)
-    pairs = [per[k:k + lpp] for k in range(0, len(per) - lpp + 1, lpp)]
-    ev = statistics.mean(p[0] for p in pairs)
-    od = statistics.mean(sum(p[1:]) for p in pairs)
-    am = (ev + od) / 2
-    out = {"fluid_nodes": fl.n_fluid, "mflups": round(fl.n_fluid / (am / 1e3) / 1e6, 1),
-           "achieved_gbs": round(B_PER_FLUP["aa"] * fl.n_fluid / (am / 1e3) / 1e9, 1),
-           "frac": round(B_PER_FLUP["aa"] * fl.n_fluid / (am / 1e3) / 1e9 / peak, 4),
-           "even_ms": round(ev, 5), "odd_ms": round(od, 5),
-           "odd_launch_ms": [round(statistics.mean(p[k] for p in pairs), 5) for k in range(1, lpp)]}
+    # one launch per pair: the PDFs have to be read and written once in it
+    # (bytes per pair); "streamed" counts both steps' accesses
+    pm = statistics.mean(ta["per_launch_ms"])
+    once = B_PER_FLUP["aa"] * fl.n_fluid / (pm / 1e3) / 1e9
+    out = {"fluid_nodes": fl.n_fluid, "mflups": round(2 * fl.n_fluid / (pm / 1e3) / 1e6, 1),
+           "bytes_per_pair": B_PER_FLUP["aa"], "achieved_gbs": round(once, 1), "frac": round(once / peak, 4),
+           "streamed_gbs": round(2 * once, 1), "pair_ms": round(pm, 5)}
     if dist.rank == 0 and dist.world == 1 and not args.no_cpu:
         probe = cpu_reference(fl, 2, kernel="aa-vec-soa")
         if probe is not None:

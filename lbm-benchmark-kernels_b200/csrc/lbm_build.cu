@@ -318,51 +318,25 @@ void list_tile_reach(const uint32_t* adj, int nFluid, long long nCells, uint32_t
   if (nTiles > 0) k_tile_reach<<<nTiles, kListTile, 0, s>>>(adj, nFluid, static_cast<uint32_t>(nCells), reach);
 }
 
-long long pair_schedule(const uint32_t* reach, const uint32_t* runOff, int nTiles, int margin,
-                        std::vector<PairItem>& items) {
-  items.clear();
-  if (nTiles <= 0) return 0;
-  // the odd steps in the order of the last even tile they need (a counting
-  // sort; with the blocked numbering this is nearly the tile order, except
-  // for the first x plane of a periodic lattice, which needs the last one)
-  std::vector<uint32_t> need(nTiles), odd(nTiles), first(static_cast<size_t>(nTiles) + 1, 0);
+double pair_schedule(const uint32_t* reach, const uint32_t* runOff, int nTiles, int margin, double maxLag,
+                     std::vector<PairItem>& items) {
+  std::vector<PairItem> work(nTiles);
+  std::vector<uint32_t> need(nTiles), home(nTiles);
   for (int t = 0; t < nTiles; ++t) {
-    uint32_t m = static_cast<uint32_t>(t);
-    for (int c = 0; c < 3; ++c) {
-      const uint32_t lo = reach[6 * (size_t)t + 2 * c], hi = reach[6 * (size_t)t + 2 * c + 1];
-      if (lo <= hi) m = std::max(m, hi);
-    }
-    need[t] = m;
-    ++first[m + 1];
-  }
-  for (int t = 0; t < nTiles; ++t) first[t + 1] += first[t];
-  for (int t = 0; t < nTiles; ++t) odd[first[need[t]]++] = static_cast<uint32_t>(t);
-  // item k = even tile k, then odd tile odd[k - lead], for the smallest lead
-  // that keeps the margin
-  long long lead = 0;
-  for (int j = 0; j < nTiles; ++j) lead = std::max(lead, static_cast<long long>(need[odd[j]]) + margin - j);
-  lead = std::min<long long>(lead, nTiles);
-  PairItem none{};
-  none.tile = kPairNone;
-  items.assign(static_cast<size_t>(nTiles + lead), none);
-  for (int j = 0; j < nTiles; ++j) {
-    const uint32_t t = odd[j];
-    PairItem& it = items[static_cast<size_t>(j + lead)];
-    it.tile = t;
+    PairItem& it = work[t];
+    it = PairItem{};
+    it.tile = home[t] = need[t] = static_cast<uint32_t>(t);
     it.run = runOff[t];
     it.run16 = runOff[t + 1] - runOff[t];
     for (int c = 0; c < 3; ++c) {
       const uint32_t lo = reach[6 * (size_t)t + 2 * c], hi = reach[6 * (size_t)t + 2 * c + 1];
       if (lo > hi) continue;
+      need[t] = std::max(need[t], hi);
       it.lo[c] = lo >> kPairGroupShift;
       it.n[c] = (hi >> kPairGroupShift) - it.lo[c] + 1;
     }
   }
-  for (size_t k = 0; k + kPairAhead < items.size(); ++k) {
-    items[k].aheadRun = items[k + kPairAhead].run;
-    items[k].aheadRun16 = items[k + kPairAhead].run16;
-  }
-  return lead;
+  return pair_order(work, need, home, static_cast<size_t>(nTiles), static_cast<size_t>(margin), maxLag, items);
 }
 
 }  // namespace lbm

@@ -82,6 +82,7 @@ struct Gpu {
   int* dOddItems;          // odd step: nOddItems interior work items (aa_interior_items)
   int* dOddCells;          // odd step: the general cells of the items, in chunks of 128
   int nOddItems;
+  bool oddItemsBuilt;
   // x-slab of a larger lattice (lbm_aa_slab_init): halo/cross flags of the two x faces
   int halo[2], cross[2];
   int* sliceMask;          // the slab's own mask (owned)
@@ -101,10 +102,12 @@ struct Gpu {
   int nFluid, nCells;
   int cur;  // pull: index of the current grid (0 = dF, 1 = dG)
 
-  // fused step pairs of a list AA instance (null: one launch per step)
-  lbm::PairItem* dPairItems;
+  // fused step pairs of an AA instance (lbm_pair.cuh; null: a launch per step)
+  void* dPairItems;        // PairItem (lists) or AaPairItem (full array) records
   uint32_t* dPairCount;
-  uint32_t pairItems, pairGroups, pairEpoch;
+  uint32_t pairItems, pairTiles, pairGroups, pairEpoch;
+  lbm::AaPairGeom pairGeom;
+  int openFaces;
 
   double* dMomOut;  // 4 doubles for lbm_b200_instance_moments (allocated on first use)
   double* dMomPartials;  // its per-block partial sums for reduced storage (first use)
@@ -304,6 +307,7 @@ lbm::AaArgs aa_args(Gpu* g) {
   a.crossLo = g->cross[0];
   a.crossHi = g->cross[1];
   a.xBase = 0;
+  a.err = g->dErr;
   const int S = (int)g->dstride;
   for (int d = 0; d < Q; ++d) {
     const int j = lbm::inv(d);
@@ -356,12 +360,13 @@ lbm::ListArgsLp list_args_lp(Gpu* g) {
 }
 
 // The arguments of the instance's next fused pair launch.
-lbm::PairArgs pair_args(Gpu* g) {
-  lbm::PairArgs p;
-  p.items = g->dPairItems;
+template <int R>
+lbm::PairArgs<R> pair_args(Gpu* g) {
+  lbm::PairArgs<R> p;
+  p.items = static_cast<const lbm::PairRec<R>*>(g->dPairItems);
   p.count = g->dPairCount;
   p.nItems = g->pairItems;
-  p.nTiles = static_cast<uint32_t>((g->nFluid + lbm::kListTile - 1) / lbm::kListTile);
+  p.nTiles = g->pairTiles;
   p.epoch = ++g->pairEpoch;
   p.prefetch = list_prefetch_enabled();
   return p;
@@ -378,7 +383,16 @@ long enqueue_steps(Gpu* g, const lbm::Trt<double>& t, int n, cudaEvent_t* ev = n
   auto mark = [&]() {
     if (ev) cudaEventRecord(ev[k], g->stream);
   };
-  if (g->kind == kAa) {
+  if (g->kind == kAa && g->dPairItems) {
+    const lbm::AaArgs a = aa_args(g);
+    for (int it = 0; it < n; it += 2) {
+      mark();
+      const lbm::AaPairArgs q{pair_args<9>(g), g->pairGeom, g->openFaces};
+      lbm::aa_pair_fp64(a, q, t, g->stream);
+      ++k;
+      g->iteration = it + 1;
+    }
+  } else if (g->kind == kAa) {
     lbm::AaArgs a = aa_args(g);
     const bool shell = lbm::aa_shell_needed(a);
     for (int it = 0; it < n; it += 2) {
@@ -401,9 +415,9 @@ long enqueue_steps(Gpu* g, const lbm::Trt<double>& t, int n, cudaEvent_t* ev = n
     for (int it = 0; it < n; it += 2) {
       mark();
       if (g->storage == lbm::kStoreF64)
-        lbm::list_pair_fp64(list_args(g), pair_args(g), t, g->stream);
+        lbm::list_pair_fp64(list_args(g), pair_args<3>(g), t, g->stream);
       else
-        lbm::list_pair_lp(list_args_lp(g), pair_args(g), to_trtw(t), g->storage, g->stream);
+        lbm::list_pair_lp(list_args_lp(g), pair_args<3>(g), to_trtw(t), g->storage, g->stream);
       ++k;
       g->iteration = it + 1;
     }
@@ -462,7 +476,7 @@ long enqueue_steps(Gpu* g, const lbm::Trt<double>& t, int n, cudaEvent_t* ev = n
 long launches_for(Gpu* g, int n) {
   if (two_grid(g->kind)) return n;
   long perPair = g->dPairItems ? 1 : 2;
-  if (g->kind == kAa) {
+  if (g->kind == kAa && !g->dPairItems) {
     const lbm::AaArgs a = aa_args(g);
     perPair = 1 + (g->nOddItems > 0) + (lbm::aa_shell_needed(a) ? 1 : 0);
   }
@@ -647,27 +661,48 @@ void cb_kernel(LatticeDesc* ld, KernelData* kd, CaseData* cd) {
   if (cd->VtkOutput) vtk_or_exit(ld, kd, cd, cd->MaxIterations);
 }
 
-// Schedules the instance's fused step pairs (lbm_pair.cuh) from its adjacency
-// and run records, or leaves it on two launches per pair.
+// Fused step pairs (lbm_pair.cuh): the order of the work. Whole full-array
+// lattices always take them; lists do unless that is the slower way (below),
+// slabs do not (their halo messages travel between the steps).
 //
 // Margin (items between an odd step and the last even tile it needs): shorter,
-// and blocks wait; longer, and the PDFs leave L2 before the odd step. FP64,
-// 256^3 packing, 444 resident blocks: 0.280 ms per step at 350, 0.275 at 444,
-// 0.276 at 520, 0.281 at 600. Reduced storage takes half the room or less:
-// FP32, 740 resident: 0.172 at 740, 0.165 at 1100, 0.171 at 1500.
+// and blocks wait; longer, and the PDFs leave L2 before the odd step. Lists,
+// FP64, 256^3 packing, 444 resident blocks: 0.280 ms per step at 350, 0.275 at
+// 444, 0.276 at 520, 0.281 at 600. Reduced storage takes half the room or
+// less: FP32, 740 resident: 0.172 at 740, 0.165 at 1100, 0.171 at 1500.
 //
-// Where the pair pays: the PDFs of the lead (about two x planes and the
-// margin) have to stay in L2. Up to 2/5 of L2 (50 MB) it is faster (FP64,
-// 256^3 packing: 25 MB 0.275 ms per step, 50 MB 0.328, two launches 0.342);
-// beyond (large cross-sections, numberings that put neighbours far apart) the
-// two launches stay. FP16 storage: the two launches' even step, staged for two
-// nodes per thread, is worth more than the traffic saved, so the pair is for
-// domains of at most 2048 tiles, where it is the launch that counts (96^3
-// packing, 1382 tiles: 0.0097 ms per step against 0.0104; 128^3, 3274 tiles:
-// 0.0185 both; 256^3: 0.145 against 0.125).
+// Where the pair pays: the PDFs written between a tile's even and odd step have
+// to stay in L2. Up to 2/5 of L2 (50 MB) it is faster (lists, FP64, 256^3
+// packing: 25 MB 0.275 ms per step, 50 MB 0.328, two launches 0.342); where
+// more than a tenth of the tiles come later than that (lists of large
+// cross-sections, numberings that put neighbours far apart) the two launches
+// stay. FP16 storage: the two launches' even step, staged for two nodes per
+// thread, is worth more than the traffic saved, so the pair is for domains of
+// at most 2048 tiles, where it is the launch that counts (96^3 packing, 1382
+// tiles: 0.0097 ms per step against 0.0104; 128^3, 3274 tiles: 0.0185 both;
+// 256^3: 0.145 against 0.125).
 constexpr int kPairF16Tiles = 2048;
+constexpr double kPairLateShare = 0.1;
 
-void schedule_pairs(Gpu* g) {
+double pair_max_lag(Gpu* g) {
+  int dev = 0, l2 = 0;
+  LBM_CK(cudaGetDevice(&dev));
+  LBM_CK(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev));
+  return 0.4 * l2 / (double)(lbm::kListTile * Q * g->elemBytes);
+}
+
+template <int R>
+void pair_upload(Gpu* g, const std::vector<lbm::PairRec<R>>& items, size_t nTiles) {
+  g->pairTiles = static_cast<uint32_t>(nTiles);
+  g->pairItems = static_cast<uint32_t>(items.size());
+  g->pairGroups = static_cast<uint32_t>((nTiles + (1u << lbm::kPairGroupShift) - 1) >> lbm::kPairGroupShift);
+  LBM_CK(cudaMalloc(&g->dPairCount, sizeof(uint32_t) * g->pairGroups));
+  LBM_CK(cudaMemset(g->dPairCount, 0, sizeof(uint32_t) * g->pairGroups));
+  LBM_CK(cudaMalloc(&g->dPairItems, sizeof(lbm::PairRec<R>) * items.size()));
+  LBM_CK(cudaMemcpy(g->dPairItems, items.data(), sizeof(lbm::PairRec<R>) * items.size(), cudaMemcpyHostToDevice));
+}
+
+void schedule_list_pairs(Gpu* g) {
   const int nTiles = (g->nFluid + lbm::kListTile - 1) / lbm::kListTile;
   if (nTiles == 0 || (g->storage == lbm::kStoreF16 && nTiles > kPairF16Tiles)) return;
   uint32_t* dReach = nullptr;
@@ -682,17 +717,57 @@ void schedule_pairs(Gpu* g) {
   const int resident = lbm::list_pair_resident(g->storage);
   const int margin = g->storage == lbm::kStoreF64 ? resident : resident * 3 / 2;
   std::vector<lbm::PairItem> items;
-  const long long lead = lbm::pair_schedule(reach.data(), off.data(), nTiles, margin, items);
-  int dev = 0, l2 = 0;
-  LBM_CK(cudaGetDevice(&dev));
-  LBM_CK(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev));
-  if (lead * lbm::kListTile * Q * (long long)g->elemBytes > (long long)l2 * 2 / 5) return;
-  g->pairGroups = static_cast<uint32_t>((nTiles + (1 << lbm::kPairGroupShift) - 1) >> lbm::kPairGroupShift);
-  LBM_CK(cudaMalloc(&g->dPairCount, sizeof(uint32_t) * g->pairGroups));
-  LBM_CK(cudaMemset(g->dPairCount, 0, sizeof(uint32_t) * g->pairGroups));
-  LBM_CK(cudaMalloc(&g->dPairItems, sizeof(lbm::PairItem) * items.size()));
-  LBM_CK(cudaMemcpy(g->dPairItems, items.data(), sizeof(lbm::PairItem) * items.size(), cudaMemcpyHostToDevice));
-  g->pairItems = static_cast<uint32_t>(items.size());
+  if (lbm::pair_schedule(reach.data(), off.data(), nTiles, margin, pair_max_lag(g), items) > kPairLateShare) return;
+  pair_upload(g, items, (size_t)nTiles);
+}
+
+void schedule_aa_pairs(Gpu* g, const LatticeDesc* ld) {
+  const lbm::AaArgs a = aa_args(g);
+  g->pairGeom = lbm::aa_pair_geom(a);
+  std::vector<lbm::AaPairItem> items;
+  lbm::aa_pair_schedule(a, g->pairGeom, lbm::aa_pair_resident(), items);
+  // a link of a fluid cell on a non-periodic face leaves into the ghost layer
+  const int* n = g->dims;
+  for (int axis = 0; axis < 3 && !g->openFaces; ++axis) {
+    if (g->per[axis]) continue;
+    const int u = (axis + 1) % 3, v = (axis + 2) % 3;
+    int p[3];
+    for (int side = 0; side < 2; ++side)
+      for (p[u] = 0; p[u] < n[u]; ++p[u])
+        for (p[v] = 0; p[v] < n[v]; ++p[v]) {
+          p[axis] = side ? n[axis] - 1 : 0;
+          g->openFaces |= ld->Lattice[lbmh_lidx(n, p[0], p[1], p[2])] != LAT_CELL_OBSTACLE;
+        }
+  }
+  pair_upload(g, items, (size_t)g->pairGeom.tpp * g->pairGeom.nX);
+}
+
+// The interior work items of the AA odd step by itself (slabs), from the link
+// words.
+void build_odd_items(Gpu* g, const uint32_t* link) {
+  g->oddItemsBuilt = true;
+  const lbm::AaArgs aa = aa_args(g);
+  if (lbm::aa_interior_block_count(aa) <= 0) return;
+  std::vector<int> items, cells;
+  lbm::aa_interior_items(aa, link, items, cells);
+  g->nOddItems = (int)items.size();
+  if (!items.empty()) {
+    LBM_CK(cudaMalloc(&g->dOddItems, sizeof(int) * items.size()));
+    LBM_CK(cudaMemcpy(g->dOddItems, items.data(), sizeof(int) * items.size(), cudaMemcpyHostToDevice));
+  }
+  if (!cells.empty()) {
+    LBM_CK(cudaMalloc(&g->dOddCells, sizeof(int) * cells.size()));
+    LBM_CK(cudaMemcpy(g->dOddCells, cells.data(), sizeof(int) * cells.size(), cudaMemcpyHostToDevice));
+  }
+}
+
+// The slab entry points also step a whole full-array AA instance half by half;
+// it gets its work items on the first such call.
+void need_odd_items(Gpu* g) {
+  if (g->kind != kAa || g->oddItemsBuilt) return;
+  std::vector<uint32_t> link((size_t)g->dstride);
+  LBM_CK(cudaMemcpy(link.data(), g->dLink, sizeof(uint32_t) * link.size(), cudaMemcpyDeviceToHost));
+  build_odd_items(g, link.data());
 }
 
 // --- Init / Deinit ----------------------------------------------------------------
@@ -789,21 +864,8 @@ Gpu* gpu_new(Kind kind, LatticeDesc* ld, Parameters* params, const SlabSpec* sla
       LBM_CK(cudaMalloc(&g->dG, sizeof(double) * g->mirrorElems));
       LBM_CK(cudaMemset(g->dG, 0, sizeof(double) * g->mirrorElems));
     }
-    // the AA odd step's interior work items
-    const lbm::AaArgs aa = aa_args(g);
-    if (kind == kAa && lbm::aa_interior_block_count(aa) > 0) {
-      std::vector<int> items, cells;
-      lbm::aa_interior_items(aa, link, items, cells);
-      g->nOddItems = (int)items.size();
-      if (!items.empty()) {
-        LBM_CK(cudaMalloc(&g->dOddItems, sizeof(int) * items.size()));
-        LBM_CK(cudaMemcpy(g->dOddItems, items.data(), sizeof(int) * items.size(), cudaMemcpyHostToDevice));
-      }
-      if (!cells.empty()) {
-        LBM_CK(cudaMalloc(&g->dOddCells, sizeof(int) * cells.size()));
-        LBM_CK(cudaMemcpy(g->dOddCells, cells.data(), sizeof(int) * cells.size(), cudaMemcpyHostToDevice));
-      }
-    }
+    if (kind == kAa && !slab) schedule_aa_pairs(g, ld);
+    if (kind == kAa && slab) build_odd_items(g, link);
     std::free(link);
   } else {
     const bool pull = kind == kListPull || kind == kListPullPlain;
@@ -874,7 +936,7 @@ Gpu* gpu_new(Kind kind, LatticeDesc* ld, Parameters* params, const SlabSpec* sla
         std::exit(1);
       }
     }
-    if (kind == kListAa && !g->listSlab) schedule_pairs(g);
+    if (kind == kListAa && !g->listSlab) schedule_list_pairs(g);
     g->mirrorElems = (size_t)Q * nCells;
     LBM_CK(cudaMalloc(&g->dF, g->elemBytes * g->mirrorElems));
     LBM_CK(cudaMemset(g->dF, 0, g->elemBytes * g->mirrorElems));
@@ -1427,6 +1489,7 @@ int lbm_aa_slab_step(KernelData* kd, CaseData* cd, int half, void* stream) {
     }
     return (int)cudaGetLastError();
   }
+  need_odd_items(g);
   const lbm::AaArgs a = aa_args(g);
   if (half == 0) {
     lbm::aa_even_fp64(a, t, s);
@@ -1514,6 +1577,7 @@ int lbm_aa_slab_odd_part(KernelData* kd, CaseData* cd, int part, void* stream) {
         lbm::list_odd_fp64_tiles(list_args(g), t, t0, t1, s);
     }
   } else {
+    need_odd_items(g);
     const lbm::AaArgs a = aa_args(g);
     if (part == 0) {
       // the interior blocks read and write only the slab's own planes

@@ -1,6 +1,7 @@
 // lbm_kernels.cuh -- argument blocks and launchers of the sm_100a D3Q19 TRT
 // time-step kernels (definitions in lbm_kernels_fp64.cu).
 #pragma once
+#include <algorithm>
 #include <atomic>
 #include <cstddef>
 #include <cstdint>
@@ -48,6 +49,7 @@ struct AaArgs {
   // also the lattice's periodic x boundary. All 0 for a whole lattice.
   int haloLo, haloHi, crossLo, crossHi;
   int xBase;  // even step: first x plane of the launch (grid z = planes launched)
+  int* err;   // device error word (fused pair: bounded waits)
 };
 
 // x-slab halo exchange (lbm_kernels_fp64.cu). A message is the 5 PDFs that
@@ -158,32 +160,32 @@ void slot_scatter(void* f, const uint32_t* idx, long long n, const void* buf, in
 int list_runs_device(const uint32_t* adj, int nFluid, cudaStream_t s, uint32_t** runs, uint32_t** runOff,
                      size_t* runBytes);
 
-// Fused list AA step pairs (lbm_pair.cuh): one launch runs the even and the
-// odd step. Item k: the even step of tile k (k < nTiles), then the odd step
-// of the tile that the record names, once the groups of 2^kPairGroupShift even
-// tiles that its links reach are complete: up to three ranges [lo, lo + n) of
-// groups (links with c_x = -1, 0, +1).
+// Fused AA step pairs (lbm_pair.cuh): one launch runs the even and the odd
+// step. Item k: the even step of the k-th tile in even order (k < nTiles), then
+// the odd step of the tile that the record names, once the even tiles that
+// its links reach are complete: up to R ranges [lo, lo + n) of groups of
+// 2^kPairGroupShift tiles consecutive in even order.
 constexpr int kPairGroupShift = 3;
-struct PairItem {
-  uint32_t tile;   // tile of the odd step, or kPairNone
-  uint32_t run;    // its run record, 16-byte units into the records
-  uint32_t run16;  // its size, 16-byte units
-  uint32_t lo[3], n[3];
-  uint32_t aheadRun, aheadRun16;  // run record of the item kPairAhead later (0: none)
-  uint32_t pad;
-};
 constexpr uint32_t kPairNone = 0xffffffffu;
 constexpr uint32_t kPairAhead = 512;  // about a wave of resident blocks
-constexpr int kPairItemWords = static_cast<int>(sizeof(PairItem) / 4);
-static_assert(sizeof(PairItem) == 48, "item records are loaded as 12 words");
-
+template <int R>
+struct PairRec {
+  uint32_t tile;   // tile of the odd step, or kPairNone
+  uint32_t extra;  // full array: the tile's x plane
+  uint32_t run;    // what the block stages into shared memory for it (run record / cell list):
+  uint32_t run16;  // offset and size in 16-byte units (size 0: nothing)
+  uint32_t aheadRun, aheadRun16;  // the same of the item kPairAhead later
+  uint32_t lo[R], n[R];
+};
+using PairItem = PairRec<3>;  // lists: tiles reached by links with c_x = -1, 0, +1
+template <int R>
 struct PairArgs {
-  const PairItem* items;  // nItems records
-  uint32_t* count;        // even tiles done per group, summed over all launches
-  uint32_t nItems;        // blocks of the launch
+  const PairRec<R>* items;  // nItems records
+  uint32_t* count;          // even tiles done per group, summed over all launches
+  uint32_t nItems;          // blocks of the launch
   uint32_t nTiles;
-  uint32_t epoch;         // launches including this one (counter targets)
-  int prefetch;           // as ListArgs::prefetch (0: none)
+  uint32_t epoch;           // launches including this one (counter targets)
+  int prefetch;             // as ListArgs::prefetch (0: none)
 };
 
 // Tiles that each tile's links reach (device; 6 words per tile: the lowest
@@ -191,15 +193,51 @@ struct PairArgs {
 // none), for the nFluid nodes of adj.
 void list_tile_reach(const uint32_t* adj, int nFluid, long long nCells, uint32_t* reach, cudaStream_t s);
 // Host: the item records of a fused pair from the tiles' reach and the run
-// records' offsets (nTiles + 1). Every odd step comes at least `margin` items
-// after the last even tile it needs, or after all of them. Returns the items
-// between a tile's even and its odd step (the lead of the even steps).
-long long pair_schedule(const uint32_t* reach, const uint32_t* runOff, int nTiles, int margin,
-                        std::vector<PairItem>& items);
+// records' offsets (nTiles + 1); see pair_order.
+double pair_schedule(const uint32_t* reach, const uint32_t* runOff, int nTiles, int margin, double maxLag,
+                     std::vector<PairItem>& items);
+
+// Host: the odd steps `work` (any order; need[i] = the last position in even
+// order that work[i] depends on, home[i] = its own tile's position) as item
+// records: each odd step follows the last even tile it needs by at least
+// `margin` items (or by all of them) and takes the first free item from there
+// on. Returns the share of the odd steps that come more than maxLag items
+// after their own tile's even step (whose PDFs may have left L2 by then).
+template <int R>
+double pair_order(const std::vector<PairRec<R>>& work, const std::vector<uint32_t>& need,
+                  const std::vector<uint32_t>& home, size_t nTiles, size_t margin, double maxLag,
+                  std::vector<PairRec<R>>& items) {
+  // counting sort by need, stable: nearly the tile order, except for tiles
+  // that need far later ones (the first x plane of a periodic lattice)
+  std::vector<uint32_t> first(nTiles + 1, 0), order(work.size());
+  for (uint32_t m : need) ++first[m + 1];
+  for (size_t t = 0; t < nTiles; ++t) first[t + 1] += first[t];
+  for (size_t i = 0; i < work.size(); ++i) order[first[need[i]]++] = static_cast<uint32_t>(i);
+  PairRec<R> none{};
+  none.tile = kPairNone;
+  items.clear();
+  items.reserve(nTiles + work.size() / 8 + margin);
+  size_t o = 0, late = 0;
+  for (size_t k = 0; k < nTiles || o < order.size(); ++k) {
+    if (o < order.size() && (k >= nTiles || need[order[o]] + margin <= k)) {
+      const size_t i = order[o++];
+      items.push_back(work[i]);
+      late += static_cast<double>(std::min(k, nTiles)) - home[i] > maxLag;
+    } else {
+      items.push_back(none);
+    }
+  }
+  for (size_t k = 0; k + kPairAhead < items.size(); ++k) {
+    items[k].aheadRun = items[k + kPairAhead].run;
+    items[k].aheadRun16 = items[k + kPairAhead].run16;
+  }
+  return work.empty() ? 0.0 : static_cast<double>(late) / static_cast<double>(work.size());
+}
+
 // Blocks of a fused kernel that run at once on the current device.
 int list_pair_resident(int storage);
-void list_pair_fp64(const ListArgs& a, const PairArgs& p, const Trt<double>& t, cudaStream_t s);
-void list_pair_lp(const ListArgsLp& a, const PairArgs& p, const TrtW& t, int storage, cudaStream_t s);
+void list_pair_fp64(const ListArgs& a, const PairArgs<3>& p, const Trt<double>& t, cudaStream_t s);
+void list_pair_lp(const ListArgsLp& a, const PairArgs<3>& p, const TrtW& t, int storage, cudaStream_t s);
 
 // Launchers (stream-ordered, no synchronisation).
 void list_even_lp(const ListArgsLp& a, const TrtW& t, int storage, cudaStream_t s);
@@ -228,6 +266,30 @@ void aa_odd_interior_fp64(const AaArgs& a, const Trt<double>& t, const int* item
 long long aa_interior_block_count(const AaArgs& a);
 void aa_interior_items(const AaArgs& a, const uint32_t* link, std::vector<int>& items, std::vector<int>& cells);
 void aa_odd_face_fp64(const AaArgs& a, const Trt<double>& t, cudaStream_t s);
+
+// The fused pair of a whole lattice (no halo faces). Tiles: 256 consecutive
+// cells of an x plane in (y, z) order, tpp per plane; even order: strips of J
+// tiles of each plane, x by x within a strip (aa_pair_geom).
+using AaPairItem = PairRec<9>;
+struct FastDiv {  // n / d for n < 2^31 by multiplication
+  uint32_t d, mul, shift;
+};
+struct AaPairGeom {
+  uint32_t plane;          // nY * nZ
+  uint32_t tpp, J, nX;
+  FastDiv byStrip;         // / (J * nX): strip of an even position
+  FastDiv byJ, byLast;     // / J, / tiles of the last strip
+  FastDiv byZ;             // / nZ
+};
+struct AaPairArgs {
+  PairArgs<9> p;
+  AaPairGeom g;
+  int openFaces;           // a fluid cell lies on a non-periodic face
+};
+AaPairGeom aa_pair_geom(const AaArgs& a);
+void aa_pair_schedule(const AaArgs& a, const AaPairGeom& g, int margin, std::vector<AaPairItem>& items);
+int aa_pair_resident();
+void aa_pair_fp64(const AaArgs& a, const AaPairArgs& p, const Trt<double>& t, cudaStream_t s);
 bool aa_has_interior(const AaArgs& a);
 // Two-grid full-array push / pull steps (push-soa / pull-soa): every fluid
 // cell from grid a.f into grid a.g.

@@ -22,7 +22,9 @@
 // its odd step and then overwrites what they wrote with the fix-up lists
 // (src/BenchKernelD3Q19Aa.c:301-311,501-511); here periodic wraps and bounce
 // back are resolved at the load/store itself, so no fix-up pass exists.
+#include <algorithm>
 #include <atomic>
+#include <utility>
 #include <vector>
 
 #include "lbm_bulk.cuh"
@@ -340,6 +342,271 @@ __global__ void __launch_bounds__(128) k_aa_odd_face_fp64(const AaArgs a, const 
     }
   };
   trt_update(t, load, store);
+}
+
+// ---------------------------------------------------------------------------
+// The fused pair of a whole lattice (lbm_pair.cuh).
+
+// The odd step of a warp of cells of which at least one has a reversed link:
+// every address is a select between the neighbour's slot and the node's own.
+struct NoWrap {
+  __device__ __forceinline__ int operator()(int) const { return 0; }
+};
+template <class Wrap>
+__device__ __forceinline__ void aa_odd_select(const AaArgs& a, const Trt<double>& t, int c, uint32_t w,
+                                              const Wrap& wrap) {
+  double* const fb = a.f + c;
+  const int S = (int)a.dstride;
+  auto load = [&](int d) -> double {
+    if (d == DC) return fb[a.ldOff[DC]] + t.force[DC];
+    const int j = inv(d);
+    return fb[(w >> j) & 1u ? d * S : a.ldOff[d] + wrap(j)] + t.force[d];
+  };
+  auto store = [&](int d, double v) {
+    double* const fs = launder(fb);
+    if (d == DC) {
+      __stcs(fs + a.stOff[DC], v + t.force[DC]);
+      return;
+    }
+    const int j = inv(d);
+    const bool rev = (w >> d) & 1u;
+    __stcs(fs + (rev ? j * S : a.stOff[d] + wrap(d)), v + (rev ? t.force[j] : t.force[d]));
+  };
+  trt_update(t, load, store);
+}
+
+__device__ __noinline__ void aa_odd_wall_cell(const AaArgs& a, const Trt<double>& t, int c, int x, int y, int z,
+                                              uint32_t w) {
+  aa_odd_select(a, t, c, w, XyzWrap(a, x, y, z));
+}
+
+// The same on a lattice with open faces: a reversed link may also leave into
+// the ghost layer, as in the face kernel.
+__device__ __noinline__ void aa_odd_open_cell(const AaArgs& a, const Trt<double>& t, int c, int x, int y, int z,
+                                              uint32_t w) {
+  const long long S = a.dstride;
+  double* const f = a.f;
+  auto load = [&](int d) -> double {
+    if (d == DC) return f[DC * S + c] + t.force[DC];
+    const int j = inv(d);
+    const bool rev = (w >> j) & 1u;
+    const bool open = rev && aa_open(a, x, y, z, j);
+    const int nb = rev ? c + aa_off(a, j) : aa_wrapped(a, x, y, z, j);
+    return f[(rev && !open) ? d * S + c : j * S + nb] + t.force[d];
+  };
+  auto store = [&](int d, double v) {
+    if (d == DC) {
+      f[DC * S + c] = v + t.force[DC];
+      return;
+    }
+    const int j = inv(d);
+    const bool rev = (w >> d) & 1u;
+    if (!rev) {
+      f[d * S + aa_wrapped(a, x, y, z, d)] = v + t.force[d];
+    } else if (aa_open(a, x, y, z, d)) {
+      f[d * S + c + aa_off(a, d)] = v;
+      f[j * S + c] = f[j * S + c] + t.force[j];
+    } else {
+      f[j * S + c] = v + t.force[j];
+    }
+  };
+  trt_update(t, load, store);
+}
+
+__device__ __forceinline__ uint32_t fast_div(uint32_t n, const FastDiv& v) {
+  return static_cast<uint32_t>((static_cast<uint64_t>(n) * v.mul) >> v.shift);
+}
+
+// Even position k -> x plane and first cell (in plane order) of its tile.
+__device__ __forceinline__ void aa_pair_tile(const AaPairGeom& g, uint32_t k, uint32_t& x, uint32_t& cell0) {
+  const uint32_t s = fast_div(k, g.byStrip);
+  const uint32_t r = k - s * g.byStrip.d;
+  const bool last = (s + 1) * g.J >= g.tpp;
+  const uint32_t width = last ? g.byLast.d : g.J;
+  x = last ? fast_div(r, g.byLast) : fast_div(r, g.byJ);
+  cell0 = (s * g.J + r - x * width) * kListTile;
+}
+
+// One thread per cell of a tile of 256 consecutive cells of an x plane in
+// (y, z) order, so that rows of any length fill the warps (64^3, whose 64-cell
+// rows left half to three quarters of the threads of row-shaped blocks idle).
+// A warp without reversed links takes the odd step by fixed offsets and the
+// periodic wraps of its cells' positions (XyzWrap); a warp with any takes a
+// selecting path for all its cells, inline where none lies on a face of the
+// lattice (channel 203 x 190 x 197 in strips of 74 tiles: 0.307 ms per step;
+// with lists of the wall cells as a second pass 0.333, with the selecting path
+// out of line 0.360; in whole planes 0.294, two launches 0.412).
+// Even loads do not wait for the link word that says whether the cell is
+// fluid (solid cells' slots exist; nothing is stored there): 0.310 against
+// 0.319 ms on that channel, 0.189 / 0.194 at 85 % fluid cells, 0.176 / 0.174
+// at 40 %.
+// Bound by L2 requests and their latency as the list pair: 256^3 fluid box
+// 0.818 -> 0.597 ms per step (28.1 GFLUP/s, half the HBM bytes), 256^3 channel
+// 0.845 -> 0.645, 64^3 channel 0.0219 -> 0.0140.
+__global__ void __launch_bounds__(kPairThreads, 3)
+    k_aa_pair_fp64(const __grid_constant__ AaArgs a, const __grid_constant__ AaPairArgs q,
+                   const __grid_constant__ Trt<double> t) {
+  __shared__ PairShared<9, 4> sh;  // nothing staged
+  pair_init(&sh);
+  const uint32_t k = blockIdx.x;
+  if (threadIdx.x >= kListTile) {
+    pair_service(&sh, q.p, nullptr, a.err, k);
+    return;
+  }
+  if (k < q.p.nTiles) {
+    uint32_t x, i;
+    aa_pair_tile(q.g, k, x, i);
+    i += threadIdx.x;
+    if (i < q.g.plane) {
+      const uint32_t y = fast_div(i, q.g.byZ), z = i - y * q.g.byZ.d;
+      const int c = aa_cell(a, x, y, z);
+      const uint32_t w = __ldg(a.link + c);
+      const double* const f = a.f + c;
+      double* const fs = launder(a.f + c);
+      const uint64_t keep = l2_keep_policy();
+      const long long S = a.dstride;
+      trt_update(t, [&](int d) { return __ldcs(f + d * S); },
+                 [&](int d, double v) {
+                   if (w & kFluidBit) st_keep(fs + inv(d) * S, v, keep);
+                 });
+    }
+    pair_even_done(&sh);
+  }
+  if (!pair_odd_named(&sh, a.err)) return;
+  const uint32_t x = sh.item.extra, i = sh.item.tile + threadIdx.x;
+  const uint32_t y = fast_div(i, q.g.byZ), z = i - y * q.g.byZ.d;
+  const int c = aa_cell(a, x, y, z);
+  const uint32_t w = i < q.g.plane ? __ldg(a.link + c) : 0u;
+  const bool fluid = w & kFluidBit;
+  const bool wall = __any_sync(0xffffffffu, fluid && (w & kLinkBits));
+  const bool face = __any_sync(0xffffffffu, fluid && XyzWrap(a, x, y, z).m != 0u);
+  if (!pair_odd_turn(&sh, a.err) || !fluid) return;
+  if (!wall) {
+    double* const fb = a.f + c;
+    const XyzWrap wrap(a, x, y, z);
+    trt_update(t, [&](int d) -> double { return fb[a.ldOff[d] + wrap(inv(d))] + t.force[d]; },
+               [&](int d, double v) { __stcs(launder(fb) + (a.stOff[d] + wrap(d)), v + t.force[d]); });
+  } else if (!face) {
+    aa_odd_select(a, t, c, w, NoWrap());
+  } else if (!q.openFaces) {
+    aa_odd_wall_cell(a, t, c, x, y, z, w);
+  } else {
+    aa_odd_open_cell(a, t, c, x, y, z, w);
+  }
+}
+
+static FastDiv fast_div_of(uint32_t d) {
+  // ceil(log2 d) bits: exact for n < 2^31
+  uint32_t l = 0;
+  while ((1ull << l) < d) ++l;
+  return FastDiv{d, static_cast<uint32_t>((1ull << (31 + l)) / d + 1), 31 + l};
+}
+
+// Strips: an odd tile needs the tiles of the neighbouring rows in three
+// planes, so with whole planes one after the other the PDFs of two planes wait
+// in L2. Planes of more than kWholePlane tiles go in strips of about
+// kStripTiles tiles of each plane; a tile at a strip's edge needs the next
+// strip and comes late (its PDFs are read again). Measured, ms per step
+// (fluid boxes): 256 tiles per plane, whole 0.597, strips of 128 0.627, of 86
+// 0.612; 352 tiles: 0.647, 0.690 (176), 0.662 (88); 625 tiles: 0.739, 0.711
+// (209), 0.683 (90); 900: 0.770, 0.703 (225), 0.697 (90). Two launches: 0.818,
+// 0.891, 0.946, 0.893.
+constexpr uint32_t kWholePlane = 384, kStripTiles = 96;
+
+AaPairGeom aa_pair_geom(const AaArgs& a) {
+  AaPairGeom g;
+  g.plane = static_cast<uint32_t>(a.nY) * static_cast<uint32_t>(a.nZ);
+  g.tpp = (g.plane + kListTile - 1) / kListTile;
+  g.nX = static_cast<uint32_t>(a.nX);
+  // rows either side of a tile, in tiles: a strip is several times as wide
+  const uint32_t halo = (2 * static_cast<uint32_t>(a.nZ) + kListTile) / kListTile;
+  const uint32_t width = std::max(kStripTiles, 8 * halo);
+  const uint32_t strips = g.tpp <= kWholePlane ? 1 : (g.tpp + width - 1) / width;
+  g.J = (g.tpp + strips - 1) / strips;
+  const uint32_t lastStrip = (g.tpp - 1) / g.J;
+  g.byStrip = fast_div_of(g.J * g.nX);
+  g.byJ = fast_div_of(g.J);
+  g.byLast = fast_div_of(g.tpp - lastStrip * g.J);
+  g.byZ = fast_div_of(static_cast<uint32_t>(a.nZ));
+  return g;
+}
+
+void aa_pair_schedule(const AaArgs& a, const AaPairGeom& g, int margin, std::vector<AaPairItem>& items) {
+  const uint32_t nTiles = g.nX * g.tpp, lastStrip = (g.tpp - 1) / g.J;
+  auto width = [&](uint32_t s) { return s == lastStrip ? g.tpp - s * g.J : g.J; };
+  auto position = [&](uint32_t x, uint32_t j) {
+    const uint32_t s = j / g.J;
+    return s * g.J * g.nX + x * width(s) + (j - s * g.J);
+  };
+  struct Range {
+    uint32_t lo, hi;
+  };
+  std::vector<AaPairItem> work(nTiles);
+  std::vector<uint32_t> need(nTiles), home(nTiles);
+  std::vector<Range> reach, pos;
+  for (uint32_t j = 0; j < g.tpp; ++j) {
+    // tiles of a plane that the tile's cells reach in y and z, wrapping at the
+    // plane's ends whether or not a link does; a link to the row before or
+    // after may wrap in z, so up to two rows away, and split at strip ends
+    reach.clear();
+    auto add = [&](long long cell0, long long cell1) {
+      const uint32_t t0 = (uint32_t)(cell0 / kListTile), t1 = (uint32_t)(cell1 / kListTile);
+      for (uint32_t s = t0 / g.J; s <= t1 / g.J; ++s)
+        reach.push_back({std::max(t0, s * g.J), std::min(t1, s * g.J + width(s) - 1)});
+    };
+    const long long n = g.plane, i0 = (long long)j * kListTile - 2LL * a.nZ;
+    const long long i1 = std::min<long long>(n, (long long)(j + 1) * kListTile) - 1 + 2LL * a.nZ;
+    if (i1 - i0 + 1 >= n) {
+      add(0, n - 1);
+    } else {
+      add(std::max(i0, 0ll), std::min(i1, n - 1));
+      if (i0 < 0) add(n + i0, n - 1);
+      if (i1 >= n) add(0, i1 - n);
+    }
+    for (uint32_t x = 0; x < g.nX; ++x) {
+      const uint32_t t = x * g.tpp + j;
+      AaPairItem& it = work[t];
+      it = AaPairItem{};
+      it.tile = j * kListTile;
+      it.extra = x;
+      home[t] = position(x, j);
+      pos.clear();
+      for (uint32_t dx = 0; dx < 3; ++dx) {
+        const uint32_t px = (x + g.nX + dx - 1) % g.nX;
+        for (const Range& v : reach) {
+          pos.push_back({position(px, v.lo) >> kPairGroupShift, position(px, v.hi) >> kPairGroupShift});
+          need[t] = std::max(need[t], position(px, v.hi));
+        }
+      }
+      std::sort(pos.begin(), pos.end(), [](const Range& u, const Range& v) { return u.lo < v.lo; });
+      size_t m = 0;
+      for (const Range& v : pos) {
+        if (m && v.lo <= pos[m - 1].hi + 1)
+          pos[m - 1].hi = std::max(pos[m - 1].hi, v.hi);
+        else
+          pos[m++] = v;
+      }
+      if (m > 9) {  // more pieces than a record holds: wait for every even tile
+        m = 1;
+        pos[0] = {0, (nTiles - 1) >> kPairGroupShift};
+        need[t] = nTiles - 1;
+      }
+      for (size_t r = 0; r < m; ++r) {
+        it.lo[r] = pos[r].lo;
+        it.n[r] = pos[r].hi - pos[r].lo + 1;
+      }
+    }
+  }
+  pair_order(work, need, home, nTiles, static_cast<size_t>(margin), 0.0, items);
+}
+
+int aa_pair_resident() {
+  static std::atomic<int> n{0};
+  return prefetch_distance(n, k_aa_pair_fp64, kPairThreads, true);
+}
+
+void aa_pair_fp64(const AaArgs& a, const AaPairArgs& q, const Trt<double>& t, cudaStream_t s) {
+  if (q.p.nItems > 0) k_aa_pair_fp64<<<q.p.nItems, kPairThreads, 0, s>>>(a, q, t);
 }
 
 // ---------------------------------------------------------------------------
@@ -684,9 +951,9 @@ __global__ void __launch_bounds__(kListTile, 3) k_list_odd_fp64(const ListArgs a
 // scatters touch 1.2-1.5 sectors per sector of payload; without any waiting
 // the 256^3 packing would take 0.247 ms per step), then the waits.
 __global__ void __launch_bounds__(kPairThreads, 3)
-    k_list_pair_fp64(const __grid_constant__ ListArgs a, const __grid_constant__ PairArgs p,
+    k_list_pair_fp64(const __grid_constant__ ListArgs a, const __grid_constant__ PairArgs<3> p,
                      const __grid_constant__ Trt<double> t) {
-  __shared__ PairShared sh;
+  __shared__ ListPairShared sh;
   pair_init(&sh);
   const uint32_t k = blockIdx.x;
   if (threadIdx.x >= kListTile) {
@@ -850,7 +1117,7 @@ void list_odd_fp64_tiles(const ListArgs& a, const Trt<double>& t, int t0, int t1
   b.prefetch = prefetch_distance(g_oddAhead, k_list_odd_fp64, kListTile, a.prefetch != 0);
   k_list_odd_fp64<<<(unsigned)(t1 - t0), kListTile, 0, s>>>(b, t);
 }
-void list_pair_fp64(const ListArgs& a, const PairArgs& p, const Trt<double>& t, cudaStream_t s) {
+void list_pair_fp64(const ListArgs& a, const PairArgs<3>& p, const Trt<double>& t, cudaStream_t s) {
   if (p.nItems > 0) k_list_pair_fp64<<<p.nItems, kPairThreads, 0, s>>>(a, p, t);
 }
 int list_pair_resident_fp64() {

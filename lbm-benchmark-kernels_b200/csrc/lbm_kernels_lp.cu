@@ -136,9 +136,9 @@ __global__ void __launch_bounds__(kListTile, LBM_LP_ODD_BLOCKS) k_list_odd_lp(co
 // 0.173 ms per step; two launches 0.185).
 template <class St>
 __global__ void __launch_bounds__(kPairThreads, 5)
-    k_list_pair_lp(const __grid_constant__ ListArgsLp a, const __grid_constant__ PairArgs p,
+    k_list_pair_lp(const __grid_constant__ ListArgsLp a, const __grid_constant__ PairArgs<3> p,
                    const __grid_constant__ TrtW w) {
-  __shared__ PairShared sh;
+  __shared__ ListPairShared sh;
   pair_init(&sh);
   const uint32_t k = blockIdx.x;
   if (threadIdx.x >= kListTile) {
@@ -160,7 +160,7 @@ __global__ void __launch_bounds__(kPairThreads, 5)
   lp_odd_node<St, true, PairAccess>(static_cast<T*>(a.f), static_cast<uint32_t>(a.nCells), n, e, off, t);
 }
 
-void list_pair_lp(const ListArgsLp& a, const PairArgs& p, const TrtW& t, int storage, cudaStream_t s) {
+void list_pair_lp(const ListArgsLp& a, const PairArgs<3>& p, const TrtW& t, int storage, cudaStream_t s) {
   if (p.nItems == 0) return;
   if (storage == kStoreF16)
     k_list_pair_lp<StoreF16><<<p.nItems, kPairThreads, 0, s>>>(a, p, t);

@@ -1,14 +1,14 @@
-// lbm_pair.cuh -- the even and the odd step of a list AA pair in one launch,
-// the odd step trailing the even one closely enough that it finds the PDFs in
-// L2 (shared by the FP64, the reduced-storage and the batched kernels).
+// lbm_pair.cuh -- the even and the odd step of an AA pair in one launch, the
+// odd step trailing the even one closely enough that it finds the PDFs in L2
+// (the list rows in FP64 and reduced storage, and the full-array row).
 //
 // What bounds the two-launch pair: each step streams all PDFs through HBM
 // (304 B per FP64 node and step). The odd step of a tile needs the even step
-// of the tiles its links reach and of no others: with the blocked x-y-z
-// numbering these lie within one x plane on either side. So block k of the
-// fused launch runs the even step of tile k and then the odd step of a tile
-// about two planes back, whose PDFs the even step wrote a few microseconds
-// earlier: HBM is read once and written once per pair.
+// of the tiles its links reach and of no others: with the x-y-z numbering
+// these lie within one x plane on either side. So block k of the fused launch
+// runs the even step of tile k and then the odd step of a tile about two
+// planes back, whose PDFs the even step wrote a few microseconds earlier: HBM
+// is read once and written once per pair.
 //
 // Order and waiting. Even steps wait for nothing. An odd step waits until the
 // groups of even tiles its links reach are complete (counters in device
@@ -67,17 +67,22 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
   asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
 }
 
-// What a block shares: the odd tile's run record, its item, and the two
-// hand-overs between the service warp and the compute warps.
+// What a block shares: what its odd item stages (kWords words), the item, and
+// the hand-overs between the service warp and the compute warps.
+template <int R, int kWords>
 struct PairShared {
-  alignas(128) uint32_t run[kRunTileWords];
-  alignas(16) PairItem item;
-  alignas(8) uint64_t go;    // the odd step may start: dependencies met, run record here
-  alignas(8) uint64_t even;  // every compute warp has stored its even nodes
+  alignas(128) uint32_t run[kWords];
+  alignas(16) PairRec<R> item;
+  alignas(8) uint64_t named;  // the item is here
+  alignas(8) uint64_t go;     // the odd step may start: dependencies met, staged data here
+  alignas(8) uint64_t even;   // every compute warp has stored its even nodes
 };
+using ListPairShared = PairShared<3, kRunTileWords>;
 
-__device__ __forceinline__ void pair_init(PairShared* sh) {
+template <int R, int kWords>
+__device__ __forceinline__ void pair_init(PairShared<R, kWords>* sh) {
   if (threadIdx.x == kListTile) {
+    mbar_init(&sh->named, 1);
     mbar_init(&sh->go, 1);
     mbar_init(&sh->even, kListTile / 32);
   }
@@ -86,34 +91,52 @@ __device__ __forceinline__ void pair_init(PairShared* sh) {
 
 // One look (by the whole warp) at the even groups the item depends on:
 // whether all are complete. Counters and targets are compared modulo 2^32.
-__device__ __forceinline__ bool pair_ready(const PairItem& it, const PairArgs& p) {
-  const uint32_t n0 = it.n[0], n01 = n0 + it.n[1], all = n01 + it.n[2];
+template <int R>
+__device__ __forceinline__ bool pair_ready(const PairRec<R>& it, const PairArgs<R>& p) {
+  uint32_t all = 0;
+#pragma unroll
+  for (int r = 0; r < R; ++r) all += it.n[r];
   bool good = true;
   for (uint32_t i = threadIdx.x & 31; i < all; i += 32) {
-    const uint32_t g = i < n0 ? it.lo[0] + i : (i < n01 ? it.lo[1] + (i - n0) : it.lo[2] + (i - n01));
+    uint32_t g = 0, j = i;
+    bool found = false;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      if (!found && j < it.n[r]) {
+        g = it.lo[r] + j;
+        found = true;
+      }
+      j -= it.n[r];
+    }
     const uint32_t size = min(p.nTiles - (g << kPairGroupShift), 1u << kPairGroupShift);
     good = good && static_cast<int32_t>(ld_acquire(p.count + g) - p.epoch * size) >= 0;
   }
   return __all_sync(0xffffffffu, good);
 }
 
-// The service warp of block k (see above).
-__device__ __forceinline__ void pair_service(PairShared* sh, const PairArgs& p, const uint32_t* runs, int* err,
-                                             uint32_t k) {
+// The service warp of block k (see above); runs: the array that the items'
+// staged data lies in.
+template <int R, int kWords>
+__device__ __forceinline__ void pair_service(PairShared<R, kWords>* sh, const PairArgs<R>& p, const void* runs,
+                                             int* err, uint32_t k) {
+  constexpr int kItemWords = static_cast<int>(sizeof(PairRec<R>) / 4);
+  static_assert(kItemWords <= 32, "one item word per lane");
   const int lane = threadIdx.x - kListTile;
   const bool even = k < p.nTiles;
-  if (lane < kPairItemWords)
+  if (lane < kItemWords)
     reinterpret_cast<uint32_t*>(&sh->item)[lane] = __ldg(reinterpret_cast<const uint32_t*>(p.items + k) + lane);
   __syncwarp();
-  const PairItem& it = sh->item;
+  const PairRec<R>& it = sh->item;
+  const char* const base = static_cast<const char*>(runs);
   if (lane == 0) {
-    if (it.tile != kPairNone) {
+    mbar_arrive(&sh->named);
+    if (it.tile != kPairNone && it.run16) {
       mbar_expect_tx(&sh->go, it.run16 * 16u);
-      bulk_g2s(sh->run, runs + static_cast<size_t>(it.run) * 4, it.run16 * 16u, &sh->go);
+      bulk_g2s(sh->run, base + static_cast<size_t>(it.run) * 16, it.run16 * 16u, &sh->go);
     }
     if (p.prefetch) {
-      // the record and the item of blocks that have not started yet, into L2
-      if (it.aheadRun16) bulk_prefetch_l2(runs + static_cast<size_t>(it.aheadRun) * 4, it.aheadRun16 * 16u);
+      // the staged data and the item of blocks that have not started yet, into L2
+      if (it.aheadRun16) bulk_prefetch_l2(base + static_cast<size_t>(it.aheadRun) * 16, it.aheadRun16 * 16u);
       if (k + 2 * kPairAhead < p.nItems) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.items + k + 2 * kPairAhead));
     }
   }
@@ -136,13 +159,25 @@ __device__ __forceinline__ void pair_service(PairShared* sh, const PairArgs& p, 
 }
 
 // Compute warps: their even nodes are stored.
-__device__ __forceinline__ void pair_even_done(PairShared* sh) {
+template <class Sh>
+__device__ __forceinline__ void pair_even_done(Sh* sh) {
   __syncwarp();
   if ((threadIdx.x & 31) == 0) mbar_arrive(&sh->even);
 }
 
+// Compute warps: waits for the item; false if it names no odd step.
+template <class Sh>
+__device__ __forceinline__ bool pair_odd_named(Sh* sh, int* err) {
+  if (!mbar_wait_bounded(&sh->named, 0)) {
+    atomicOr(err, 1);
+    return false;
+  }
+  return sh->item.tile != kPairNone;
+}
+
 // Compute warps: waits for the odd step's turn; false if there is none.
-__device__ __forceinline__ bool pair_odd_turn(PairShared* sh, int* err) {
+template <class Sh>
+__device__ __forceinline__ bool pair_odd_turn(Sh* sh, int* err) {
   if (!mbar_wait_bounded(&sh->go, 0)) {
     atomicOr(err, 1);
     return false;

@@ -1,4 +1,4 @@
-"""The fused even/odd launch of the list AA rows (csrc/lbm_pair.cuh) where it
+"""The fused even/odd launch of the AA rows (csrc/lbm_pair.cuh) where it
 has to wait: lattices with more tiles than the lead of the even steps, so that
 blocks run the even step of one tile and the odd step of another while the
 steps they depend on are still under way. Small lattices, whose odd steps all
@@ -50,3 +50,64 @@ def test_fused_pairs_equal_separate_steps(make, kargs):
     got = _run_slabs(lat, 2, init, cd, 4, layout="list", kargs=kargs)
     m = lat.mask != 0
     assert np.array_equal(got[m], whole[m])
+
+
+AA_CASES = [
+    (lambda: lbmb200.geometry("fluid", (40, 61, 59), (1, 1, 1))),
+    (lambda: lbmb200.geometry("channel", (45, 70, 64), (1, 0, 0))),
+    (lambda: lbmb200.geometry("channel", (70, 50, 49), (0, 0, 0))),   # open x faces
+    (lambda: lbmb200.geometry("fluid", (30, 66, 67), (0, 1, 0))),     # open and periodic faces
+    (lambda: _spheres((60, 47, 53), 0.5)),
+    # planes in strips, with and without tiles that need the next strip through a periodic face
+    (lambda: lbmb200.geometry("fluid", (9, 330, 310), (1, 1, 1))),
+    (lambda: lbmb200.geometry("channel", (10, 317, 331), (1, 0, 0))),
+    # rows longer than a tile, planes of one tile
+    (lambda: lbmb200.geometry("fluid", (5, 150, 700), (1, 0, 1))),
+    (lambda: lbmb200.geometry("fluid", (900, 11, 13), (1, 1, 1))),
+]
+
+
+@pytest.mark.parametrize("make", AA_CASES)
+def test_fused_full_array_pairs_equal_separate_steps(make):
+    lat = make()
+    init = random_pdfs(lat.mask.size, 59)
+    cd = lbmb200.case(omega=1.2, xforce=2e-4, iterations=8)
+    inst = lbmb200.kernel("cuda-aa-soa").init(lat, kernel_args=["-lambda", "3/16"])
+    try:
+        assert inst.launches_for(2) == 1 and inst.launches_for(7) == 4
+        inst.set_field(init)
+        inst.run(cd)
+        whole = inst.get_field()
+    finally:
+        inst.deinit()
+    got = _run_slabs(lat, 2, init, cd, 4)
+    m = lat.mask != 0
+    assert np.array_equal(got[m], whole[m])
+
+
+def test_slab_steps_on_a_whole_lattice():
+    """The slab entry points step a whole-lattice instance half by half; fused
+    pairs before and after them continue the same run."""
+    import ctypes
+    lat = lbmb200.geometry("blocks-4", (30, 26, 25), (1, 1, 1))
+    init = random_pdfs(lat.mask.size, 61)
+    cd = lbmb200.case(omega=1.1, xforce=2e-4, iterations=4)
+    fields = []
+    L = lbmb200.lib()
+    for halves in (False, True):
+        inst = lbmb200.kernel("cuda-aa-soa").init(lat, kernel_args=["-lambda", "3/16"])
+        try:
+            inst.set_field(init)
+            inst.run(cd)
+            if halves:
+                for half in (0, 1, 0, 1):
+                    assert L.lbm_aa_slab_step(inst.kdp, ctypes.byref(cd), half, None) == 0
+                inst.sync_mirror()
+            else:
+                inst.run(cd)
+            inst.run(cd)
+            fields.append(inst.get_field())
+        finally:
+            inst.deinit()
+    m = lat.mask != 0
+    assert np.array_equal(fields[0][m], fields[1][m])
