@@ -9,6 +9,7 @@
 // already in flight.
 #include "lbm_batch.cuh"
 #include "lbm_bulk.cuh"
+#include "lbm_chain.cuh"
 #include "lbm_store.cuh"
 
 namespace lbm {
@@ -35,8 +36,12 @@ __device__ __forceinline__ void batch_even_node(const BatchTile& T, int n) {
 template <class St>
 __global__ void __launch_bounds__(256) k_batch_even(const BatchArgs a) {
   __shared__ __align__(16) BatchTile st[2];
-  const int nT = *a.nTiles;
-  if (static_cast<int>(blockIdx.x) >= nT) return;
+  chain_next();
+  const int nT = *a.nTiles;  // the tables do not change between chained steps
+  if (static_cast<int>(blockIdx.x) >= nT) {
+    chain_wait();
+    return;
+  }
   const bool warp0 = threadIdx.x < 32;
   uint32_t r = 0;
   if (warp0) {
@@ -44,6 +49,7 @@ __global__ void __launch_bounds__(256) k_batch_even(const BatchArgs a) {
     tile_store(&st[0], r);
     if (static_cast<int>(blockIdx.x + gridDim.x) < nT) r = tile_load(a.tiles, blockIdx.x + gridDim.x);
   }
+  chain_wait();
   int it = 0;
   for (int tile = blockIdx.x; tile < nT; tile += gridDim.x, ++it) {
     const int buf = it & 1;
@@ -84,8 +90,12 @@ __global__ void __launch_bounds__(256) k_batch_odd(const BatchArgs a) {
   extern __shared__ __align__(128) uint32_t sadj[];  // 2 x kRunTileWords
   __shared__ alignas(8) uint64_t bar[2];
   __shared__ __align__(16) BatchTile st[2];
-  const int nT = *a.nTiles;
-  if (static_cast<int>(blockIdx.x) >= nT) return;
+  chain_next();
+  const int nT = *a.nTiles;  // the tables do not change between chained steps
+  if (static_cast<int>(blockIdx.x) >= nT) {
+    chain_wait();
+    return;
+  }
   const bool warp0 = threadIdx.x < 32;
   uint32_t r = 0;
   auto issue = [&](int buf) {  // thread 0, once st[buf] holds the tile's record
@@ -111,6 +121,7 @@ __global__ void __launch_bounds__(256) k_batch_odd(const BatchArgs a) {
     }
     if (static_cast<int>(blockIdx.x + gridDim.x) < nT) r = tile_load(a.tiles, blockIdx.x + gridDim.x);
   }
+  chain_wait();
   int it = 0;
   for (int tile = blockIdx.x; tile < nT; tile += gridDim.x, ++it) {
     const int buf = it & 1;
@@ -147,9 +158,14 @@ __global__ void __launch_bounds__(256) k_batch_odd(const BatchArgs a) {
 template <class St, int NPT>
 __global__ void __launch_bounds__(kBatchTileNodes / NPT) k_batch_even_tile(const BatchArgs a) {
   __shared__ __align__(16) BatchTile st;
-  if (static_cast<int>(blockIdx.x) >= *a.nTiles) return;
+  chain_next();
+  if (static_cast<int>(blockIdx.x) >= *a.nTiles) {
+    chain_wait();
+    return;
+  }
   if (threadIdx.x < 32) tile_store(&st, tile_load(a.tiles, blockIdx.x));
   __syncthreads();
+  chain_wait();
 #pragma unroll 1
   for (int k = 0; k < NPT; ++k) {
     const int local = threadIdx.x + k * (kBatchTileNodes / NPT);
@@ -164,7 +180,11 @@ __global__ void __launch_bounds__(kBatchTileNodes / NPT, 6 * NPT) k_batch_odd_ti
   __shared__ __align__(128) uint32_t srun[kRunTileWords];
   __shared__ alignas(8) uint64_t bar;
   __shared__ __align__(16) BatchTile st;
-  if (static_cast<int>(blockIdx.x) >= *a.nTiles) return;
+  chain_next();
+  if (static_cast<int>(blockIdx.x) >= *a.nTiles) {
+    chain_wait();
+    return;
+  }
   if (threadIdx.x < 32) {
     tile_store(&st, tile_load(a.tiles, blockIdx.x));
     __syncwarp();
@@ -179,6 +199,7 @@ __global__ void __launch_bounds__(kBatchTileNodes / NPT, 6 * NPT) k_batch_odd_ti
     }
   }
   __syncthreads();
+  chain_wait();
   if (!run_bytes_ok(st.runBytes)) return;
   if (!mbar_wait_bounded(&bar, 0)) {
     if (threadIdx.x == 0) atomicOr(a.err, 1);
@@ -194,25 +215,25 @@ __global__ void __launch_bounds__(kBatchTileNodes / NPT, 6 * NPT) k_batch_odd_ti
 template <class St>
 static void launch_even(const BatchArgs& a, const BatchLaunch& l, int grid, cudaStream_t s) {
   if (l.blocks > 0)
-    k_batch_even<St><<<grid, l.threads, 0, s>>>(a);
+    launch_chained(k_batch_even<St>, grid, l.threads, 0, s, a);
   else if (l.nodesPerThread == 4)
-    k_batch_even_tile<St, 4><<<grid, kBatchTileNodes / 4, 0, s>>>(a);
+    launch_chained(k_batch_even_tile<St, 4>, grid, kBatchTileNodes / 4, 0, s, a);
   else if (l.nodesPerThread == 2)
-    k_batch_even_tile<St, 2><<<grid, kBatchTileNodes / 2, 0, s>>>(a);
+    launch_chained(k_batch_even_tile<St, 2>, grid, kBatchTileNodes / 2, 0, s, a);
   else
-    k_batch_even_tile<St, 1><<<grid, kBatchTileNodes, 0, s>>>(a);
+    launch_chained(k_batch_even_tile<St, 1>, grid, kBatchTileNodes, 0, s, a);
 }
 
 template <class St>
 static void launch_odd(const BatchArgs& a, const BatchLaunch& l, int grid, cudaStream_t s) {
   if (l.blocks > 0)
-    k_batch_odd<St><<<grid, l.threads, 2 * (size_t)kRunRecordMax, s>>>(a);
+    launch_chained(k_batch_odd<St>, grid, l.threads, 2 * (size_t)kRunRecordMax, s, a);
   else if (l.nodesPerThread == 4)
-    k_batch_odd_tile<St, 4><<<grid, kBatchTileNodes / 4, 0, s>>>(a);
+    launch_chained(k_batch_odd_tile<St, 4>, grid, kBatchTileNodes / 4, 0, s, a);
   else if (l.nodesPerThread == 2)
-    k_batch_odd_tile<St, 2><<<grid, kBatchTileNodes / 2, 0, s>>>(a);
+    launch_chained(k_batch_odd_tile<St, 2>, grid, kBatchTileNodes / 2, 0, s, a);
   else
-    k_batch_odd_tile<St, 1><<<grid, kBatchTileNodes, 0, s>>>(a);
+    launch_chained(k_batch_odd_tile<St, 1>, grid, kBatchTileNodes, 0, s, a);
 }
 
 void batch_even_lp(const BatchArgs& a, const BatchLaunch& l, int grid, cudaStream_t s) {

@@ -6,6 +6,7 @@
 #pragma once
 #include <cstdint>
 
+#include "lbm_chain.cuh"
 #include "lbm_kernels.cuh"
 
 namespace lbm {
@@ -71,6 +72,7 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
 template <class A>
 __device__ __forceinline__ bool stage_run_tile_issue(const A& a, uint32_t* srun, uint64_t* bar, int* ok) {
   const unsigned tile = blockIdx.x + static_cast<unsigned>(a.tileBase);
+  chain_next();
   if (threadIdx.x == 0) {
     const uint32_t o0 = a.runOff[tile], o1 = a.runOff[tile + 1];
     const uint32_t bytes = (o1 - o0) * 16u;
@@ -84,6 +86,7 @@ __device__ __forceinline__ bool stage_run_tile_issue(const A& a, uint32_t* srun,
     }
   }
   __syncthreads();
+  chain_wait();  // the record never changes; everything after this may
   return *ok != 0;
 }
 

@@ -104,8 +104,10 @@ struct Gpu {
 
   // fused step pairs of an AA instance (lbm_pair.cuh; null: a launch per step)
   void* dPairItems;        // PairItem (lists) or AaPairItem (full array) records
-  uint32_t* dPairCount;
-  uint32_t pairItems, pairTiles, pairGroups, pairEpoch;
+  uint32_t* dPairCount;    // even tiles done per group, then the launch counters
+  uint32_t pairItems, pairTiles, pairGroups;
+  // small domains: many pairs in one launch (null: not small)
+  uint32_t* dMeet;
   lbm::AaPairGeom pairGeom;
   int openFaces;
 
@@ -367,12 +369,15 @@ lbm::PairArgs<R> pair_args(Gpu* g) {
   p.count = g->dPairCount;
   p.nItems = g->pairItems;
   p.nTiles = g->pairTiles;
-  p.epoch = ++g->pairEpoch;
+  p.launches = g->dPairCount + g->pairGroups;
   p.prefetch = list_prefetch_enabled();
   return p;
 }
 
 double* current_grid(Gpu* g) { return (two_grid(g->kind) && g->cur == 1) ? g->dG : g->dF; }
+
+// Pairs in one launch of a small domain at most (a few milliseconds).
+constexpr int kResidentPairs = 1024;
 
 // Enqueues n time steps (AA kernels: rounded up to whole even/odd pairs, as
 // the reference's loop `for (iter = 0; iter < n; iter += 2)`); returns the
@@ -383,7 +388,21 @@ long enqueue_steps(Gpu* g, const lbm::Trt<double>& t, int n, cudaEvent_t* ev = n
   auto mark = [&]() {
     if (ev) cudaEventRecord(ev[k], g->stream);
   };
-  if (g->kind == kAa && g->dPairItems) {
+  if (g->dMeet) {
+    for (int done = 0; done < n; done += 2 * kResidentPairs) {
+      mark();
+      const int pairs = std::min((n - done + 1) / 2, kResidentPairs);
+      const lbm::ResidentArgs r{g->dMeet, pairs};
+      if (g->kind == kAa)
+        lbm::aa_resident_fp64(aa_args(g), g->pairGeom, g->openFaces, r, t, g->stream);
+      else if (g->storage == lbm::kStoreF64)
+        lbm::list_resident_fp64(list_args(g), r, t, g->stream);
+      else
+        lbm::list_resident_lp(list_args_lp(g), r, to_trtw(t), g->storage, g->stream);
+      ++k;
+      g->iteration = done + 2 * pairs - 1;
+    }
+  } else if (g->kind == kAa && g->dPairItems) {
     const lbm::AaArgs a = aa_args(g);
     for (int it = 0; it < n; it += 2) {
       mark();
@@ -475,6 +494,7 @@ long enqueue_steps(Gpu* g, const lbm::Trt<double>& t, int n, cudaEvent_t* ev = n
 
 long launches_for(Gpu* g, int n) {
   if (two_grid(g->kind)) return n;
+  if (g->dMeet) return ((n + 1) / 2 + kResidentPairs - 1) / kResidentPairs;
   long perPair = g->dPairItems ? 1 : 2;
   if (g->kind == kAa && !g->dPairItems) {
     const lbm::AaArgs a = aa_args(g);
@@ -546,11 +566,10 @@ void raw_to_mirror(Gpu* g) {
 void clear_lost(Gpu* g) {
   if (!g->stateLost) return;
   LBM_CK(cudaMemsetAsync(g->dErr, 0, sizeof(int), g->stream));
-  if (g->dPairCount) {
-    // fused pairs count from zero again, whatever the lost launch left
-    LBM_CK(cudaMemsetAsync(g->dPairCount, 0, sizeof(uint32_t) * g->pairGroups, g->stream));
-    g->pairEpoch = 0;
-  }
+  // fused pairs count from zero again, whatever the lost launch left
+  if (g->dMeet) LBM_CK(cudaMemsetAsync(g->dMeet, 0, sizeof(uint32_t), g->stream));
+  if (g->dPairCount)
+    LBM_CK(cudaMemsetAsync(g->dPairCount, 0, sizeof(uint32_t) * (g->pairGroups + 2), g->stream));
   g->stateLost = false;
 }
 
@@ -684,6 +703,15 @@ void cb_kernel(LatticeDesc* ld, KernelData* kd, CaseData* cd) {
 constexpr int kPairF16Tiles = 2048;
 constexpr double kPairLateShare = 0.1;
 
+// Small domains: all tiles resident, many pairs per launch.
+bool schedule_resident(Gpu* g, size_t nTiles, int most) {
+  if (nTiles == 0 || nTiles > (size_t)most) return false;
+  g->pairTiles = static_cast<uint32_t>(nTiles);
+  LBM_CK(cudaMalloc(&g->dMeet, sizeof(uint32_t)));
+  LBM_CK(cudaMemset(g->dMeet, 0, sizeof(uint32_t)));
+  return true;
+}
+
 double pair_max_lag(Gpu* g) {
   int dev = 0, l2 = 0;
   LBM_CK(cudaGetDevice(&dev));
@@ -696,8 +724,8 @@ void pair_upload(Gpu* g, const std::vector<lbm::PairRec<R>>& items, size_t nTile
   g->pairTiles = static_cast<uint32_t>(nTiles);
   g->pairItems = static_cast<uint32_t>(items.size());
   g->pairGroups = static_cast<uint32_t>((nTiles + (1u << lbm::kPairGroupShift) - 1) >> lbm::kPairGroupShift);
-  LBM_CK(cudaMalloc(&g->dPairCount, sizeof(uint32_t) * g->pairGroups));
-  LBM_CK(cudaMemset(g->dPairCount, 0, sizeof(uint32_t) * g->pairGroups));
+  LBM_CK(cudaMalloc(&g->dPairCount, sizeof(uint32_t) * (g->pairGroups + 2)));
+  LBM_CK(cudaMemset(g->dPairCount, 0, sizeof(uint32_t) * (g->pairGroups + 2)));
   LBM_CK(cudaMalloc(&g->dPairItems, sizeof(lbm::PairRec<R>) * items.size()));
   LBM_CK(cudaMemcpy(g->dPairItems, items.data(), sizeof(lbm::PairRec<R>) * items.size(), cudaMemcpyHostToDevice));
 }
@@ -705,6 +733,7 @@ void pair_upload(Gpu* g, const std::vector<lbm::PairRec<R>>& items, size_t nTile
 void schedule_list_pairs(Gpu* g) {
   const int nTiles = (g->nFluid + lbm::kListTile - 1) / lbm::kListTile;
   if (nTiles == 0 || (g->storage == lbm::kStoreF16 && nTiles > kPairF16Tiles)) return;
+  if (schedule_resident(g, (size_t)nTiles, lbm::list_resident_tiles(g->storage))) return;
   uint32_t* dReach = nullptr;
   std::vector<uint32_t> reach(6 * (size_t)nTiles), off((size_t)nTiles + 1);
   LBM_CK(cudaMallocAsync(&dReach, sizeof(uint32_t) * reach.size(), g->stream));
@@ -724,8 +753,6 @@ void schedule_list_pairs(Gpu* g) {
 void schedule_aa_pairs(Gpu* g, const LatticeDesc* ld) {
   const lbm::AaArgs a = aa_args(g);
   g->pairGeom = lbm::aa_pair_geom(a);
-  std::vector<lbm::AaPairItem> items;
-  lbm::aa_pair_schedule(a, g->pairGeom, lbm::aa_pair_resident(), items);
   // a link of a fluid cell on a non-periodic face leaves into the ghost layer
   const int* n = g->dims;
   for (int axis = 0; axis < 3 && !g->openFaces; ++axis) {
@@ -739,7 +766,11 @@ void schedule_aa_pairs(Gpu* g, const LatticeDesc* ld) {
           g->openFaces |= ld->Lattice[lbmh_lidx(n, p[0], p[1], p[2])] != LAT_CELL_OBSTACLE;
         }
   }
-  pair_upload(g, items, (size_t)g->pairGeom.tpp * g->pairGeom.nX);
+  const size_t nTiles = (size_t)g->pairGeom.tpp * g->pairGeom.nX;
+  if (schedule_resident(g, nTiles, lbm::aa_resident_tiles())) return;
+  std::vector<lbm::AaPairItem> items;
+  lbm::aa_pair_schedule(a, g->pairGeom, lbm::aa_pair_resident(), items);
+  pair_upload(g, items, nTiles);
 }
 
 // The interior work items of the AA odd step by itself (slabs), from the link
@@ -986,6 +1017,7 @@ void gpu_free(KernelData** kernelData) {
   cudaFree(g->dRunOff);
   cudaFree(g->dPairItems);
   cudaFree(g->dPairCount);
+  cudaFree(g->dMeet);
   for (int side = 0; side < 2; ++side)
     for (int list = 0; list < 2; ++list) cudaFree(g->dHalo[side][list]);
   cudaFree(g->dErr);

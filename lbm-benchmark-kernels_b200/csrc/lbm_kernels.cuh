@@ -182,9 +182,9 @@ template <int R>
 struct PairArgs {
   const PairRec<R>* items;  // nItems records
   uint32_t* count;          // even tiles done per group, summed over all launches
+  uint32_t* launches;       // [0] launches completed, [1] blocks of this one that have read [0]
   uint32_t nItems;          // blocks of the launch
   uint32_t nTiles;
-  uint32_t epoch;           // launches including this one (counter targets)
   int prefetch;             // as ListArgs::prefetch (0: none)
 };
 
@@ -236,8 +236,39 @@ double pair_order(const std::vector<PairRec<R>>& work, const std::vector<uint32_
 
 // Blocks of a fused kernel that run at once on the current device.
 int list_pair_resident(int storage);
+
+// Small domains: many pairs in one cooperative launch, one block per tile
+// (lbm_pair.cuh).
+struct ResidentArgs {
+  uint32_t* meet;  // arrivals of the launch (0 between launches)
+  int pairs;
+};
+// Tiles up to which that is the faster way: `perSM` blocks on every SM (fewer
+// where fewer of `kernel` fit; 0 without cooperative launches; cached in `n`).
+// Fuller SMs leave too little beside the blocks that wait. us per step, pairs
+// as launches of their own / in one launch: lists FP64 172 tiles 5.2 / 4.3, 408
+// tiles 5.9 / 6.1; FP32 172 tiles 4.2 / 3.2, 408 tiles 5.2 / 4.4, 680 tiles
+// 5.8 / 6.5; full array 128 tiles 4.1 / 3.0, 432 tiles 7.9 / 9.9.
+template <class K>
+int resident_tiles(std::atomic<int>& n, K kernel, int threads, int perSM) {
+  int v = n.load(std::memory_order_acquire);
+  if (v == 0) {
+    int dev = 0, sms = 0, per = 0, coop = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, threads, 0);
+    v = coop && per > 0 ? sms * std::min(per, perSM) : -1;
+    n.store(v, std::memory_order_release);
+  }
+  return v > 0 ? v : 0;
+}
+int list_resident_tiles(int storage);
+int aa_resident_tiles();
 void list_pair_fp64(const ListArgs& a, const PairArgs<3>& p, const Trt<double>& t, cudaStream_t s);
 void list_pair_lp(const ListArgsLp& a, const PairArgs<3>& p, const TrtW& t, int storage, cudaStream_t s);
+void list_resident_fp64(const ListArgs& a, const ResidentArgs& r, const Trt<double>& t, cudaStream_t s);
+void list_resident_lp(const ListArgsLp& a, const ResidentArgs& r, const TrtW& t, int storage, cudaStream_t s);
 
 // Launchers (stream-ordered, no synchronisation).
 void list_even_lp(const ListArgsLp& a, const TrtW& t, int storage, cudaStream_t s);
@@ -289,6 +320,8 @@ struct AaPairArgs {
 AaPairGeom aa_pair_geom(const AaArgs& a);
 void aa_pair_schedule(const AaArgs& a, const AaPairGeom& g, int margin, std::vector<AaPairItem>& items);
 int aa_pair_resident();
+void aa_resident_fp64(const AaArgs& a, const AaPairGeom& g, int openFaces, const ResidentArgs& r,
+                      const Trt<double>& t, cudaStream_t s);
 void aa_pair_fp64(const AaArgs& a, const AaPairArgs& p, const Trt<double>& t, cudaStream_t s);
 bool aa_has_interior(const AaArgs& a);
 // Two-grid full-array push / pull steps (push-soa / pull-soa): every fluid

@@ -427,6 +427,48 @@ __device__ __forceinline__ void aa_pair_tile(const AaPairGeom& g, uint32_t k, ui
   cell0 = (s * g.J + r - x * width) * kListTile;
 }
 
+// The even step of cell c (link word w). The loads do not wait for the word
+// (solid cells' slots exist; nothing is stored there).
+__device__ __forceinline__ void aa_pair_even_cell(const AaArgs& a, const Trt<double>& t, int c, uint32_t w) {
+  const double* const f = a.f + c;
+  double* const fs = launder(a.f + c);
+  const uint64_t keep = l2_keep_policy();
+  const long long S = a.dstride;
+  trt_update(t, [&](int d) { return __ldcs(f + d * S); },
+             [&](int d, double v) {
+               if (w & kFluidBit) st_keep(fs + inv(d) * S, v, keep);
+             });
+}
+
+// What a warp's odd step has to provide for: any reversed link, any fluid cell
+// on a face of the lattice.
+struct AaWarpKind {
+  bool wall, face;
+};
+__device__ __forceinline__ AaWarpKind aa_warp_kind(const AaArgs& a, int x, int y, int z, uint32_t w) {
+  const bool fluid = w & kFluidBit;
+  AaWarpKind k;
+  k.wall = __any_sync(0xffffffffu, fluid && (w & kLinkBits));
+  k.face = __any_sync(0xffffffffu, fluid && XyzWrap(a, x, y, z).m != 0u);
+  return k;
+}
+__device__ __forceinline__ void aa_pair_odd_cell(const AaArgs& a, const Trt<double>& t, int c, int x, int y, int z,
+                                                 uint32_t w, const AaWarpKind& kind, int openFaces) {
+  if (!(w & kFluidBit)) return;
+  if (!kind.wall) {
+    double* const fb = a.f + c;
+    const XyzWrap wrap(a, x, y, z);
+    trt_update(t, [&](int d) -> double { return fb[a.ldOff[d] + wrap(inv(d))] + t.force[d]; },
+               [&](int d, double v) { __stcs(launder(fb) + (a.stOff[d] + wrap(d)), v + t.force[d]); });
+  } else if (!kind.face) {
+    aa_odd_select(a, t, c, w, NoWrap());
+  } else if (!openFaces) {
+    aa_odd_wall_cell(a, t, c, x, y, z, w);
+  } else {
+    aa_odd_open_cell(a, t, c, x, y, z, w);
+  }
+}
+
 // One thread per cell of a tile of 256 consecutive cells of an x plane in
 // (y, z) order, so that rows of any length fill the warps (64^3, whose 64-cell
 // rows left half to three quarters of the threads of row-shaped blocks idle).
@@ -453,6 +495,7 @@ __global__ void __launch_bounds__(kPairThreads, 3)
     pair_service(&sh, q.p, nullptr, a.err, k);
     return;
   }
+  chain_wait();
   if (k < q.p.nTiles) {
     uint32_t x, i;
     aa_pair_tile(q.g, k, x, i);
@@ -460,15 +503,7 @@ __global__ void __launch_bounds__(kPairThreads, 3)
     if (i < q.g.plane) {
       const uint32_t y = fast_div(i, q.g.byZ), z = i - y * q.g.byZ.d;
       const int c = aa_cell(a, x, y, z);
-      const uint32_t w = __ldg(a.link + c);
-      const double* const f = a.f + c;
-      double* const fs = launder(a.f + c);
-      const uint64_t keep = l2_keep_policy();
-      const long long S = a.dstride;
-      trt_update(t, [&](int d) { return __ldcs(f + d * S); },
-                 [&](int d, double v) {
-                   if (w & kFluidBit) st_keep(fs + inv(d) * S, v, keep);
-                 });
+      aa_pair_even_cell(a, t, c, __ldg(a.link + c));
     }
     pair_even_done(&sh);
   }
@@ -477,21 +512,28 @@ __global__ void __launch_bounds__(kPairThreads, 3)
   const uint32_t y = fast_div(i, q.g.byZ), z = i - y * q.g.byZ.d;
   const int c = aa_cell(a, x, y, z);
   const uint32_t w = i < q.g.plane ? __ldg(a.link + c) : 0u;
-  const bool fluid = w & kFluidBit;
-  const bool wall = __any_sync(0xffffffffu, fluid && (w & kLinkBits));
-  const bool face = __any_sync(0xffffffffu, fluid && XyzWrap(a, x, y, z).m != 0u);
-  if (!pair_odd_turn(&sh, a.err) || !fluid) return;
-  if (!wall) {
-    double* const fb = a.f + c;
-    const XyzWrap wrap(a, x, y, z);
-    trt_update(t, [&](int d) -> double { return fb[a.ldOff[d] + wrap(inv(d))] + t.force[d]; },
-               [&](int d, double v) { __stcs(launder(fb) + (a.stOff[d] + wrap(d)), v + t.force[d]); });
-  } else if (!face) {
-    aa_odd_select(a, t, c, w, NoWrap());
-  } else if (!q.openFaces) {
-    aa_odd_wall_cell(a, t, c, x, y, z, w);
-  } else {
-    aa_odd_open_cell(a, t, c, x, y, z, w);
+  const AaWarpKind kind = aa_warp_kind(a, x, y, z, w);
+  if (pair_odd_turn(&sh, a.err)) aa_pair_odd_cell(a, t, c, x, y, z, w, kind, q.openFaces);
+}
+
+// Small lattices (lbm_pair.cuh): block b on tile b for all pairs of the launch.
+__global__ void __launch_bounds__(kListTile, 3)
+    k_aa_resident_fp64(const __grid_constant__ AaArgs a, const __grid_constant__ AaPairGeom g, int openFaces,
+                       const __grid_constant__ ResidentArgs r, const __grid_constant__ Trt<double> t) {
+  __shared__ int ok;
+  chain_wait();
+  uint32_t x, i;
+  aa_pair_tile(g, blockIdx.x, x, i);
+  i += threadIdx.x;
+  const uint32_t y = fast_div(i, g.byZ), z = i - y * g.byZ.d;
+  const int c = aa_cell(a, x, y, z);
+  const uint32_t w = i < g.plane ? __ldg(a.link + c) : 0u;
+  const AaWarpKind kind = aa_warp_kind(a, x, y, z, w);
+  for (int p = 0; p < r.pairs; ++p) {
+    if (i < g.plane) aa_pair_even_cell(a, t, c, w);
+    if (!resident_meet(r, 2 * p + 1, a.err, &ok)) return;
+    aa_pair_odd_cell(a, t, c, x, y, z, w, kind, openFaces);
+    if (!resident_meet(r, 2 * p + 2, a.err, &ok)) return;
   }
 }
 
@@ -600,13 +642,23 @@ void aa_pair_schedule(const AaArgs& a, const AaPairGeom& g, int margin, std::vec
   pair_order(work, need, home, nTiles, static_cast<size_t>(margin), 0.0, items);
 }
 
+int aa_resident_tiles() {
+  static std::atomic<int> n{0};
+  return resident_tiles(n, k_aa_resident_fp64, kListTile, 2);
+}
+
+void aa_resident_fp64(const AaArgs& a, const AaPairGeom& g, int openFaces, const ResidentArgs& r,
+                      const Trt<double>& t, cudaStream_t s) {
+  launch_together(k_aa_resident_fp64, g.nX * g.tpp, kListTile, s, a, g, openFaces, r, t);
+}
+
 int aa_pair_resident() {
   static std::atomic<int> n{0};
   return prefetch_distance(n, k_aa_pair_fp64, kPairThreads, true);
 }
 
 void aa_pair_fp64(const AaArgs& a, const AaPairArgs& q, const Trt<double>& t, cudaStream_t s) {
-  if (q.p.nItems > 0) k_aa_pair_fp64<<<q.p.nItems, kPairThreads, 0, s>>>(a, q, t);
+  if (q.p.nItems > 0) launch_chained(k_aa_pair_fp64, q.p.nItems, kPairThreads, 0, s, a, q, t);
 }
 
 // ---------------------------------------------------------------------------
@@ -698,6 +750,7 @@ constexpr int kFaBZ = 32, kFaBY = 4;
 // node's own slot inv(d); an open face leaves that slot untouched by the step,
 // so only the force increment is added to what the grid held.
 __global__ void __launch_bounds__(128) k_fa_push_fp64(const AaArgs a, const Trt<double> t) {
+  chain_wait();
   const int z = blockIdx.x * kFaBZ + threadIdx.x;
   const int y = blockIdx.y * kFaBY + threadIdx.y;
   const int x = blockIdx.z;
@@ -740,6 +793,7 @@ __global__ void __launch_bounds__(128) k_fa_push_fp64(const AaArgs a, const Trt<
 // image q = wrap(x + c_e) gets it at (q - c_e, e), and an open slot only gets
 // the force increment.
 __global__ void __launch_bounds__(128) k_fa_pull_fp64(const AaArgs a, const Trt<double> t) {
+  chain_wait();
   const int z = blockIdx.x * kFaBZ + threadIdx.x;
   const int y = blockIdx.y * kFaBY + threadIdx.y;
   const int x = blockIdx.z;
@@ -777,10 +831,12 @@ __global__ void __launch_bounds__(128) k_fa_pull_fp64(const AaArgs a, const Trt<
 }
 
 void fa_push_fp64(const AaArgs& a, const Trt<double>& t, cudaStream_t s) {
-  k_fa_push_fp64<<<dim3((a.nZ + kFaBZ - 1) / kFaBZ, (a.nY + kFaBY - 1) / kFaBY, a.nX), dim3(kFaBZ, kFaBY), 0, s>>>(a, t);
+  launch_chained(k_fa_push_fp64, dim3((a.nZ + kFaBZ - 1) / kFaBZ, (a.nY + kFaBY - 1) / kFaBY, a.nX),
+                 dim3(kFaBZ, kFaBY), 0, s, a, t);
 }
 void fa_pull_fp64(const AaArgs& a, const Trt<double>& t, cudaStream_t s) {
-  k_fa_pull_fp64<<<dim3((a.nZ + kFaBZ - 1) / kFaBZ, (a.nY + kFaBY - 1) / kFaBY, a.nX), dim3(kFaBZ, kFaBY), 0, s>>>(a, t);
+  launch_chained(k_fa_pull_fp64, dim3((a.nZ + kFaBZ - 1) / kFaBZ, (a.nY + kFaBY - 1) / kFaBY, a.nX),
+                 dim3(kFaBZ, kFaBY), 0, s, a, t);
 }
 
 long long aa_shell_cells(const AaArgs& a) {
@@ -875,6 +931,8 @@ void aa_odd_face_fp64(const AaArgs& a, const Trt<double>& t, cudaStream_t s) {
 
 // 4 blocks of 256 threads per SM (64 registers, no spills)
 __global__ void __launch_bounds__(kListTile, 4) k_list_even_fp64(const ListArgs a, const Trt<double> t) {
+  chain_next();
+  chain_wait();
   const int n = (blockIdx.x + a.tileBase) * kListTile + threadIdx.x;
   if (n >= a.nFluid) return;
   double* const f = a.f + n;
@@ -944,39 +1002,19 @@ __global__ void __launch_bounds__(kListTile, 3) k_list_odd_fp64(const ListArgs a
   trt_update(t, load, store);
 }
 
-// The fused pair (lbm_pair.cuh): the arithmetic of the two kernels above. The
-// parameters are read in place (__grid_constant__), which leaves room for
-// both steps under the 72 registers of 3 blocks of 288 threads per SM. What
-// bounds it: L2 and the fabric between its halves (the odd step's gathers and
-// scatters touch 1.2-1.5 sectors per sector of payload; without any waiting
-// the 256^3 packing would take 0.247 ms per step), then the waits.
-__global__ void __launch_bounds__(kPairThreads, 3)
-    k_list_pair_fp64(const __grid_constant__ ListArgs a, const __grid_constant__ PairArgs<3> p,
-                     const __grid_constant__ Trt<double> t) {
-  __shared__ ListPairShared sh;
-  pair_init(&sh);
-  const uint32_t k = blockIdx.x;
-  if (threadIdx.x >= kListTile) {
-    pair_service(&sh, p, a.runs, a.err, k);
-    return;
-  }
+// The two steps of node n in the fused kernels: the arithmetic of the two
+// kernels above, with the cache hints of lbm_pair.cuh.
+__device__ __forceinline__ void pair_even_node(const ListArgs& a, const Trt<double>& t, int n) {
   const long long S = a.nCells;
-  if (k < p.nTiles) {
-    const int n = static_cast<int>(k) * kListTile + threadIdx.x;
-    if (n < a.nFluid) {
-      const double* const f = a.f + n;
-      double* const fs = launder(a.f + n);
-      const uint64_t keep = l2_keep_policy();
-      trt_update(t, [&](int d) { return __ldcs(f + d * S); },
-                 [&](int d, double v) { st_keep(fs + inv(d) * S, v, keep); });
-    }
-    pair_even_done(&sh);
-  }
-  if (!pair_odd_turn(&sh, a.err)) return;
-  const int n = static_cast<int>(sh.item.tile) * kListTile + threadIdx.x;
-  if (n >= a.nFluid) return;
-  uint32_t off;
-  const uint32_t* e = run_row(sh.run, threadIdx.x, off);
+  const double* const f = a.f + n;
+  double* const fs = launder(a.f + n);
+  const uint64_t keep = l2_keep_policy();
+  trt_update(t, [&](int d) { return __ldcs(f + d * S); },
+             [&](int d, double v) { st_keep(fs + inv(d) * S, v, keep); });
+}
+__device__ __forceinline__ void pair_odd_node(const ListArgs& a, const Trt<double>& t, int n, const uint32_t* e,
+                                              uint32_t off) {
+  const long long S = a.nCells;
   double* const f = a.f;
   auto load = [&](int d) -> double { return (d == DC ? f[DC * S + n] : f[e[inv(d)] + off]) + t.force[d]; };
   auto store = [&](int d, double v) {
@@ -987,6 +1025,55 @@ __global__ void __launch_bounds__(kPairThreads, 3)
     __stcs(f + dst, v + (bounce ? t.force[j] : t.force[d]));
   };
   trt_update(t, load, store);
+}
+
+// The fused pair (lbm_pair.cuh). The parameters are read in place
+// (__grid_constant__), which leaves room for both steps under the 72 registers
+// of 3 blocks of 288 threads per SM. What bounds it: L2 and the fabric between
+// its halves (the odd step's gathers and scatters touch 1.2-1.5 sectors per
+// sector of payload; without any waiting the 256^3 packing would take 0.247 ms
+// per step), then the waits.
+__global__ void __launch_bounds__(kPairThreads, 3)
+    k_list_pair_fp64(const __grid_constant__ ListArgs a, const __grid_constant__ PairArgs<3> p,
+                     const __grid_constant__ Trt<double> t) {
+  __shared__ ListPairShared sh;
+  pair_init(&sh);
+  const uint32_t k = blockIdx.x;
+  if (threadIdx.x >= kListTile) {
+    pair_service(&sh, p, a.runs, a.err, k);
+    return;
+  }
+  chain_wait();
+  if (k < p.nTiles) {
+    const int n = static_cast<int>(k) * kListTile + threadIdx.x;
+    if (n < a.nFluid) pair_even_node(a, t, n);
+    pair_even_done(&sh);
+  }
+  if (!pair_odd_turn(&sh, a.err)) return;
+  const int n = static_cast<int>(sh.item.tile) * kListTile + threadIdx.x;
+  if (n >= a.nFluid) return;
+  uint32_t off;
+  const uint32_t* e = run_row(sh.run, threadIdx.x, off);
+  pair_odd_node(a, t, n, e, off);
+}
+
+// Small domains (lbm_pair.cuh): block b on tile b for all pairs of the launch.
+__global__ void __launch_bounds__(kListTile, 3)
+    k_list_resident_fp64(const __grid_constant__ ListArgs a, const __grid_constant__ ResidentArgs r,
+                         const __grid_constant__ Trt<double> t) {
+  __shared__ alignas(128) uint32_t srun[kRunTileWords];
+  __shared__ alignas(8) uint64_t bar;
+  __shared__ int ok;
+  if (!stage_run_tile(a, srun, &bar, &ok)) return;
+  const int n = static_cast<int>(blockIdx.x) * kListTile + threadIdx.x;
+  uint32_t off = 0;
+  const uint32_t* e = run_row(srun, threadIdx.x, off);
+  for (int p = 0; p < r.pairs; ++p) {
+    if (n < a.nFluid) pair_even_node(a, t, n);
+    if (!resident_meet(r, 2 * p + 1, a.err, &ok)) return;
+    if (n < a.nFluid) pair_odd_node(a, t, n, e, off);
+    if (!resident_meet(r, 2 * p + 2, a.err, &ok)) return;
+  }
 }
 
 __global__ void __launch_bounds__(kListTile) k_list_pull_fp64(const ListArgs a, const Trt<double> t) {
@@ -1091,14 +1178,14 @@ static unsigned list_blocks(const ListArgs& a) { return (a.nFluid + kListTile - 
 void list_even_fp64(const ListArgs& a, const Trt<double>& t, cudaStream_t s) {
   ListArgs b = a;
   b.tileBase = 0;
-  if (a.nFluid > 0) k_list_even_fp64<<<list_blocks(b), kListTile, 0, s>>>(b, t);
+  if (a.nFluid > 0) launch_chained(k_list_even_fp64, list_blocks(b), kListTile, 0, s, b, t);
 }
 
 void list_even_fp64_tiles(const ListArgs& a, const Trt<double>& t, int t0, int t1, cudaStream_t s) {
   if (a.nFluid <= 0 || t1 <= t0) return;
   ListArgs b = a;
   b.tileBase = t0;
-  k_list_even_fp64<<<(unsigned)(t1 - t0), kListTile, 0, s>>>(b, t);
+  launch_chained(k_list_even_fp64, (unsigned)(t1 - t0), kListTile, 0, s, b, t);
 }
 static std::atomic<int> g_oddAhead{0};
 
@@ -1107,7 +1194,7 @@ void list_odd_fp64(const ListArgs& a, const Trt<double>& t, cudaStream_t s) {
   ListArgs b = a;
   b.tileBase = 0;
   b.prefetch = prefetch_distance(g_oddAhead, k_list_odd_fp64, kListTile, a.prefetch != 0);
-  k_list_odd_fp64<<<list_blocks(b), kListTile, 0, s>>>(b, t);
+  launch_chained(k_list_odd_fp64, list_blocks(b), kListTile, 0, s, b, t);
 }
 
 void list_odd_fp64_tiles(const ListArgs& a, const Trt<double>& t, int t0, int t1, cudaStream_t s) {
@@ -1115,10 +1202,20 @@ void list_odd_fp64_tiles(const ListArgs& a, const Trt<double>& t, int t0, int t1
   ListArgs b = a;
   b.tileBase = t0;
   b.prefetch = prefetch_distance(g_oddAhead, k_list_odd_fp64, kListTile, a.prefetch != 0);
-  k_list_odd_fp64<<<(unsigned)(t1 - t0), kListTile, 0, s>>>(b, t);
+  launch_chained(k_list_odd_fp64, (unsigned)(t1 - t0), kListTile, 0, s, b, t);
 }
 void list_pair_fp64(const ListArgs& a, const PairArgs<3>& p, const Trt<double>& t, cudaStream_t s) {
-  if (p.nItems > 0) k_list_pair_fp64<<<p.nItems, kPairThreads, 0, s>>>(a, p, t);
+  if (p.nItems > 0) launch_chained(k_list_pair_fp64, p.nItems, kPairThreads, 0, s, a, p, t);
+}
+void list_resident_fp64(const ListArgs& a, const ResidentArgs& r, const Trt<double>& t, cudaStream_t s) {
+  ListArgs b = a;
+  b.tileBase = 0;
+  b.prefetch = 0;
+  launch_together(k_list_resident_fp64, list_blocks(b), kListTile, s, b, r, t);
+}
+int list_resident_tiles_fp64() {
+  static std::atomic<int> n{0};
+  return resident_tiles(n, k_list_resident_fp64, kListTile, 2);
 }
 int list_pair_resident_fp64() {
   static std::atomic<int> n{0};
@@ -1130,14 +1227,14 @@ void list_pull_fp64(const ListArgs& a, const Trt<double>& t, cudaStream_t s) {
   if (a.nFluid <= 0) return;
   ListArgs b = a;
   b.prefetch = 0;
-  k_list_pull_fp64<<<list_blocks(b), kListTile, 0, s>>>(b, t);
+  launch_chained(k_list_pull_fp64, list_blocks(b), kListTile, 0, s, b, t);
 }
 void list_push_fp64(const ListArgs& a, const Trt<double>& t, cudaStream_t s) {
   static std::atomic<int> ahead{0};
   if (a.nFluid <= 0) return;
   ListArgs b = a;
   b.prefetch = prefetch_distance(ahead, k_list_push_fp64, kListTile, a.prefetch != 0);
-  k_list_push_fp64<<<list_blocks(b), kListTile, 0, s>>>(b, t);
+  launch_chained(k_list_push_fp64, list_blocks(b), kListTile, 0, s, b, t);
 }
 
 }  // namespace lbm

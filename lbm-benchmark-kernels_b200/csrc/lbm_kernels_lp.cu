@@ -14,6 +14,8 @@ namespace lbm {
 
 template <class St>
 __global__ void __launch_bounds__(kListTile) k_list_even_lp(const ListArgsLp a, const TrtW w) {
+  chain_next();
+  chain_wait();
   const int n = (blockIdx.x + a.tileBase) * kListTile + threadIdx.x;
   if (n >= a.nFluid) return;
   lp_even_node<St>(static_cast<typename St::T*>(a.f), a.nCells, n, TrtDev<St>(w));
@@ -29,6 +31,8 @@ __global__ void __launch_bounds__(kListTile) k_list_even_lp(const ListArgsLp a, 
 // it to whole kLpTileNodes tiles).
 template <class St, int StageBytes, int Stages>
 __global__ void __launch_bounds__(256, 2) k_list_even_staged(const ListArgsLp a, const TrtW w) {
+  chain_next();
+  chain_wait();
   using T = typename St::T;
   const TrtDev<St> t(w);
   constexpr int TN = StageBytes / (int)sizeof(T);
@@ -45,6 +49,8 @@ __global__ void __launch_bounds__(256, 2) k_list_even_staged(const ListArgsLp a,
     for (int d = 0; d < Q; ++d) bulk_g2s(dst + d * StageBytes, f + d * S + (long long)tile * TN, StageBytes, &full[st]);
   };
   if (threadIdx.x == 0) {
+    // the copies below read what the previous step stored
+    asm volatile("fence.proxy.async.global;" ::: "memory");
     for (int st = 0; st < Stages; ++st) mbar_init(&full[st], 1);
     for (int st = 0; st < Stages - 1; ++st)
       if (blockIdx.x + st * gridDim.x < nTiles) issue(blockIdx.x + st * gridDim.x, st);
@@ -145,6 +151,7 @@ __global__ void __launch_bounds__(kPairThreads, 5)
     pair_service(&sh, p, a.runs, a.err, k);
     return;
   }
+  chain_wait();
   using T = typename St::T;
   const TrtDev<St> t(w);
   if (k < p.nTiles) {
@@ -160,12 +167,54 @@ __global__ void __launch_bounds__(kPairThreads, 5)
   lp_odd_node<St, true, PairAccess>(static_cast<T*>(a.f), static_cast<uint32_t>(a.nCells), n, e, off, t);
 }
 
+// Small domains (lbm_pair.cuh): block b on tile b for all pairs of the launch.
+template <class St>
+__global__ void __launch_bounds__(kListTile, 5)
+    k_list_resident_lp(const __grid_constant__ ListArgsLp a, const __grid_constant__ ResidentArgs r,
+                       const __grid_constant__ TrtW w) {
+  __shared__ alignas(128) uint32_t srun[kRunTileWords];
+  __shared__ alignas(8) uint64_t bar;
+  __shared__ int ok;
+  if (!stage_run_tile(a, srun, &bar, &ok)) return;
+  const int n = static_cast<int>(blockIdx.x) * kListTile + threadIdx.x;
+  uint32_t off = 0;
+  const uint32_t* e = run_row(srun, threadIdx.x, off);
+  using T = typename St::T;
+  const TrtDev<St> t(w);
+  for (int p = 0; p < r.pairs; ++p) {
+    if (n < a.nFluid) lp_even_node<St>(static_cast<T*>(a.f), a.nCells, n, t);
+    if (!resident_meet(r, 2 * p + 1, a.err, &ok)) return;
+    if (n < a.nFluid) lp_odd_node<St>(static_cast<T*>(a.f), static_cast<uint32_t>(a.nCells), n, e, off, t);
+    if (!resident_meet(r, 2 * p + 2, a.err, &ok)) return;
+  }
+}
+
+void list_resident_lp(const ListArgsLp& a, const ResidentArgs& r, const TrtW& t, int storage, cudaStream_t s) {
+  ListArgsLp b = a;
+  b.tileBase = 0;
+  b.prefetch = 0;
+  const unsigned blocks = (a.nFluid + kListTile - 1) / kListTile;
+  if (storage == kStoreF16)
+    launch_together(k_list_resident_lp<StoreF16>, blocks, kListTile, s, b, r, t);
+  else
+    launch_together(k_list_resident_lp<StoreF32>, blocks, kListTile, s, b, r, t);
+}
+
+int list_resident_tiles_fp64();
+
+int list_resident_tiles(int storage) {
+  static std::atomic<int> n32{0}, n16{0};
+  if (storage == kStoreF16) return resident_tiles(n16, k_list_resident_lp<StoreF16>, kListTile, 3);
+  if (storage == kStoreF32) return resident_tiles(n32, k_list_resident_lp<StoreF32>, kListTile, 3);
+  return list_resident_tiles_fp64();
+}
+
 void list_pair_lp(const ListArgsLp& a, const PairArgs<3>& p, const TrtW& t, int storage, cudaStream_t s) {
   if (p.nItems == 0) return;
   if (storage == kStoreF16)
-    k_list_pair_lp<StoreF16><<<p.nItems, kPairThreads, 0, s>>>(a, p, t);
+    launch_chained(k_list_pair_lp<StoreF16>, p.nItems, kPairThreads, 0, s, a, p, t);
   else
-    k_list_pair_lp<StoreF32><<<p.nItems, kPairThreads, 0, s>>>(a, p, t);
+    launch_chained(k_list_pair_lp<StoreF32>, p.nItems, kPairThreads, 0, s, a, p, t);
 }
 
 int list_pair_resident_fp64();
@@ -202,7 +251,7 @@ static void launch_even_staged(const ListArgsLp& a, const TrtW& t, cudaStream_t 
     g = sms * kEvenBlocksPerSM;
     if (dev < kMaxDevices) grid[dev].store(g, std::memory_order_release);
   }
-  kern<<<g, 256, smem, s>>>(a, t);
+  launch_chained(kern, g, 256, smem, s, a, t);
 }
 
 // FP16: the staged even step (0.118 -> 0.100 ms at 6.7M nodes on B200, 66 ->
@@ -215,7 +264,7 @@ void list_even_lp(const ListArgsLp& a, const TrtW& t, int storage, cudaStream_t 
   if (storage == kStoreF16)
     launch_even_staged<StoreF16>(b, t, s);
   else
-    k_list_even_lp<StoreF32><<<lp_blocks(b), kListTile, 0, s>>>(b, t);
+    launch_chained(k_list_even_lp<StoreF32>, lp_blocks(b), kListTile, 0, s, b, t);
 }
 
 // Tile ranges run the per-node kernel for both storages (the FP16 staged
@@ -225,9 +274,9 @@ void list_even_lp_tiles(const ListArgsLp& a, const TrtW& t, int storage, int t0,
   ListArgsLp b = a;
   b.tileBase = t0;
   if (storage == kStoreF16)
-    k_list_even_lp<StoreF16><<<(unsigned)(t1 - t0), kListTile, 0, s>>>(b, t);
+    launch_chained(k_list_even_lp<StoreF16>, (unsigned)(t1 - t0), kListTile, 0, s, b, t);
   else
-    k_list_even_lp<StoreF32><<<(unsigned)(t1 - t0), kListTile, 0, s>>>(b, t);
+    launch_chained(k_list_even_lp<StoreF32>, (unsigned)(t1 - t0), kListTile, 0, s, b, t);
 }
 
 static std::atomic<int> ahead16{0}, ahead32{0};
@@ -238,10 +287,10 @@ void list_odd_lp_tiles(const ListArgsLp& a, const TrtW& t, int storage, int t0, 
   b.tileBase = t0;
   if (storage == kStoreF16) {
     b.prefetch = prefetch_distance(ahead16, k_list_odd_lp<StoreF16>, kListTile, a.prefetch != 0);
-    k_list_odd_lp<StoreF16><<<(unsigned)(t1 - t0), kListTile, 0, s>>>(b, t);
+    launch_chained(k_list_odd_lp<StoreF16>, (unsigned)(t1 - t0), kListTile, 0, s, b, t);
   } else {
     b.prefetch = prefetch_distance(ahead32, k_list_odd_lp<StoreF32>, kListTile, a.prefetch != 0);
-    k_list_odd_lp<StoreF32><<<(unsigned)(t1 - t0), kListTile, 0, s>>>(b, t);
+    launch_chained(k_list_odd_lp<StoreF32>, (unsigned)(t1 - t0), kListTile, 0, s, b, t);
   }
 }
 
@@ -251,10 +300,10 @@ void list_odd_lp(const ListArgsLp& a, const TrtW& t, int storage, cudaStream_t s
   b.tileBase = 0;
   if (storage == kStoreF16) {
     b.prefetch = prefetch_distance(ahead16, k_list_odd_lp<StoreF16>, kListTile, a.prefetch != 0);
-    k_list_odd_lp<StoreF16><<<lp_blocks(b), kListTile, 0, s>>>(b, t);
+    launch_chained(k_list_odd_lp<StoreF16>, lp_blocks(b), kListTile, 0, s, b, t);
   } else {
     b.prefetch = prefetch_distance(ahead32, k_list_odd_lp<StoreF32>, kListTile, a.prefetch != 0);
-    k_list_odd_lp<StoreF32><<<lp_blocks(b), kListTile, 0, s>>>(b, t);
+    launch_chained(k_list_odd_lp<StoreF32>, lp_blocks(b), kListTile, 0, s, b, t);
   }
 }
 

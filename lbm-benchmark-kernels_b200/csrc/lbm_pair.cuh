@@ -31,12 +31,14 @@
 #include <cstdint>
 
 #include "lbm_bulk.cuh"
+#include "lbm_chain.cuh"
 #include "lbm_kernels.cuh"
 
 namespace lbm {
 
 constexpr int kPairThreads = kListTile + 32;
-constexpr uint32_t kPairSpinLimit = 1u << 20;  // polls before giving up
+constexpr uint32_t kPairSpinLimit = 1u << 20;      // polls before giving up
+constexpr uint32_t kResidentSpinLimit = 1u << 22;  // the same between resident blocks
 
 // Cache hints. A slot written by the even step is read back by the odd step
 // soon, one written by the odd step not before the next pair: even loads and
@@ -55,6 +57,11 @@ __device__ __forceinline__ void st_keep(double* a, double v, uint64_t pol) {
 __device__ __forceinline__ uint32_t ld_acquire(const uint32_t* p) {
   uint32_t v;
   asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ uint32_t ld_relaxed(const uint32_t* p) {
+  uint32_t v;
+  asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
 __device__ __forceinline__ void red_release(uint32_t* p, uint32_t v) {
@@ -87,12 +94,14 @@ __device__ __forceinline__ void pair_init(PairShared<R, kWords>* sh) {
     mbar_init(&sh->even, kListTile / 32);
   }
   __syncthreads();
+  chain_next();
 }
 
 // One look (by the whole warp) at the even groups the item depends on:
-// whether all are complete. Counters and targets are compared modulo 2^32.
+// whether all are complete in launch number `launch` (from 1). Counters and
+// targets are compared modulo 2^32.
 template <int R>
-__device__ __forceinline__ bool pair_ready(const PairRec<R>& it, const PairArgs<R>& p) {
+__device__ __forceinline__ bool pair_ready(const PairRec<R>& it, const PairArgs<R>& p, uint32_t launch) {
   uint32_t all = 0;
 #pragma unroll
   for (int r = 0; r < R; ++r) all += it.n[r];
@@ -109,7 +118,7 @@ __device__ __forceinline__ bool pair_ready(const PairRec<R>& it, const PairArgs<
       j -= it.n[r];
     }
     const uint32_t size = min(p.nTiles - (g << kPairGroupShift), 1u << kPairGroupShift);
-    good = good && static_cast<int32_t>(ld_acquire(p.count + g) - p.epoch * size) >= 0;
+    good = static_cast<int32_t>(ld_acquire(p.count + g) - launch * size) >= 0 && good;
   }
   return __all_sync(0xffffffffu, good);
 }
@@ -140,14 +149,20 @@ __device__ __forceinline__ void pair_service(PairShared<R, kWords>* sh, const Pa
       if (k + 2 * kPairAhead < p.nItems) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.items + k + 2 * kPairAhead));
     }
   }
-  const bool ready = it.tile == kPairNone || pair_ready(it, p);
+  chain_wait();
+  // the launch counts itself: its arguments never change, so that a captured
+  // launch can be replayed
+  const uint32_t launch = ld_relaxed(p.launches) + 1u;
+  const bool ready = it.tile == kPairNone || pair_ready(it, p, launch);
   if (ready && lane == 0) mbar_arrive(&sh->go);
   if (even) {
     if (!mbar_wait_bounded(&sh->even, 0)) atomicOr(err, 1);
     if (lane == 0) red_release(p.count + (k >> kPairGroupShift), 1u);
   }
+  // the last block to have read the launch number moves it on
+  if (lane == 0 && atomicInc(p.launches + 1, p.nItems - 1u) == p.nItems - 1u) atomicAdd(p.launches, 1u);
   if (!ready) {
-    for (uint32_t spin = 0; !pair_ready(it, p); ++spin) {
+    for (uint32_t spin = 0; !pair_ready(it, p, launch); ++spin) {
       const bool stop = spin >= kPairSpinLimit || ((spin & 255u) == 255u && *reinterpret_cast<volatile int*>(err) != 0);
       if (__any_sync(0xffffffffu, stop)) {
         if (lane == 0) atomicOr(err, 1);
@@ -183,6 +198,39 @@ __device__ __forceinline__ bool pair_odd_turn(Sh* sh, int* err) {
     return false;
   }
   return sh->item.tile != kPairNone;
+}
+
+// ---------------------------------------------------------------------------
+// Small domains: all tiles resident, many pairs in one launch.
+//
+// A domain of few tiles takes many pairs in one cooperative launch, block b on
+// tile b throughout: the run record is staged once, and between the half steps
+// the blocks meet at a counter instead of ending and starting again. What
+// bounds such a domain is that chain of latencies: 48^3 packing (172 tiles),
+// FP64, 13.5 us per pair as two launches, 10.4 as one, 8.7 here; 32^3 fluid
+// box 12.3, 8.3, 6.0.
+
+// Meeting n (from 1) of the 2 * pairs that the blocks of the (cooperative)
+// grid hold. Nobody waits at the last one, which only clears the counter for
+// the next launch. False when the bounded wait ran out; every thread of the
+// block returns the same.
+__device__ __forceinline__ bool resident_meet(const ResidentArgs& r, uint32_t n, int* err, int* shOk) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const uint32_t want = n * gridDim.x, last = 2u * static_cast<uint32_t>(r.pairs) * gridDim.x;
+    int ok = 0;
+    if (want == last) {
+      if (atomicAdd(r.meet, 1u) == last - 1u) atomicExch(r.meet, 0u);
+      ok = 1;
+    } else {
+      red_release(r.meet, 1u);
+      for (uint32_t spin = 0; spin < kResidentSpinLimit && !ok; ++spin) ok = ld_acquire(r.meet) >= want;
+      if (!ok) atomicOr(err, 1);
+    }
+    *shOk = ok;
+  }
+  __syncthreads();
+  return *shOk != 0;
 }
 
 }  // namespace lbm

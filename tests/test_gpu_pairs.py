@@ -111,3 +111,63 @@ def test_slab_steps_on_a_whole_lattice():
             inst.deinit()
     m = lat.mask != 0
     assert np.array_equal(fields[0][m], fields[1][m])
+
+
+@pytest.mark.parametrize("prec", ["fp64", "fp32", "fp16"])
+@pytest.mark.parametrize("dims,steps", [((9, 8, 7), 2), ((30, 27, 29), 9), ((47, 44, 45), 6)])
+def test_small_domains_in_one_launch(prec, dims, steps):
+    """Domains whose tiles are all resident take many pairs per launch; one
+    tile, a part tile, several blocks, odd step counts (rounded up to pairs)."""
+    lat = _spheres(dims, 0.6) if dims[0] > 9 else lbmb200.geometry("fluid", dims, (1, 1, 1))
+    init = random_pdfs(lat.mask.size, 67)
+    cd = lbmb200.case(omega=1.2, xforce=2e-4, iterations=steps)
+    kargs = ["-lambda", "3/16", "-precision", prec]
+    inst = lbmb200.kernel("cuda-list-aa-pv-soa").init(lat, kernel_args=kargs)
+    try:
+        assert inst.launches_for(steps) == 1
+        inst.set_field(init)
+        inst.run(cd)
+        assert inst.last_launches == 1
+        inst.run(cd)
+        whole = inst.get_field()
+    finally:
+        inst.deinit()
+    got = _run_slabs(lat, 2, init, cd, 2 * ((steps + 1) // 2), layout="list", kargs=kargs)
+    m = lat.mask != 0
+    assert np.array_equal(got[m], whole[m])
+
+
+def test_captured_steps_replay():
+    """A captured sequence of fused pairs can be replayed: the launches count
+    themselves on the device."""
+    import ctypes
+
+    import torch
+    cd = lbmb200.case(omega=1.1, xforce=1e-4, iterations=4)
+    L = lbmb200.lib()
+    for lat in (_spheres((130, 44, 40), 0.6), _spheres((30, 27, 29), 0.6)):
+        init = random_pdfs(lat.mask.size, 71)
+        fields = []
+        for replay in (False, True):
+            inst = lbmb200.kernel("cuda-list-aa-pv-soa").init(lat, kernel_args=["-lambda", "3/16"])
+            try:
+                inst.set_field(init)
+                inst.run(cd)
+                if replay:
+                    st = ctypes.c_void_p()
+                    assert L.lbm_b200_device_state(inst.kdp, None, None, None, ctypes.byref(st)) == 0
+                    stream = torch.cuda.ExternalStream(st.value)
+                    g = torch.cuda.CUDAGraph()
+                    with torch.cuda.graph(g, stream=stream):
+                        inst.step_device(cd, 4)
+                    for _ in range(3):
+                        g.replay()
+                    torch.cuda.synchronize()
+                    inst.sync_mirror()
+                else:
+                    inst.run(lbmb200.case(omega=1.1, xforce=1e-4, iterations=12))
+                fields.append(inst.get_field())
+            finally:
+                inst.deinit()
+        m = lat.mask != 0
+        assert np.array_equal(fields[0][m], fields[1][m])
