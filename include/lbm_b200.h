@@ -390,6 +390,11 @@ int lbm_aa_list_slab_layout(const LatticeDesc *global, int x0, int x1, int haloL
  * CUDA error code. */
 int lbm_b200_selftest_bounded_wait(unsigned polls, int *status);
 
+/* Gives back the device memory that the library keeps for reuse on the current
+ * device after instances and batches were freed (at most 256 MB). Returns 0 or
+ * a CUDA error code. */
+int lbm_b200_release_memory(void);
+
 /* Selects the CUDA device used by subsequent Init calls of this thread. */
 int lbm_b200_set_device(int device);
 
@@ -434,6 +439,10 @@ const char *lbm_b200_last_error(void);
  * lattice cell, cells x fastest (src/Lattice.h:60-76), obstacle cells skipped. */
 void lbm_b200_get_field(KernelData *kd, LatticeDesc *ld, double *out);
 void lbm_b200_set_field(KernelData *kd, LatticeDesc *ld, const double *in);
+
+/* The same 19 PDFs in every fluid cell (as lbm_b200_set_field of a field that
+ * repeats them, without the field). */
+void lbm_b200_set_uniform(KernelData *kd, LatticeDesc *ld, const double *pdfs);
 
 /* Host-built list layout of a list-kernel instance: fluid-node numbering
  * (nX*nY*nZ entries, obstacles 0xffffffff), adjacency (nFluid*18, the

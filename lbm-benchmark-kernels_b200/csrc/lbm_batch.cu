@@ -14,6 +14,7 @@
 #include "../../include/lbm_b200.h"
 #include "lbm_batch.cuh"
 #include "lbm_host.h"
+#include "lbm_mem.cuh"
 
 namespace {
 
@@ -119,11 +120,11 @@ int publish(Batch* b) {
     // records are reallocated: graphs captured with the old table go
     BCK(cudaStreamSynchronize(b->stream));
     drop_graphs(b);
-    cudaFree(b->dTiles);
+    lbm::dev_free(b->dTiles);
     b->dTiles = nullptr;
     b->tileCap = 0;
     const int cap = std::min(b->maxTiles, std::max(b->nTiles + b->nTiles / 2, 1024));
-    BCK(cudaMalloc(&b->dTiles, sizeof(lbm::BatchTile) * (size_t)cap));
+    BCK(lbm::dev_alloc(&b->dTiles, sizeof(lbm::BatchTile) * (size_t)cap));
     b->tileCap = cap;
   }
   // the grid of one-block-per-tile launches keeps some headroom, so that
@@ -235,14 +236,16 @@ void* lbm_batch_create(int storage, double budgetGB, int maxDomains) {
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&b->numSMs, cudaDevAttrMultiProcessorCount, dev);
   bool ok = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) == cudaSuccess &&
-            cudaMalloc(&b->dDoms, sizeof(lbm::BatchDomain) * b->maxSlots) == cudaSuccess &&
-            cudaMalloc(&b->dTileDom, sizeof(int) * b->maxTiles) == cudaSuccess &&
-            cudaMalloc(&b->dNTiles, sizeof(int)) == cudaSuccess && cudaMalloc(&b->dErr, sizeof(int)) == cudaSuccess &&
-            cudaMalloc(&b->dPartials, sizeof(double) * 4 * (size_t)b->maxTiles) == cudaSuccess &&
-            cudaMalloc(&b->dDomTileStart, sizeof(int) * b->maxSlots) == cudaSuccess &&
-            cudaMalloc(&b->dDomTileCount, sizeof(int) * b->maxSlots) == cudaSuccess &&
-            cudaMalloc(&b->dMoments, sizeof(double) * 4 * b->maxSlots) == cudaSuccess &&
-            cudaMemset(b->dErr, 0, sizeof(int)) == cudaSuccess && cudaMemset(b->dNTiles, 0, sizeof(int)) == cudaSuccess;
+            lbm::dev_alloc(&b->dDoms, sizeof(lbm::BatchDomain) * b->maxSlots) == cudaSuccess &&
+            lbm::dev_alloc(&b->dTileDom, sizeof(int) * b->maxTiles) == cudaSuccess &&
+            lbm::dev_alloc(&b->dNTiles, sizeof(int)) == cudaSuccess &&
+            lbm::dev_alloc(&b->dErr, sizeof(int)) == cudaSuccess &&
+            lbm::dev_alloc(&b->dPartials, sizeof(double) * 4 * (size_t)b->maxTiles) == cudaSuccess &&
+            lbm::dev_alloc(&b->dDomTileStart, sizeof(int) * b->maxSlots) == cudaSuccess &&
+            lbm::dev_alloc(&b->dDomTileCount, sizeof(int) * b->maxSlots) == cudaSuccess &&
+            lbm::dev_alloc(&b->dMoments, sizeof(double) * 4 * b->maxSlots) == cudaSuccess &&
+            cudaMemsetAsync(b->dErr, 0, sizeof(int), b->stream) == cudaSuccess &&
+            cudaMemsetAsync(b->dNTiles, 0, sizeof(int), b->stream) == cudaSuccess;
   if (!ok) {
     g_batchError = "device allocation of the batch tables failed";
     delete b;
@@ -258,19 +261,19 @@ void lbm_batch_destroy(void* h) {
   cudaStreamSynchronize(b->stream);
   drop_graphs(b);
   for (auto& s : b->slots) {
-    cudaFree(s.pdfs);
-    cudaFree(s.runs);
-    cudaFree(s.runOff);
+    lbm::dev_free(s.pdfs);
+    lbm::dev_free(s.runs);
+    lbm::dev_free(s.runOff);
   }
-  cudaFree(b->dDoms);
-  cudaFree(b->dTileDom);
-  cudaFree(b->dTiles);
-  cudaFree(b->dNTiles);
-  cudaFree(b->dErr);
-  cudaFree(b->dPartials);
-  cudaFree(b->dDomTileStart);
-  cudaFree(b->dDomTileCount);
-  cudaFree(b->dMoments);
+  lbm::dev_free(b->dDoms);
+  lbm::dev_free(b->dTileDom);
+  lbm::dev_free(b->dTiles);
+  lbm::dev_free(b->dNTiles);
+  lbm::dev_free(b->dErr);
+  lbm::dev_free(b->dPartials);
+  lbm::dev_free(b->dDomTileStart);
+  lbm::dev_free(b->dDomTileCount);
+  lbm::dev_free(b->dMoments);
   cudaStreamDestroy(b->stream);
   delete b;
 }
@@ -296,16 +299,16 @@ int lbm_batch_add(void* h, const LatticeDesc* ld, double omega, double lambda, d
   d = DomainSlot();
   const long ncell = (long)ld->Dims[0] * ld->Dims[1] * ld->Dims[2];
   d.grid.resize(ncell);
-  BCK(cudaMalloc(&d.pdfs, (size_t)nCells * Q * b->elemBytes));
+  BCK(lbm::dev_alloc(&d.pdfs, (size_t)nCells * Q * b->elemBytes));
   uint32_t* adj = nullptr;
-  BCK(cudaMalloc(&adj, (size_t)nCells * QM * 4));
+  BCK(lbm::dev_alloc(&adj, (size_t)nCells * QM * 4));
   // numbering and adjacency built on the device (lbm_build.cu); padding
   // nodes then point at their own slots so that every entry is in range;
   // the steps read the run-compressed form, built from it
   int* dMask = nullptr;
   uint32_t* dGrid = nullptr;
-  BCK(cudaMallocAsync(&dMask, sizeof(int) * ncell, b->stream));
-  BCK(cudaMallocAsync(&dGrid, sizeof(uint32_t) * ncell, b->stream));
+  BCK(lbm::dev_alloc(&dMask, sizeof(int) * ncell));
+  BCK(lbm::dev_alloc(&dGrid, sizeof(uint32_t) * ncell));
   BCK(cudaMemcpyAsync(dMask, ld->Lattice, sizeof(int) * ncell, cudaMemcpyHostToDevice, b->stream));
   const int blk[3] = {0, 0, 0}, per[3] = {ld->PeriodicX, ld->PeriodicY, ld->PeriodicZ};
   const char* berr = "";
@@ -315,17 +318,18 @@ int lbm_batch_add(void* h, const LatticeDesc* ld, double omega, double lambda, d
     lbm::batch_pad_adjacency(adj, nFluid, nCells, b->stream);
     BCK(cudaMemcpyAsync(d.grid.data(), dGrid, sizeof(uint32_t) * ncell, cudaMemcpyDeviceToHost, b->stream));
   }
-  cudaFreeAsync(dGrid, b->stream);
-  cudaFreeAsync(dMask, b->stream);
-  BCK(cudaStreamSynchronize(b->stream));
+  const cudaError_t built = cudaStreamSynchronize(b->stream);
+  lbm::dev_free(dGrid);
+  lbm::dev_free(dMask);
+  BCK(built);
   int rrc = 0;
   size_t runBytes = 0;
   if (nf == nFluid) rrc = lbm::list_runs_device(adj, (int)nCells, b->stream, &d.runs, &d.runOff, &runBytes);
-  cudaFree(adj);
+  lbm::dev_free(adj);
   if (nf != nFluid || rrc) {
     g_batchError = rrc ? "building the run-compressed adjacency failed"
                        : (nf < 0 ? berr : "the mask's fluid cell count differs from the lattice's");
-    cudaFree(d.pdfs);
+    lbm::dev_free(d.pdfs);
     d = DomainSlot();
     return -6;
   }
@@ -354,9 +358,9 @@ int lbm_batch_remove(void* h, int slot) {
   if (slot < 0 || slot >= b->maxSlots || !b->slots[slot].active) return -1;
   BCK(cudaStreamSynchronize(b->stream));
   DomainSlot& d = b->slots[slot];
-  cudaFree(d.pdfs);
-  cudaFree(d.runs);
-  cudaFree(d.runOff);
+  lbm::dev_free(d.pdfs);
+  lbm::dev_free(d.runs);
+  lbm::dev_free(d.runOff);
   b->used -= d.bytes;
   d = DomainSlot();
   return publish(b);

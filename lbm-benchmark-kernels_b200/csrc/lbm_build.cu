@@ -20,6 +20,7 @@
 #include "../../include/lbm_b200.h"
 #include "lbm_d3q19.cuh"
 #include "lbm_kernels.cuh"
+#include "lbm_mem.cuh"
 
 namespace lbm {
 
@@ -132,10 +133,10 @@ long long list_build_device(const int* mask, const int dims[3], const int period
   long long count = -1;
   uint32_t last[2] = {0, 0};
   const unsigned blocks = (unsigned)((g.n + 255) / 256);
-  cudaError_t e = cudaMallocAsync(&flag, sizeof(uint32_t) * g.n, s);
-  if (e == cudaSuccess) e = cudaMallocAsync(&node, sizeof(uint32_t) * g.n, s);
+  cudaError_t e = dev_alloc(&flag, sizeof(uint32_t) * g.n);
+  if (e == cudaSuccess) e = dev_alloc(&node, sizeof(uint32_t) * g.n);
   if (e == cudaSuccess) e = cub::DeviceScan::ExclusiveSum(nullptr, tmpBytes, flag, node, (int)g.n, s);
-  if (e == cudaSuccess) e = cudaMallocAsync(&tmp, tmpBytes, s);
+  if (e == cudaSuccess) e = dev_alloc(&tmp, tmpBytes);
   if (e == cudaSuccess) {
     k_build_flags<<<blocks, 256, 0, s>>>(g, mask, flag, grid);
     e = cudaGetLastError();
@@ -158,9 +159,10 @@ long long list_build_device(const int* mask, const int dims[3], const int period
     e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   }
-  cudaFreeAsync(tmp, s);
-  cudaFreeAsync(node, s);
-  cudaFreeAsync(flag, s);
+  cudaStreamSynchronize(s);
+  dev_free(tmp);
+  dev_free(node);
+  dev_free(flag);
   if (e != cudaSuccess) {
     *err = cudaGetErrorString(e);
     return -1;
@@ -236,11 +238,11 @@ int list_runs_device(const uint32_t* adj, int nFluid, cudaStream_t s, uint32_t**
   void* tmp = nullptr;
   size_t tmpBytes = 0;
   uint32_t total = 0;
-  cudaError_t e = cudaMalloc(runOff, sizeof(uint32_t) * (nTiles + 1));
-  if (e == cudaSuccess) e = cudaMallocAsync(&mask, sizeof(uint32_t) * (size_t)(nTiles > 0 ? nTiles : 1) * 8, s);
-  if (e == cudaSuccess) e = cudaMallocAsync(&size16, sizeof(uint32_t) * (nTiles + 1), s);
+  cudaError_t e = dev_alloc(runOff, sizeof(uint32_t) * (nTiles + 1));
+  if (e == cudaSuccess) e = dev_alloc(&mask, sizeof(uint32_t) * (size_t)(nTiles > 0 ? nTiles : 1) * 8);
+  if (e == cudaSuccess) e = dev_alloc(&size16, sizeof(uint32_t) * (nTiles + 1));
   if (e == cudaSuccess) e = cub::DeviceScan::ExclusiveSum(nullptr, tmpBytes, size16, *runOff, nTiles + 1, s);
-  if (e == cudaSuccess) e = cudaMallocAsync(&tmp, tmpBytes, s);
+  if (e == cudaSuccess) e = dev_alloc(&tmp, tmpBytes);
   if (e == cudaSuccess && nTiles > 0) {
     k_run_heads<<<nTiles, kListTile, 0, s>>>(adj, nFluid, mask);
     e = cudaGetLastError();
@@ -254,7 +256,7 @@ int list_runs_device(const uint32_t* adj, int nFluid, cudaStream_t s, uint32_t**
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e == cudaSuccess) {
     *runBytes = (size_t)(total > 0 ? total : 1) * 16;
-    e = cudaMalloc(runs, *runBytes);
+    e = dev_alloc(runs, *runBytes);
   }
   if (e == cudaSuccess) e = cudaMemsetAsync(*runs, 0, *runBytes, s);
   if (e == cudaSuccess && nTiles > 0) {
@@ -262,13 +264,13 @@ int list_runs_device(const uint32_t* adj, int nFluid, cudaStream_t s, uint32_t**
     e = cudaGetLastError();
   }
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  cudaFreeAsync(tmp, s);
-  cudaFreeAsync(size16, s);
-  cudaFreeAsync(mask, s);
   cudaStreamSynchronize(s);
+  dev_free(tmp);
+  dev_free(size16);
+  dev_free(mask);
   if (e != cudaSuccess) {
-    cudaFree(*runs);
-    cudaFree(*runOff);
+    dev_free(*runs);
+    dev_free(*runOff);
     *runs = nullptr;
     *runOff = nullptr;
     return (int)e;
@@ -355,10 +357,10 @@ int lbm_b200_list_build(const LatticeDesc* ld, int pull, const int blk[3], int n
   long long count = -1;
   const char* err = "";
   cudaError_t e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
-  if (e == cudaSuccess) e = cudaMalloc(&dMask, sizeof(int) * n);
-  if (e == cudaSuccess) e = cudaMalloc(&dGrid, sizeof(uint32_t) * n);
-  if (e == cudaSuccess) e = cudaMalloc(&dAdj, sizeof(uint32_t) * adjN);
-  if (e == cudaSuccess) e = cudaMemcpy(dMask, ld->Lattice, sizeof(int) * n, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = lbm::dev_alloc(&dMask, sizeof(int) * n);
+  if (e == cudaSuccess) e = lbm::dev_alloc(&dGrid, sizeof(uint32_t) * n);
+  if (e == cudaSuccess) e = lbm::dev_alloc(&dAdj, sizeof(uint32_t) * adjN);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(dMask, ld->Lattice, sizeof(int) * n, cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess) {
     count = lbm::list_build_device(dMask, ld->Dims, per, pull, blk, nCells, dGrid, dAdj,
                                    ld->nFluid > 0 ? ld->nFluid : 0, s, &err);
@@ -369,9 +371,10 @@ int lbm_b200_list_build(const LatticeDesc* ld, int pull, const int blk[3], int n
     if (e == cudaSuccess && count > 0) e = cudaMemcpy(adj, dAdj, sizeof(uint32_t) * count * lbm::QM, cudaMemcpyDeviceToHost);
   }
   if (e != cudaSuccess) std::fprintf(stderr, "lbm_b200_list_build: %s\n", cudaGetErrorString(e));
-  cudaFree(dAdj);
-  cudaFree(dGrid);
-  cudaFree(dMask);
+  if (s) cudaStreamSynchronize(s);
+  lbm::dev_free(dAdj);
+  lbm::dev_free(dGrid);
+  lbm::dev_free(dMask);
   if (s) cudaStreamDestroy(s);
   if (e != cudaSuccess) return -1;
   return (int)count;

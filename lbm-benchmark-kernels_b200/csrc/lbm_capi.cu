@@ -24,6 +24,7 @@
 #include "../../include/lbm_b200.h"
 #include "lbm_host.h"
 #include "lbm_kernels.cuh"
+#include "lbm_mem.cuh"
 
 namespace {
 
@@ -53,6 +54,7 @@ struct Gpu {
   // pinned host mirror of the current PDF array (FP64 whatever the storage)
   double* mirror;
   size_t mirrorElems;
+  int* errHost;  // page-locked copy of the device error word (behind the mirror)
   bool dirty;
   int storage;       // lbm::kStoreF64 / F32 / F16
   size_t elemBytes;  // bytes per stored PDF
@@ -112,7 +114,7 @@ struct Gpu {
   int openFaces;
 
   double* dMomOut;  // 4 doubles for lbm_b200_instance_moments (allocated on first use)
-  double* dMomPartials;  // its per-block partial sums for reduced storage (first use)
+  double* dMomPartials;  // its per-block partial sums (first use)
 
   // last Kernel call
   double lastDeviceMs;
@@ -594,11 +596,8 @@ void download(Gpu* g) {
   if (g->storage != lbm::kStoreF64) raw_to_mirror(g);
 }
 
-// Reads the device error word (synchronous); a non-zero word marks the
-// device state as lost. Returns the word.
-int read_device_error(Gpu* g) {
-  int err = 0;
-  LBM_CK(cudaMemcpy(&err, g->dErr, sizeof(int), cudaMemcpyDeviceToHost));
+// A non-zero device error word marks the device state as lost.
+int note_device_error(Gpu* g, int err) {
   if (err) {
     g->stateLost = true;
     g_lastError = "a device wait exceeded its limit or a tile was skipped (error word " + std::to_string(err) +
@@ -607,11 +606,11 @@ int read_device_error(Gpu* g) {
   return err;
 }
 
-void check_device_error(Gpu* g) {
-  if (read_device_error(g)) {
-    std::printf("ERROR: %s\n", g_lastError.c_str());
-    std::exit(1);
-  }
+// Reads the device error word (synchronous). Returns the word.
+int read_device_error(Gpu* g) {
+  int err = 0;
+  LBM_CK(cudaMemcpy(&err, g->dErr, sizeof(int), cudaMemcpyDeviceToHost));
+  return note_device_error(g, err);
 }
 
 // Steps refuse to run on a lost device state (see Gpu::stateLost).
@@ -669,13 +668,17 @@ void cb_kernel(LatticeDesc* ld, KernelData* kd, CaseData* cd) {
   g->lastLaunches = cd->VtkOutput ? enqueue_steps_vtk(ld, g, cd, t) : enqueue_steps(g, t, cd->MaxIterations);
   LBM_CK(cudaGetLastError());
   LBM_CK(cudaEventRecord(g->ev1, g->stream));
+  LBM_CK(cudaMemcpyAsync(g->errHost, g->dErr, sizeof(int), cudaMemcpyDeviceToHost, g->stream));
   LBM_CK(cudaStreamSynchronize(g->stream));
   auto w1 = std::chrono::steady_clock::now();
   float ms = 0.f;
   LBM_CK(cudaEventElapsedTime(&ms, g->ev0, g->ev1));
   g->lastDeviceMs = ms;
   kd->Duration = std::chrono::duration<double>(w1 - w0).count();
-  check_device_error(g);
+  if (note_device_error(g, *g->errHost)) {
+    std::printf("ERROR: %s\n", g_lastError.c_str());
+    std::exit(1);
+  }
   download(g);
   if (cd->VtkOutput) vtk_or_exit(ld, kd, cd, cd->MaxIterations);
 }
@@ -707,8 +710,8 @@ constexpr double kPairLateShare = 0.1;
 bool schedule_resident(Gpu* g, size_t nTiles, int most) {
   if (nTiles == 0 || nTiles > (size_t)most) return false;
   g->pairTiles = static_cast<uint32_t>(nTiles);
-  LBM_CK(cudaMalloc(&g->dMeet, sizeof(uint32_t)));
-  LBM_CK(cudaMemset(g->dMeet, 0, sizeof(uint32_t)));
+  LBM_CK(lbm::dev_alloc(&g->dMeet, sizeof(uint32_t)));
+  LBM_CK(cudaMemsetAsync(g->dMeet, 0, sizeof(uint32_t), g->stream));
   return true;
 }
 
@@ -724,10 +727,10 @@ void pair_upload(Gpu* g, const std::vector<lbm::PairRec<R>>& items, size_t nTile
   g->pairTiles = static_cast<uint32_t>(nTiles);
   g->pairItems = static_cast<uint32_t>(items.size());
   g->pairGroups = static_cast<uint32_t>((nTiles + (1u << lbm::kPairGroupShift) - 1) >> lbm::kPairGroupShift);
-  LBM_CK(cudaMalloc(&g->dPairCount, sizeof(uint32_t) * (g->pairGroups + 2)));
-  LBM_CK(cudaMemset(g->dPairCount, 0, sizeof(uint32_t) * (g->pairGroups + 2)));
-  LBM_CK(cudaMalloc(&g->dPairItems, sizeof(lbm::PairRec<R>) * items.size()));
-  LBM_CK(cudaMemcpy(g->dPairItems, items.data(), sizeof(lbm::PairRec<R>) * items.size(), cudaMemcpyHostToDevice));
+  LBM_CK(lbm::dev_alloc(&g->dPairCount, sizeof(uint32_t) * (g->pairGroups + 2)));
+  LBM_CK(cudaMemsetAsync(g->dPairCount, 0, sizeof(uint32_t) * (g->pairGroups + 2), g->stream));
+  LBM_CK(lbm::dev_alloc(&g->dPairItems, sizeof(lbm::PairRec<R>) * items.size()));
+  LBM_CK(cudaMemcpyAsync(g->dPairItems, items.data(), sizeof(lbm::PairRec<R>) * items.size(), cudaMemcpyHostToDevice, g->stream));
 }
 
 void schedule_list_pairs(Gpu* g) {
@@ -736,13 +739,13 @@ void schedule_list_pairs(Gpu* g) {
   if (schedule_resident(g, (size_t)nTiles, lbm::list_resident_tiles(g->storage))) return;
   uint32_t* dReach = nullptr;
   std::vector<uint32_t> reach(6 * (size_t)nTiles), off((size_t)nTiles + 1);
-  LBM_CK(cudaMallocAsync(&dReach, sizeof(uint32_t) * reach.size(), g->stream));
+  LBM_CK(lbm::dev_alloc(&dReach, sizeof(uint32_t) * reach.size()));
   lbm::list_tile_reach(g->dAdj, g->nFluid, g->nCells, dReach, g->stream);
   LBM_CK(cudaGetLastError());
   LBM_CK(cudaMemcpyAsync(reach.data(), dReach, sizeof(uint32_t) * reach.size(), cudaMemcpyDeviceToHost, g->stream));
   LBM_CK(cudaMemcpyAsync(off.data(), g->dRunOff, sizeof(uint32_t) * off.size(), cudaMemcpyDeviceToHost, g->stream));
-  LBM_CK(cudaFreeAsync(dReach, g->stream));
   LBM_CK(cudaStreamSynchronize(g->stream));
+  lbm::dev_free(dReach);
   const int resident = lbm::list_pair_resident(g->storage);
   const int margin = g->storage == lbm::kStoreF64 ? resident : resident * 3 / 2;
   std::vector<lbm::PairItem> items;
@@ -783,12 +786,12 @@ void build_odd_items(Gpu* g, const uint32_t* link) {
   lbm::aa_interior_items(aa, link, items, cells);
   g->nOddItems = (int)items.size();
   if (!items.empty()) {
-    LBM_CK(cudaMalloc(&g->dOddItems, sizeof(int) * items.size()));
-    LBM_CK(cudaMemcpy(g->dOddItems, items.data(), sizeof(int) * items.size(), cudaMemcpyHostToDevice));
+    LBM_CK(lbm::dev_alloc(&g->dOddItems, sizeof(int) * items.size()));
+    LBM_CK(cudaMemcpyAsync(g->dOddItems, items.data(), sizeof(int) * items.size(), cudaMemcpyHostToDevice, g->stream));
   }
   if (!cells.empty()) {
-    LBM_CK(cudaMalloc(&g->dOddCells, sizeof(int) * cells.size()));
-    LBM_CK(cudaMemcpy(g->dOddCells, cells.data(), sizeof(int) * cells.size(), cudaMemcpyHostToDevice));
+    LBM_CK(lbm::dev_alloc(&g->dOddCells, sizeof(int) * cells.size()));
+    LBM_CK(cudaMemcpyAsync(g->dOddCells, cells.data(), sizeof(int) * cells.size(), cudaMemcpyHostToDevice, g->stream));
   }
 }
 
@@ -797,7 +800,7 @@ void build_odd_items(Gpu* g, const uint32_t* link) {
 void need_odd_items(Gpu* g) {
   if (g->kind != kAa || g->oddItemsBuilt) return;
   std::vector<uint32_t> link((size_t)g->dstride);
-  LBM_CK(cudaMemcpy(link.data(), g->dLink, sizeof(uint32_t) * link.size(), cudaMemcpyDeviceToHost));
+  LBM_CK(cudaMemcpyAsync(link.data(), g->dLink, sizeof(uint32_t) * link.size(), cudaMemcpyDeviceToHost));
   build_odd_items(g, link.data());
 }
 
@@ -834,8 +837,8 @@ Gpu* gpu_new(Kind kind, LatticeDesc* ld, Parameters* params, const SlabSpec* sla
   LBM_CK(cudaStreamCreateWithFlags(&g->stream, cudaStreamNonBlocking));
   LBM_CK(cudaEventCreate(&g->ev0));
   LBM_CK(cudaEventCreate(&g->ev1));
-  LBM_CK(cudaMalloc(&g->dErr, sizeof(int)));
-  LBM_CK(cudaMemset(g->dErr, 0, sizeof(int)));
+  LBM_CK(lbm::dev_alloc(&g->dErr, sizeof(int)));
+  LBM_CK(cudaMemsetAsync(g->dErr, 0, sizeof(int), g->stream));
 
   KernelData* kd = &g->kd;
   kd->Dims[0] = ld->Dims[0];
@@ -887,13 +890,13 @@ Gpu* gpu_new(Kind kind, LatticeDesc* ld, Parameters* params, const SlabSpec* sla
     } else {
       lbmh_aa_links(ld, g->xs, g->pitch, lbm::kZOff, link);
     }
-    LBM_CK(cudaMalloc(&g->dLink, sizeof(uint32_t) * (size_t)g->dstride));
-    LBM_CK(cudaMemcpy(g->dLink, link, sizeof(uint32_t) * (size_t)g->dstride, cudaMemcpyHostToDevice));
-    LBM_CK(cudaMalloc(&g->dF, sizeof(double) * g->mirrorElems));
-    LBM_CK(cudaMemset(g->dF, 0, sizeof(double) * g->mirrorElems));
+    LBM_CK(lbm::dev_alloc(&g->dLink, sizeof(uint32_t) * (size_t)g->dstride));
+    LBM_CK(cudaMemcpyAsync(g->dLink, link, sizeof(uint32_t) * (size_t)g->dstride, cudaMemcpyHostToDevice, g->stream));
+    LBM_CK(lbm::dev_alloc(&g->dF, sizeof(double) * g->mirrorElems));
+    LBM_CK(cudaMemsetAsync(g->dF, 0, sizeof(double) * g->mirrorElems, g->stream));
     if (kind != kAa) {
-      LBM_CK(cudaMalloc(&g->dG, sizeof(double) * g->mirrorElems));
-      LBM_CK(cudaMemset(g->dG, 0, sizeof(double) * g->mirrorElems));
+      LBM_CK(lbm::dev_alloc(&g->dG, sizeof(double) * g->mirrorElems));
+      LBM_CK(cudaMemsetAsync(g->dG, 0, sizeof(double) * g->mirrorElems, g->stream));
     }
     if (kind == kAa && !slab) schedule_aa_pairs(g, ld);
     if (kind == kAa && slab) build_odd_items(g, link);
@@ -915,8 +918,8 @@ Gpu* gpu_new(Kind kind, LatticeDesc* ld, Parameters* params, const SlabSpec* sla
     const size_t adjElems = (size_t)(nTiles > 0 ? nTiles : 1) * lbm::kListTile * QM;
     // numbering and adjacency built on the device (lbm_build.cu); the host
     // keeps the numbering for GetNode/SetNode
-    LBM_CK(cudaMalloc(&g->dAdj, sizeof(uint32_t) * adjElems));
-    LBM_CK(cudaMemset(g->dAdj, 0, sizeof(uint32_t) * adjElems));
+    LBM_CK(lbm::dev_alloc(&g->dAdj, sizeof(uint32_t) * adjElems));
+    LBM_CK(cudaMemsetAsync(g->dAdj, 0, sizeof(uint32_t) * adjElems, g->stream));
     if (slab && slab->list) {
       // a list-AA slab: the host-built layout with ghost nodes after the owned ones
       LbmhListSlab* ls = slab->list;
@@ -925,15 +928,15 @@ Gpu* gpu_new(Kind kind, LatticeDesc* ld, Parameters* params, const SlabSpec* sla
       g->grid = ls->grid;
       ls->grid = nullptr;
       if (ls->nOwned > 0)
-        LBM_CK(cudaMemcpy(g->dAdj, ls->adj, sizeof(uint32_t) * QM * (size_t)ls->nOwned, cudaMemcpyHostToDevice));
+        LBM_CK(cudaMemcpyAsync(g->dAdj, ls->adj, sizeof(uint32_t) * QM * (size_t)ls->nOwned, cudaMemcpyHostToDevice, g->stream));
       for (int side = 0; side < 2; ++side)
         for (int list = 0; list < 2; ++list) {
           const uint32_t* h = list == 0 ? ls->own[side] : ls->ghost[side];
           const long n = list == 0 ? ls->nOwnSlots[side] : ls->nGhostSlots[side];
           g->nHalo[side][list] = h ? n : -1;
           if (h && n > 0) {
-            LBM_CK(cudaMalloc(&g->dHalo[side][list], sizeof(uint32_t) * (size_t)n));
-            LBM_CK(cudaMemcpy(g->dHalo[side][list], h, sizeof(uint32_t) * (size_t)n, cudaMemcpyHostToDevice));
+            LBM_CK(lbm::dev_alloc(&g->dHalo[side][list], sizeof(uint32_t) * (size_t)n));
+            LBM_CK(cudaMemcpyAsync(g->dHalo[side][list], h, sizeof(uint32_t) * (size_t)n, cudaMemcpyHostToDevice, g->stream));
           }
         }
       g->listSlab = true;
@@ -943,9 +946,9 @@ Gpu* gpu_new(Kind kind, LatticeDesc* ld, Parameters* params, const SlabSpec* sla
       // a slab's layout came from the host builder above
       int* dMask = nullptr;
       uint32_t* dGrid = nullptr;
-      LBM_CK(cudaMalloc(&dMask, sizeof(int) * ncell));
-      LBM_CK(cudaMalloc(&dGrid, sizeof(uint32_t) * ncell));
-      LBM_CK(cudaMemcpy(dMask, ld->Lattice, sizeof(int) * ncell, cudaMemcpyHostToDevice));
+      LBM_CK(lbm::dev_alloc(&dMask, sizeof(int) * ncell));
+      LBM_CK(lbm::dev_alloc(&dGrid, sizeof(uint32_t) * ncell));
+      LBM_CK(cudaMemcpyAsync(dMask, ld->Lattice, sizeof(int) * ncell, cudaMemcpyHostToDevice, g->stream));
       const int per3[3] = {ld->PeriodicX, ld->PeriodicY, ld->PeriodicZ};
       const char* berr = "";
       const long long nf = lbm::list_build_device(dMask, ld->Dims, per3, pull ? 1 : 0, a.blk, nCells, dGrid, g->dAdj,
@@ -955,8 +958,8 @@ Gpu* gpu_new(Kind kind, LatticeDesc* ld, Parameters* params, const SlabSpec* sla
         std::exit(1);
       }
       LBM_CK(cudaMemcpy(g->grid, dGrid, sizeof(uint32_t) * ncell, cudaMemcpyDeviceToHost));
-      LBM_CK(cudaFree(dGrid));
-      LBM_CK(cudaFree(dMask));
+      lbm::dev_free(dGrid);
+      lbm::dev_free(dMask);
     }
     {
       // the adjacency-driven steps read the run-compressed form (the full
@@ -969,11 +972,11 @@ Gpu* gpu_new(Kind kind, LatticeDesc* ld, Parameters* params, const SlabSpec* sla
     }
     if (kind == kListAa && !g->listSlab) schedule_list_pairs(g);
     g->mirrorElems = (size_t)Q * nCells;
-    LBM_CK(cudaMalloc(&g->dF, g->elemBytes * g->mirrorElems));
-    LBM_CK(cudaMemset(g->dF, 0, g->elemBytes * g->mirrorElems));
+    LBM_CK(lbm::dev_alloc(&g->dF, g->elemBytes * g->mirrorElems));
+    LBM_CK(cudaMemsetAsync(g->dF, 0, g->elemBytes * g->mirrorElems, g->stream));
     if (two_grid(kind)) {
-      LBM_CK(cudaMalloc(&g->dG, sizeof(double) * g->mirrorElems));
-      LBM_CK(cudaMemset(g->dG, 0, sizeof(double) * g->mirrorElems));
+      LBM_CK(lbm::dev_alloc(&g->dG, sizeof(double) * g->mirrorElems));
+      LBM_CK(cudaMemsetAsync(g->dG, 0, sizeof(double) * g->mirrorElems, g->stream));
     }
     kd->GlobalDims[0] = ld->Dims[0];
     kd->GlobalDims[1] = ld->Dims[1];
@@ -985,15 +988,18 @@ Gpu* gpu_new(Kind kind, LatticeDesc* ld, Parameters* params, const SlabSpec* sla
     kd->LoopBalance = two_grid(kind) ? pb + ab : (pb + (pb + ab)) / 2.0;
   }
 
-  LBM_CK(cudaMallocHost(&g->mirror, sizeof(double) * g->mirrorElems));
-  std::memset(g->mirror, 0, sizeof(double) * g->mirrorElems);
+  LBM_CK(lbm::host_alloc(&g->mirror, sizeof(double) * (g->mirrorElems + 1)));
+  g->errHost = reinterpret_cast<int*>(g->mirror + g->mirrorElems);
   g->dirty = false;  // device and mirror both hold zeros
   if (g->storage != lbm::kStoreF64) {
-    LBM_CK(cudaMallocHost(&g->rawStage, g->elemBytes * g->mirrorElems));
-    // the device holds raw zeros; keep the mirror consistent with them
-    LBM_CK(cudaMemcpy(g->rawStage, g->dF, g->elemBytes * g->mirrorElems, cudaMemcpyDeviceToHost));
+    LBM_CK(lbm::host_alloc(&g->rawStage, g->elemBytes * g->mirrorElems));
+    // the device holds raw zeros, as the staging buffer; keep the mirror
+    // consistent with them
     raw_to_mirror(g);
   }
+  // the device arrays are filled on the instance's stream; from here on other
+  // streams may use them
+  LBM_CK(cudaStreamSynchronize(g->stream));
   kd->Pdfs[0] = g->mirror;
   kd->Pdfs[1] = nullptr;
   kd->PdfsActive = g->mirror;
@@ -1003,28 +1009,30 @@ Gpu* gpu_new(Kind kind, LatticeDesc* ld, Parameters* params, const SlabSpec* sla
 void gpu_free(KernelData** kernelData) {
   if (kernelData == nullptr || *kernelData == nullptr) return;
   Gpu* g = reinterpret_cast<Gpu*>(*kernelData);
-  cudaStreamSynchronize(g->stream);
-  cudaFree(g->dF);
-  cudaFree(g->dG);
-  cudaFree(g->dLink);
-  cudaFree(g->dOddItems);
-  cudaFree(g->dVerify);
-  cudaFree(g->dVerifyBase);
-  cudaFree(g->dOddCells);
+  // all streams: slab steps, or a caller that reads the device state, may
+  // still use the memory on another one
+  cudaDeviceSynchronize();
+  lbm::dev_free(g->dF);
+  lbm::dev_free(g->dG);
+  lbm::dev_free(g->dLink);
+  lbm::dev_free(g->dOddItems);
+  lbm::dev_free(g->dVerify);
+  lbm::dev_free(g->dVerifyBase);
+  lbm::dev_free(g->dOddCells);
   std::free(g->sliceMask);
-  cudaFree(g->dAdj);
-  cudaFree(g->dRuns);
-  cudaFree(g->dRunOff);
-  cudaFree(g->dPairItems);
-  cudaFree(g->dPairCount);
-  cudaFree(g->dMeet);
+  lbm::dev_free(g->dAdj);
+  lbm::dev_free(g->dRuns);
+  lbm::dev_free(g->dRunOff);
+  lbm::dev_free(g->dPairItems);
+  lbm::dev_free(g->dPairCount);
+  lbm::dev_free(g->dMeet);
   for (int side = 0; side < 2; ++side)
-    for (int list = 0; list < 2; ++list) cudaFree(g->dHalo[side][list]);
-  cudaFree(g->dErr);
-  cudaFree(g->dMomOut);
-  cudaFree(g->dMomPartials);
-  cudaFreeHost(g->mirror);
-  cudaFreeHost(g->rawStage);
+    for (int list = 0; list < 2; ++list) lbm::dev_free(g->dHalo[side][list]);
+  lbm::dev_free(g->dErr);
+  lbm::dev_free(g->dMomOut);
+  lbm::dev_free(g->dMomPartials);
+  lbm::host_free(g->mirror);
+  lbm::host_free(g->rawStage);
   cudaEventDestroy(g->ev0);
   cudaEventDestroy(g->ev1);
   cudaStreamDestroy(g->stream);
@@ -1233,8 +1241,8 @@ int lbm_b200_verify_device(LatticeDesc* ld, KernelData* kd, CaseData* cd, int wr
     }
   }
   cudaError_t e = cudaSuccess;
-  if (!g->dVerify) e = cudaMalloc(&g->dVerify, sizeof(double) * (n + 1));
-  if (e == cudaSuccess && !g->dVerifyBase) e = cudaMalloc(&g->dVerifyBase, sizeof(long long) * n);
+  if (!g->dVerify) e = lbm::dev_alloc(&g->dVerify, sizeof(double) * (n + 1));
+  if (e == cudaSuccess && !g->dVerifyBase) e = lbm::dev_alloc(&g->dVerifyBase, sizeof(long long) * n);
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(g->dVerifyBase, base.data(), sizeof(long long) * n, cudaMemcpyHostToDevice, g->stream);
   if (e == cudaSuccess) {
@@ -1728,36 +1736,34 @@ int lbm_b200_device_state(KernelData* kd, double** pdfs, long long* nCells, int*
   return 0;
 }
 
-int lbm_b200_moments_device(const double* pdfs, long long nCells, int nFluid, double* out_device, void* stream);
-
 int lbm_b200_instance_moments(KernelData* kd, double* out) {
   Gpu* g = reinterpret_cast<Gpu*>(kd);
   if (full_array(g->kind)) return -1;
   if (g->dirty) upload_if_dirty(g);
   if (g->dMomOut == nullptr) {
-    cudaError_t e = cudaMalloc(&g->dMomOut, 4 * sizeof(double));
+    cudaError_t e = lbm::dev_alloc(&g->dMomOut, 4 * sizeof(double));
     if (e != cudaSuccess) { g_lastError = cudaGetErrorString(e); return (int)e; }
   }
-  if (g->storage != lbm::kStoreF64) {
-    // reduced storage: FP64 sums of the stored deviations (scratch kept by
-    // the instance)
-    if (g->dMomPartials == nullptr) {
-      cudaError_t e = cudaMalloc(&g->dMomPartials, sizeof(double) * 4 * lbm::moment_blocks(g->nFluid));
-      if (e != cudaSuccess) { g_lastError = cudaGetErrorString(e); return (int)e; }
-    }
-    lbm::moments_enqueue_lp(g->dF, g->storage, g->nCells, g->nFluid, g->dMomPartials, g->dMomOut, g->stream);
-    cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
-    if (e == cudaSuccess) e = cudaMemcpy(out, g->dMomOut, 4 * sizeof(double), cudaMemcpyDeviceToHost);
-    if (e != cudaSuccess) g_lastError = cudaGetErrorString(e);
-    if (e == cudaSuccess && (g->stateLost || read_device_error(g))) return -4;  // sums of a lost state
+  // the sums' scratch is kept by the instance
+  cudaError_t e = cudaSuccess;
+  if (g->dMomPartials == nullptr)
+    e = lbm::dev_alloc(&g->dMomPartials, sizeof(double) * 4 * lbm::moment_blocks(g->nFluid));
+  if (e == cudaSuccess) {
+    if (g->storage != lbm::kStoreF64)  // FP64 sums of the stored deviations
+      lbm::moments_enqueue_lp(g->dF, g->storage, g->nCells, g->nFluid, g->dMomPartials, g->dMomOut, g->stream);
+    else
+      lbm::moments_enqueue(current_grid(g), g->nCells, g->nFluid, g->dMomPartials, g->dMomOut, g->stream);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) e = cudaMemcpyAsync(out, g->dMomOut, 4 * sizeof(double), cudaMemcpyDeviceToHost, g->stream);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(g->errHost, g->dErr, sizeof(int), cudaMemcpyDeviceToHost, g->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
+  if (e != cudaSuccess) {
+    g_lastError = cudaGetErrorString(e);
     return (int)e;
   }
-  int rc = lbm_b200_moments_device(current_grid(g), g->nCells, g->nFluid, g->dMomOut, g->stream);
-  if (rc) return rc;
-  cudaError_t e = cudaMemcpy(out, g->dMomOut, 4 * sizeof(double), cudaMemcpyDeviceToHost);
-  if (e == cudaSuccess && (g->stateLost || read_device_error(g))) return -4;  // sums of a lost state
-  return (int)e;
+  if (g->stateLost || note_device_error(g, *g->errHost)) return -4;  // sums of a lost state
+  return 0;
 }
 
 int lbm_b200_set_device(int device) {
@@ -1788,6 +1794,22 @@ void lbm_b200_set_field(KernelData* kd, LatticeDesc* ld, const double* in) {
         if (ld->Lattice[c] == LAT_CELL_OBSTACLE) continue;
         kd->SetNode(kd, x, y, z, const_cast<double*>(in + c * Q));
       }
+}
+
+// One state for every fluid cell: the list planes are filled directly.
+void lbm_b200_set_uniform(KernelData* kd, LatticeDesc* ld, const double* pdfs) {
+  Gpu* g = reinterpret_cast<Gpu*>(kd);
+  if (!full_array(g->kind)) {
+    for (int d = 0; d < Q; ++d) std::fill_n(g->mirror + (size_t)d * g->nCells, g->nFluid, pdfs[d]);
+    g->dirty = true;
+    return;
+  }
+  const int* dims = ld->Dims;
+  for (int z = 0; z < dims[2]; ++z)
+    for (int y = 0; y < dims[1]; ++y)
+      for (int x = 0; x < dims[0]; ++x)
+        if (ld->Lattice[lbmh_lidx(dims, x, y, z)] != LAT_CELL_OBSTACLE)
+          kd->SetNode(kd, x, y, z, const_cast<double*>(pdfs));
 }
 
 // The host-built list layout of a list kernel instance (for parity checks):

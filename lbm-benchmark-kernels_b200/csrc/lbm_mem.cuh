@@ -1,0 +1,38 @@
+// lbm_mem.cuh -- memory of instances and batches.
+//
+// Device memory: cudaMalloc and cudaFree take 0.3-0.5 ms each and wait for the
+// device, and an instance or a batched domain makes a dozen of them. Blocks up
+// to kPoolBlock come from a stream-ordered pool per device instead, which keeps
+// at most kPoolKeep bytes of freed memory (lbm_b200_release_memory gives it
+// back). A block is ready for any stream when dev_alloc returns; dev_free
+// wants the work on it complete, as seen from the host. Safe from several
+// threads.
+//
+// Host memory: page-locked, zeroed. 2 MiB pages make locking about three times
+// as fast as cudaMallocHost (40 MB: 5.8 ms against 17 and 2.7 for clearing it;
+// freeing 1.0 against 4.2).
+#pragma once
+#include <cstddef>
+
+#include <cuda_runtime.h>
+
+namespace lbm {
+
+constexpr size_t kPoolBlock = 64ull << 20;
+constexpr size_t kPoolKeep = 256ull << 20;
+
+cudaError_t dev_alloc(void** p, size_t bytes);
+template <class T>
+cudaError_t dev_alloc(T** p, size_t bytes) {
+  return dev_alloc(reinterpret_cast<void**>(p), bytes);
+}
+void dev_free(void* p);
+
+cudaError_t host_alloc(void** p, size_t bytes);
+template <class T>
+cudaError_t host_alloc(T** p, size_t bytes) {
+  return host_alloc(reinterpret_cast<void**>(p), bytes);
+}
+void host_free(void* p);
+
+}  // namespace lbm

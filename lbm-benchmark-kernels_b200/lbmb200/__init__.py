@@ -286,6 +286,12 @@ class Instance:
         return out.reshape(-1, Q)
 
     def set_field(self, pdfs):
+        if getattr(pdfs, "shape", None) == (self.lattice.mask.size, Q) and pdfs.strides[0] == 0:
+            # one row repeated (np.broadcast_to): no need to write it out
+            row = np.ascontiguousarray(pdfs[0], dtype=np.float64)
+            lib().lbm_b200_set_uniform(self.kdp, ctypes.byref(self.lattice.desc),
+                                       row.ctypes.data_as(ctypes.POINTER(ctypes.c_double)))
+            return
         pdfs = np.ascontiguousarray(pdfs, dtype=np.float64).reshape(-1)
         lib().lbm_b200_set_field(self.kdp, ctypes.byref(self.lattice.desc),
                                  pdfs.ctypes.data_as(ctypes.POINTER(ctypes.c_double)))
