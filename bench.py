@@ -300,6 +300,17 @@ def _cpu_ranges(cpus):
     return ",".join(out)
 
 
+def two_grid_line(t, nodes, adj_node, peak):
+    """Throughput and HBM fraction of a two-grid row. Two steps in one launch
+    (launches_per_pair 1) have to read and write one grid and write the other;
+    one launch per step reads one grid and writes the other each time."""
+    ms = t["ms"] / t["steps_run"]
+    bpf = (1.5 if t["launches_per_pair"] == 1 else 2) * 19 * 8 + adj_node
+    gbs = bpf * nodes / (ms / 1e3) / 1e9
+    return {"mflups": round(nodes / (ms / 1e3) / 1e6, 1), "step_ms": round(ms, 5), "bytes_per_flup": round(bpf, 2),
+            "achieved_gbs": round(gbs, 1), "frac": round(gbs / peak, 4)}
+
+
 def list_aa_roofline(t, nodes, pdf_bytes, adj_node, peak, names):
     """HBM roofline entry of a list AA row from its per-launch times. One
     launch per pair (fused even and odd step): every PDF has to be read and
@@ -719,26 +730,12 @@ def run_ours(args, dist):
     # single-GPU measurements (every rank would repeat them on its own GPU)
     if not args.no_extra and dist.world == 1:
         extra = {}
-        # pull kernel on the same domain
-        tp = time_kernel(lbmb200, "cuda-list-pull-split-nt-1s-soa", lat, min(args.steps, 200), 3, kargs, dist, "pull")
-        bpf = B_PER_FLUP["even"] + adjacency_bytes_per_node(lbmb200, tp["inst"], lat.n_fluid)
-        tp["inst"].deinit()
-        pm = statistics.mean(tp["per_launch_ms"])
-        extra["cuda-list-pull-split-nt-1s-soa"] = {
-            "mflups": round(lat.n_fluid / (pm / 1e3) / 1e6, 1), "launch_ms": round(pm, 5),
-            "bytes_per_flup": round(bpf, 2),
-            "achieved_gbs": round(bpf * lat.n_fluid / (pm / 1e3) / 1e9, 1),
-            "frac": round(bpf * lat.n_fluid / (pm / 1e3) / 1e9 / peak, 4)}
-        # the two-grid list rows on the same domain (304 B of PDFs plus the adjacency each reads per node update)
-        for kname in ("cuda-list-push-soa", "cuda-list-pull-soa"):
-            tq = time_kernel(lbmb200, kname, lat, min(args.steps, 200), 3, kargs, dist, "pull")
-            bpf = B_PER_FLUP["even"] + adjacency_bytes_per_node(lbmb200, tq["inst"], lat.n_fluid)
+        # the two-grid list rows on the same domain
+        for kname in ("cuda-list-pull-split-nt-1s-soa", "cuda-list-push-soa", "cuda-list-pull-soa"):
+            tq = time_kernel(lbmb200, kname, lat, min(args.steps, 200), 4, kargs, dist, "pull")
+            adj = adjacency_bytes_per_node(lbmb200, tq["inst"], lat.n_fluid)
             tq["inst"].deinit()
-            qm = statistics.mean(tq["per_launch_ms"])
-            extra[kname] = {"mflups": round(lat.n_fluid / (qm / 1e3) / 1e6, 1), "launch_ms": round(qm, 5),
-                            "bytes_per_flup": round(bpf, 2),
-                            "achieved_gbs": round(bpf * lat.n_fluid / (qm / 1e3) / 1e9, 1),
-                            "frac": round(bpf * lat.n_fluid / (qm / 1e3) / 1e9 / peak, 4)}
+            extra[kname] = two_grid_line(tq, lat.n_fluid, adj, peak)
         # full-array AA at 256^3: the reference's -geometry fluid with -periodic-x -periodic-y
         # -periodic-z, and -geometry channel (x periodic, walls in y and z)
         for key, geo, per_flags in (("cuda-aa-soa", "fluid", (1, 1, 1)), ("cuda-aa-soa/channel", "channel", (0, 0, 0))):
@@ -746,16 +743,13 @@ def run_ours(args, dist):
             extra[key] = aa_line(lbmb200, fl, args, kargs, dist, peak)
             extra[key]["workload"] = "%d^3 %s" % (args.edge, "fully periodic fluid box" if geo == "fluid"
                                                   else "channel, periodic x, walls in y and z")
-        # the two-grid full-array rows on the fluid box (304 B per node update)
+        # the two-grid full-array rows on the fluid box
         fl = lbmb200.geometry("fluid", (args.edge,) * 3, (1, 1, 1))
         for kname in ("cuda-push-soa", "cuda-pull-soa"):
-            tq = time_kernel(lbmb200, kname, fl, min(args.steps, 100), 3, kargs, dist, "aa")
+            tq = time_kernel(lbmb200, kname, fl, min(args.steps, 100), 4, kargs, dist, "aa")
             tq["inst"].deinit()
-            qm = statistics.mean(tq["per_launch_ms"])
             extra[kname] = {"workload": "%d^3 fully periodic fluid box" % args.edge,
-                            "mflups": round(fl.n_fluid / (qm / 1e3) / 1e6, 1), "launch_ms": round(qm, 5),
-                            "achieved_gbs": round(B_PER_FLUP["aa"] * fl.n_fluid / (qm / 1e3) / 1e9, 1),
-                            "frac": round(B_PER_FLUP["aa"] * fl.n_fluid / (qm / 1e3) / 1e9 / peak, 4)}
+                            **two_grid_line(tq, fl.n_fluid, 0.0, peak)}
         # reduced storage list AA on the porous domain (FP32 arithmetic)
         for prec, pb in (("fp32", 4), ("fp16", 2)):
             tl = time_kernel(lbmb200, "cuda-list-aa-pv-soa", lat, min(args.steps, 200), 4,

@@ -282,9 +282,10 @@ int lbm_b200_time_steps(KernelData *kd, CaseData *cd, int n, double *total_ms, d
 
 /* Number of kernel launches that n time steps take on this instance (the
  * size of lbm_b200_time_steps' per_launch_ms): AA kernels run whole even/odd
- * pairs, 1 launch per pair (both steps fused) or, for lists in FP16 with many
- * nodes or whose fused order would not stay in L2, 2 (even, odd); two-grid
- * kernels 1 per step. */
+ * pairs, 1 launch per pair (both steps fused; small domains many pairs) or, for
+ * lists in FP16 with many nodes or whose fused order would not stay in L2, 2
+ * (even, odd). Two-grid kernels take 1 per two steps (full array; lists with
+ * many nodes) and 1 for a last odd step, or 1 per step. */
 long lbm_b200_launches_for(KernelData *kd, int n);
 
 /* Adjacency bytes one adjacency-driven launch of a list instance reads (the

@@ -338,7 +338,13 @@ double pair_schedule(const uint32_t* reach, const uint32_t* runOff, int nTiles, 
       it.n[c] = (hi >> kPairGroupShift) - it.lo[c] + 1;
     }
   }
-  return pair_order(work, need, home, static_cast<size_t>(nTiles), static_cast<size_t>(margin), maxLag, items);
+  const double late =
+      pair_order(work, need, home, static_cast<size_t>(nTiles), static_cast<size_t>(margin), maxLag, items);
+  for (int t = 0; t < nTiles; ++t) {
+    items[t].firstRun = runOff[t];
+    items[t].firstRun16 = runOff[t + 1] - runOff[t];
+  }
+  return late;
 }
 
 }  // namespace lbm

@@ -110,6 +110,7 @@ struct Gpu {
   uint32_t pairItems, pairTiles, pairGroups;
   // small domains: many pairs in one launch (null: not small)
   uint32_t* dMeet;
+  uint32_t recordBytes;  // two-grid lists: the largest run record
   lbm::AaPairGeom pairGeom;
   int openFaces;
 
@@ -315,7 +316,8 @@ lbm::AaArgs aa_args(Gpu* g) {
   const int S = (int)g->dstride;
   for (int d = 0; d < Q; ++d) {
     const int j = lbm::inv(d);
-    a.ldOff[d] = d == lbm::DC ? lbm::DC * S : j * S + lbm::cx(j) * g->xs + lbm::cy(j) * g->pitch + lbm::cz(j);
+    a.ldOff[d] = d == lbm::DC ? lbm::DC * S
+                              : (g->kind == kFaPull ? d : j) * S + lbm::cx(j) * g->xs + lbm::cy(j) * g->pitch + lbm::cz(j);
     a.stOff[d] = d == lbm::DC ? lbm::DC * S : d * S + lbm::cx(d) * g->xs + lbm::cy(d) * g->pitch + lbm::cz(d);
   }
   return a;
@@ -466,7 +468,16 @@ long enqueue_steps(Gpu* g, const lbm::Trt<double>& t, int n, cudaEvent_t* ev = n
       g->iteration = it + 1;
     }
   } else if (g->kind == kFaPush || g->kind == kFaPull) {
-    for (int it = 0; it < n; ++it) {
+    int it = 0;
+    if (g->dPairItems)
+      for (; it + 1 < n; it += 2) {  // two steps in one launch: the state stays in its grid
+        mark();
+        const lbm::AaPairArgs q{pair_args<9>(g), g->pairGeom, g->openFaces};
+        lbm::fa_two_fp64(aa_args(g), q, t, g->kind == kFaPush, g->stream);
+        ++k;
+        g->iteration = it + 1;
+      }
+    for (; it < n; ++it) {
       const lbm::AaArgs a = aa_args(g);
       mark();
       if (g->kind == kFaPush)
@@ -478,7 +489,15 @@ long enqueue_steps(Gpu* g, const lbm::Trt<double>& t, int n, cudaEvent_t* ev = n
       g->iteration = it;
     }
   } else {
-    for (int it = 0; it < n; ++it) {
+    int it = 0;
+    if (g->dPairItems)
+      for (; it + 1 < n; it += 2) {  // two steps in one launch: the state stays in its grid
+        mark();
+        lbm::list_two_fp64(list_args(g), pair_args<3>(g), t, g->kind == kListPush, g->recordBytes, g->stream);
+        ++k;
+        g->iteration = it + 1;
+      }
+    for (; it < n; ++it) {
       lbm::ListArgs a = list_args(g);
       mark();
       if (g->kind == kListPush)
@@ -495,7 +514,7 @@ long enqueue_steps(Gpu* g, const lbm::Trt<double>& t, int n, cudaEvent_t* ev = n
 }
 
 long launches_for(Gpu* g, int n) {
-  if (two_grid(g->kind)) return n;
+  if (two_grid(g->kind)) return g->dPairItems ? n / 2 + n % 2 : n;
   if (g->dMeet) return ((n + 1) / 2 + kResidentPairs - 1) / kResidentPairs;
   long perPair = g->dPairItems ? 1 : 2;
   if (g->kind == kAa && !g->dPairItems) {
@@ -683,9 +702,9 @@ void cb_kernel(LatticeDesc* ld, KernelData* kd, CaseData* cd) {
   if (cd->VtkOutput) vtk_or_exit(ld, kd, cd, cd->MaxIterations);
 }
 
-// Fused step pairs (lbm_pair.cuh): the order of the work. Whole full-array
-// lattices always take them; lists do unless that is the slower way (below),
-// slabs do not (their halo messages travel between the steps).
+// Fused steps (lbm_pair.cuh): the order of the work. Whole full-array lattices
+// always take two steps per launch; lists do unless that is the slower way
+// (below), slabs do not (their halo messages travel between the steps).
 //
 // Margin (items between an odd step and the last even tile it needs): shorter,
 // and blocks wait; longer, and the PDFs leave L2 before the odd step. Lists,
@@ -705,6 +724,12 @@ void cb_kernel(LatticeDesc* ld, KernelData* kd, CaseData* cd) {
 // 256^3: 0.145 against 0.125).
 constexpr int kPairF16Tiles = 2048;
 constexpr double kPairLateShare = 0.1;
+// Two-grid lists: two steps in one launch from this many tiles on (us per step,
+// one launch each / one for two: pull 410 tiles 4.9 / 5.4, 800 tiles 8.9 / 9.4,
+// 1382 tiles 19.7 / 17.8); both grids wait in L2, so the margin is 3/4 of the
+// resident blocks (pull, 256^3 packing: 0.310 ms at 333, 0.315 at 444, 0.342 at
+// 600).
+constexpr int kTwoGridTiles = 1024;
 
 // Small domains: all tiles resident, many pairs per launch.
 bool schedule_resident(Gpu* g, size_t nTiles, int most) {
@@ -719,7 +744,7 @@ double pair_max_lag(Gpu* g) {
   int dev = 0, l2 = 0;
   LBM_CK(cudaGetDevice(&dev));
   LBM_CK(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev));
-  return 0.4 * l2 / (double)(lbm::kListTile * Q * g->elemBytes);
+  return 0.4 * l2 / (double)(lbm::kListTile * Q * g->elemBytes * (two_grid(g->kind) ? 2 : 1));
 }
 
 template <int R>
@@ -736,7 +761,9 @@ void pair_upload(Gpu* g, const std::vector<lbm::PairRec<R>>& items, size_t nTile
 void schedule_list_pairs(Gpu* g) {
   const int nTiles = (g->nFluid + lbm::kListTile - 1) / lbm::kListTile;
   if (nTiles == 0 || (g->storage == lbm::kStoreF16 && nTiles > kPairF16Tiles)) return;
-  if (schedule_resident(g, (size_t)nTiles, lbm::list_resident_tiles(g->storage))) return;
+  const bool two = two_grid(g->kind);
+  if (two && nTiles < kTwoGridTiles) return;
+  if (!two && schedule_resident(g, (size_t)nTiles, lbm::list_resident_tiles(g->storage))) return;
   uint32_t* dReach = nullptr;
   std::vector<uint32_t> reach(6 * (size_t)nTiles), off((size_t)nTiles + 1);
   LBM_CK(lbm::dev_alloc(&dReach, sizeof(uint32_t) * reach.size()));
@@ -746,8 +773,14 @@ void schedule_list_pairs(Gpu* g) {
   LBM_CK(cudaMemcpyAsync(off.data(), g->dRunOff, sizeof(uint32_t) * off.size(), cudaMemcpyDeviceToHost, g->stream));
   LBM_CK(cudaStreamSynchronize(g->stream));
   lbm::dev_free(dReach);
-  const int resident = lbm::list_pair_resident(g->storage);
-  const int margin = g->storage == lbm::kStoreF64 ? resident : resident * 3 / 2;
+  int margin;
+  if (two) {
+    for (int t = 0; t < nTiles; ++t) g->recordBytes = std::max(g->recordBytes, (off[t + 1] - off[t]) * 16u);
+    margin = lbm::list_two_resident(g->kind == kListPush, g->recordBytes) * 3 / 4;
+  } else {
+    const int resident = lbm::list_pair_resident(g->storage);
+    margin = g->storage == lbm::kStoreF64 ? resident : resident * 3 / 2;
+  }
   std::vector<lbm::PairItem> items;
   if (lbm::pair_schedule(reach.data(), off.data(), nTiles, margin, pair_max_lag(g), items) > kPairLateShare) return;
   pair_upload(g, items, (size_t)nTiles);
@@ -770,7 +803,7 @@ void schedule_aa_pairs(Gpu* g, const LatticeDesc* ld) {
         }
   }
   const size_t nTiles = (size_t)g->pairGeom.tpp * g->pairGeom.nX;
-  if (schedule_resident(g, nTiles, lbm::aa_resident_tiles())) return;
+  if (g->kind == kAa && schedule_resident(g, nTiles, lbm::aa_resident_tiles())) return;
   std::vector<lbm::AaPairItem> items;
   lbm::aa_pair_schedule(a, g->pairGeom, lbm::aa_pair_resident(), items);
   pair_upload(g, items, nTiles);
@@ -898,7 +931,7 @@ Gpu* gpu_new(Kind kind, LatticeDesc* ld, Parameters* params, const SlabSpec* sla
       LBM_CK(lbm::dev_alloc(&g->dG, sizeof(double) * g->mirrorElems));
       LBM_CK(cudaMemsetAsync(g->dG, 0, sizeof(double) * g->mirrorElems, g->stream));
     }
-    if (kind == kAa && !slab) schedule_aa_pairs(g, ld);
+    if (!slab) schedule_aa_pairs(g, ld);
     if (kind == kAa && slab) build_odd_items(g, link);
     std::free(link);
   } else {
@@ -970,7 +1003,7 @@ Gpu* gpu_new(Kind kind, LatticeDesc* ld, Parameters* params, const SlabSpec* sla
         std::exit(1);
       }
     }
-    if (kind == kListAa && !g->listSlab) schedule_list_pairs(g);
+    if (!g->listSlab) schedule_list_pairs(g);
     g->mirrorElems = (size_t)Q * nCells;
     LBM_CK(lbm::dev_alloc(&g->dF, g->elemBytes * g->mirrorElems));
     LBM_CK(cudaMemsetAsync(g->dF, 0, g->elemBytes * g->mirrorElems, g->stream));

@@ -41,7 +41,8 @@ struct AaArgs {
   int perX, perY, perZ;
   // element offsets from a cell's slot of plane 0, per direction d, read from
   // the parameter bank: the odd step's load of d (slot inv(d) of x + c_inv(d))
-  // and store of d (slot d of x + c_d); the centre uses its own slot
+  // and store of d (slot d of x + c_d); the centre uses its own slot. Two-grid
+  // pull: the load of d is slot d of x - c_d
   int ldOff[Q], stOff[Q];
   // x-slab of a larger lattice: a halo face (haloLo at x = 0, haloHi at
   // x = nX-1) borders the neighbouring slab, whose face plane the ghost plane
@@ -175,6 +176,7 @@ struct PairRec {
   uint32_t run;    // what the block stages into shared memory for it (run record / cell list):
   uint32_t run16;  // offset and size in 16-byte units (size 0: nothing)
   uint32_t aheadRun, aheadRun16;  // the same of the item kPairAhead later
+  uint32_t firstRun, firstRun16;  // two-grid lists: the run record of the item's first tile
   uint32_t lo[R], n[R];
 };
 using PairItem = PairRec<3>;  // lists: tiles reached by links with c_x = -1, 0, +1
@@ -267,6 +269,11 @@ int list_resident_tiles(int storage);
 int aa_resident_tiles();
 void list_pair_fp64(const ListArgs& a, const PairArgs<3>& p, const Trt<double>& t, cudaStream_t s);
 void list_pair_lp(const ListArgsLp& a, const PairArgs<3>& p, const TrtW& t, int storage, cudaStream_t s);
+// Two steps of a two-grid row in one launch: grid f into g and back.
+// recordBytes: the instance's largest run record.
+int list_two_resident(bool push, uint32_t recordBytes);
+void list_two_fp64(const ListArgs& a, const PairArgs<3>& p, const Trt<double>& t, bool push, uint32_t recordBytes,
+                   cudaStream_t s);
 void list_resident_fp64(const ListArgs& a, const ResidentArgs& r, const Trt<double>& t, cudaStream_t s);
 void list_resident_lp(const ListArgsLp& a, const ResidentArgs& r, const TrtW& t, int storage, cudaStream_t s);
 
@@ -320,6 +327,7 @@ struct AaPairArgs {
 AaPairGeom aa_pair_geom(const AaArgs& a);
 void aa_pair_schedule(const AaArgs& a, const AaPairGeom& g, int margin, std::vector<AaPairItem>& items);
 int aa_pair_resident();
+void fa_two_fp64(const AaArgs& a, const AaPairArgs& p, const Trt<double>& t, bool push, cudaStream_t s);
 void aa_resident_fp64(const AaArgs& a, const AaPairGeom& g, int openFaces, const ResidentArgs& r,
                       const Trt<double>& t, cudaStream_t s);
 void aa_pair_fp64(const AaArgs& a, const AaPairArgs& p, const Trt<double>& t, cudaStream_t s);

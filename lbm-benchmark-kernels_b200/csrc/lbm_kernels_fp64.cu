@@ -375,11 +375,6 @@ __device__ __forceinline__ void aa_odd_select(const AaArgs& a, const Trt<double>
   trt_update(t, load, store);
 }
 
-__device__ __noinline__ void aa_odd_wall_cell(const AaArgs& a, const Trt<double>& t, int c, int x, int y, int z,
-                                              uint32_t w) {
-  aa_odd_select(a, t, c, w, XyzWrap(a, x, y, z));
-}
-
 // The same on a lattice with open faces: a reversed link may also leave into
 // the ghost layer, as in the face kernel.
 __device__ __noinline__ void aa_odd_open_cell(const AaArgs& a, const Trt<double>& t, int c, int x, int y, int z,
@@ -463,7 +458,7 @@ __device__ __forceinline__ void aa_pair_odd_cell(const AaArgs& a, const Trt<doub
   } else if (!kind.face) {
     aa_odd_select(a, t, c, w, NoWrap());
   } else if (!openFaces) {
-    aa_odd_wall_cell(a, t, c, x, y, z, w);
+    aa_odd_select(a, t, c, w, XyzWrap(a, x, y, z));
   } else {
     aa_odd_open_cell(a, t, c, x, y, z, w);
   }
@@ -474,17 +469,18 @@ __device__ __forceinline__ void aa_pair_odd_cell(const AaArgs& a, const Trt<doub
 // rows left half to three quarters of the threads of row-shaped blocks idle).
 // A warp without reversed links takes the odd step by fixed offsets and the
 // periodic wraps of its cells' positions (XyzWrap); a warp with any takes a
-// selecting path for all its cells, inline where none lies on a face of the
-// lattice (channel 203 x 190 x 197 in strips of 74 tiles: 0.307 ms per step;
-// with lists of the wall cells as a second pass 0.333, with the selecting path
-// out of line 0.360; in whole planes 0.294, two launches 0.412).
+// selecting path for all its cells, without the wraps where none lies on a face
+// of the lattice. Open faces have a path of their own, out of line. Channel 203
+// x 190 x 197: 0.277 ms per step; one selecting path with the wraps 0.287; that
+// path out of line 0.35; lists of the wall cells as a second pass 0.32 (two
+// launches 0.412).
 // Even loads do not wait for the link word that says whether the cell is
 // fluid (solid cells' slots exist; nothing is stored there): 0.310 against
 // 0.319 ms on that channel, 0.189 / 0.194 at 85 % fluid cells, 0.176 / 0.174
 // at 40 %.
 // Bound by L2 requests and their latency as the list pair: 256^3 fluid box
-// 0.818 -> 0.597 ms per step (28.1 GFLUP/s, half the HBM bytes), 256^3 channel
-// 0.845 -> 0.645, 64^3 channel 0.0219 -> 0.0140.
+// 0.818 -> 0.597 ms per step (28.1 GFLUP/s, half the HBM bytes), 64^3 channel
+// 0.0220 -> 0.0106, 128 x 112 x 120 blocks, periodic, 0.101 -> 0.064.
 __global__ void __launch_bounds__(kPairThreads, 3)
     k_aa_pair_fp64(const __grid_constant__ AaArgs a, const __grid_constant__ AaPairArgs q,
                    const __grid_constant__ Trt<double> t) {
@@ -535,6 +531,118 @@ __global__ void __launch_bounds__(kListTile, 3)
     aa_pair_odd_cell(a, t, c, x, y, z, w, kind, openFaces);
     if (!resident_meet(r, 2 * p + 2, a.err, &ok)) return;
   }
+}
+
+// Two steps of a two-grid full-array row in one launch: the tiles, order and
+// waits of the AA pair, the first step from grid f into g and the second back
+// (k_list_two_fp64 says why, with the same 3/4 of the HBM traffic; tiles of
+// consecutive cells fill the warps of short rows). ms per step, one launch each
+// / one for two: pull 256^3 fluid box 0.891 / 0.749, 128 x 112 x 120 box 0.110 /
+// 0.082, periodic blocks 0.132 / 0.088, 64^3 0.0205 / 0.0114; push 0.857 / 0.748,
+// 0.100 / 0.079, 0.113 / 0.080, 0.0174 / 0.0112 (push with streaming loads 10 %
+// slower). Warps with wall cells take one selecting path, wraps included.
+
+// A warp with wall cells and open faces, as k_fa_push_fp64 and k_fa_pull_fp64.
+template <bool kPush>
+__device__ __noinline__ void fa_general_cell(const AaArgs& a, const Trt<double>& t, const double* f, double* g0, int c,
+                                             int x, int y, int z, uint32_t w) {
+  const long long S = a.dstride;
+  double* const g = launder(g0);
+  trt_update(t, [&](int d) -> double { return kPush ? f[d * S + c] : f[a.ldOff[d] + c]; },
+             [&](int e, double v) {
+               if (!kPush || e == DC) g[e * S + c] = v + t.force[e];
+               if (e == DC) return;
+               const int j = inv(e);
+               const int n = c + aa_off(a, e);
+               if (!((w >> e) & 1u)) {
+                 const int q = aa_wrapped(a, x, y, z, e);
+                 if (kPush)
+                   g[e * S + q] = v + t.force[e];
+                 else if (q != n)
+                   g[e * S + q - aa_off(a, e)] = v + t.force[e];  // periodic image's ghost slot
+               } else {
+                 double* const s = g + j * S + (kPush ? c : n);
+                 *s = (aa_open(a, x, y, z, e) ? *s : v) + t.force[j];
+               }
+             });
+}
+
+template <bool kPush, bool kLast>
+__device__ __forceinline__ void fa_pair_cell(const AaArgs& a, const Trt<double>& t, const double* f, double* g, int c,
+                                             int x, int y, int z, uint32_t w, int openFaces) {
+  const AaWarpKind kind = aa_warp_kind(a, x, y, z, w);
+  if (!(w & kFluidBit)) return;
+  if (kind.wall && kind.face && openFaces) {
+    fa_general_cell<kPush>(a, t, f, g, c, x, y, z, w);
+    return;
+  }
+  const int S = (int)a.dstride;
+  const double* const fb = f + c;
+  const uint64_t keep = l2_keep_policy();
+  auto put = [&](int o, double v) {
+    double* const q = launder(g + c) + o;
+    if (kLast)
+      __stcs(q, v);
+    else
+      st_keep(q, v, keep);
+  };
+  auto load = [&](int d) -> double { return kPush ? fb[d * S] : fb[a.ldOff[d]]; };
+  if (!kind.wall) {
+    const XyzWrap wrap(a, x, y, z);
+    trt_update(t, load, [&](int e, double v) {
+      if (kPush) {
+        put(a.stOff[e] + wrap(e), v + t.force[e]);
+      } else {
+        put(e * S, v + t.force[e]);
+        const int o = wrap(e);
+        if (o != 0) put(e * S + o, v + t.force[e]);  // periodic image's ghost slot
+      }
+    });
+  } else {
+    const XyzWrap wrap(a, x, y, z);
+    trt_update(t, load, [&](int e, double v) {
+      const int j = inv(e);
+      const bool rev = e != DC && ((w >> e) & 1u);
+      if (kPush) {
+        put(rev ? j * S : a.stOff[e] + wrap(e), v + (rev ? t.force[j] : t.force[e]));
+      } else {
+        put(e * S, v + t.force[e]);
+        if (rev) put(j * S + aa_off(a, e), v + t.force[j]);  // wall slot
+        const int o = wrap(e);
+        if (!rev && o != 0) put(e * S + o, v + t.force[e]);  // periodic image's ghost slot
+      }
+    });
+  }
+}
+
+template <bool kPush>
+__global__ void __launch_bounds__(kPairThreads, 3)
+    k_fa_two_fp64(const __grid_constant__ AaArgs a, const __grid_constant__ AaPairArgs q,
+                  const __grid_constant__ Trt<double> t) {
+  __shared__ PairShared<9, 4> sh;  // nothing staged
+  pair_init(&sh);
+  const uint32_t k = blockIdx.x;
+  if (threadIdx.x >= kListTile) {
+    pair_service(&sh, q.p, nullptr, a.err, k);
+    return;
+  }
+  chain_wait();
+  if (k < q.p.nTiles) {
+    uint32_t x, i;
+    aa_pair_tile(q.g, k, x, i);
+    i += threadIdx.x;
+    const uint32_t y = fast_div(i, q.g.byZ), z = i - y * q.g.byZ.d;
+    const int c = aa_cell(a, x, y, z);
+    fa_pair_cell<kPush, false>(a, t, a.f, a.g, c, x, y, z, i < q.g.plane ? __ldg(a.link + c) : 0u,
+                               q.openFaces);
+    pair_even_done(&sh);
+  }
+  if (!pair_odd_named(&sh, a.err)) return;
+  const uint32_t x = sh.item.extra, i = sh.item.tile + threadIdx.x;
+  const uint32_t y = fast_div(i, q.g.byZ), z = i - y * q.g.byZ.d;
+  const int c = aa_cell(a, x, y, z);
+  const uint32_t w = i < q.g.plane ? __ldg(a.link + c) : 0u;
+  if (pair_odd_turn(&sh, a.err)) fa_pair_cell<kPush, true>(a, t, a.g, a.f, c, x, y, z, w, q.openFaces);
 }
 
 static FastDiv fast_div_of(uint32_t d) {
@@ -640,6 +748,13 @@ void aa_pair_schedule(const AaArgs& a, const AaPairGeom& g, int margin, std::vec
     }
   }
   pair_order(work, need, home, nTiles, static_cast<size_t>(margin), 0.0, items);
+}
+
+void fa_two_fp64(const AaArgs& a, const AaPairArgs& q, const Trt<double>& t, bool push, cudaStream_t s) {
+  if (push)
+    launch_chained(k_fa_two_fp64<true>, q.p.nItems, kPairThreads, 0, s, a, q, t);
+  else
+    launch_chained(k_fa_two_fp64<false>, q.p.nItems, kPairThreads, 0, s, a, q, t);
 }
 
 int aa_resident_tiles() {
@@ -1131,6 +1246,94 @@ __global__ void __launch_bounds__(kListTile, 3) k_list_push_fp64(const ListArgs 
   trt_update(t, [&](int d) { return x[d]; }, store);
 }
 
+// Two steps of a two-grid list row in one launch (lbm_pair.cuh): block k steps
+// its first tile from grid f into grid g, then a tile two planes back from g
+// into f once the first steps of all tiles that its links reach are done (they
+// wrote the slots of g it reads and have read the slots of f it writes). The
+// second step finds g in L2: per two steps HBM sees f read and written and g
+// written, 3/4 of two launches' traffic. ms per step, one launch each / one for
+// two: pull 256^3 packing 0.342 / 0.309, 160^3 0.0864 / 0.0768, 96^3 0.0197 /
+// 0.0178; push 0.401 / 0.396, 0.0988 / 0.0935, 0.0230 / 0.0210. Loads ask for
+// no early eviction: the second step overwrites the lines of f that the first
+// one read, and a push into lines that have left L2 reads them back for the
+// sectors it fills in part (push with streaming loads: 0.433 ms). Both tiles'
+// run records are staged, in dynamic shared memory sized to the instance's
+// largest record (the rest of the 256 KB holds the loads in flight).
+template <bool kPush, bool kLast>
+__device__ __forceinline__ void two_grid_node(const ListArgs& a, const Trt<double>& t, const double* src, double* dst,
+                                              int n, const uint32_t* e, uint32_t off) {
+  const long long S = a.nCells;
+  const uint64_t keep = l2_keep_policy();
+  auto put = [&](double* q, double v) {
+    if (kLast)
+      __stcs(q, v);
+    else
+      st_keep(q, v, keep);
+  };
+  auto load = [&](int d) -> double { return kPush || d == DC ? src[d * S + n] : src[e[d] + off]; };
+  trt_update(t, load, [&](int d, double v) {
+    if (!kPush || d == DC) {
+      put(launder(dst) + d * S + n, v + t.force[d]);
+      return;
+    }
+    const uint32_t to = reinterpret_cast<const volatile uint32_t*>(e)[d] + off;
+    const int j = inv(d);
+    const bool bounce = to == static_cast<uint32_t>(j * S + n);
+    put(dst + to, v + (bounce ? t.force[j] : t.force[d]));
+  });
+}
+
+template <bool kPush>
+__global__ void __launch_bounds__(kPairThreads, 3)
+    k_list_two_fp64(const __grid_constant__ ListArgs a, const __grid_constant__ PairArgs<3> p,
+                    const __grid_constant__ Trt<double> t, uint32_t recordWords) {
+  extern __shared__ __align__(128) uint32_t records[];
+  __shared__ PairShared<3, 4> sh;
+  pair_init(&sh);
+  const uint32_t k = blockIdx.x;
+  if (threadIdx.x >= kListTile) {
+    pair_service(&sh, p, a.runs, a.err, k, records + recordWords, records);
+    return;
+  }
+  if (k < p.nTiles) {
+    const int n = static_cast<int>(k) * kListTile + threadIdx.x;
+    pair_odd_named(&sh, a.err);  // the first tile's run record
+    chain_wait();
+    if (n < a.nFluid) {
+      uint32_t off;
+      const uint32_t* e = run_row(records, threadIdx.x, off);
+      two_grid_node<kPush, false>(a, t, a.f, a.g, n, e, off);
+    }
+    pair_even_done(&sh);
+  } else {
+    chain_wait();
+  }
+  if (!pair_odd_turn(&sh, a.err)) return;
+  const int n = static_cast<int>(sh.item.tile) * kListTile + threadIdx.x;
+  if (n >= a.nFluid) return;
+  uint32_t off;
+  const uint32_t* e = run_row(records + recordWords, threadIdx.x, off);
+  two_grid_node<kPush, true>(a, t, a.g, a.f, n, e, off);
+}
+
+// Shared memory of the two records, each 128-byte aligned.
+static uint32_t two_record_words(uint32_t recordBytes) { return (recordBytes + 127u) / 128u * 32u; }
+template <bool kPush>
+static size_t two_smem(uint32_t recordBytes) {
+  // the opt-in is a per-device attribute, set once to the most any record needs
+  // (concurrent first calls set the same value)
+  constexpr int kMaxDevices = 64;
+  static std::atomic<bool> set[kMaxDevices];
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev >= kMaxDevices || !set[dev].load(std::memory_order_acquire)) {
+    cudaFuncSetAttribute(k_list_two_fp64<kPush>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)(2 * sizeof(uint32_t) * two_record_words(kRunTileWords * 4)));
+    if (dev < kMaxDevices) set[dev].store(true, std::memory_order_release);
+  }
+  return 2 * sizeof(uint32_t) * two_record_words(recordBytes);
+}
+
 template <typename E>
 __global__ void k_slot_gather(const E* __restrict__ f, const uint32_t* __restrict__ idx, long long n,
                               E* __restrict__ buf) {
@@ -1220,6 +1423,25 @@ int list_resident_tiles_fp64() {
 int list_pair_resident_fp64() {
   static std::atomic<int> n{0};
   return prefetch_distance(n, k_list_pair_fp64, kPairThreads, true);
+}
+int list_two_resident(bool push, uint32_t recordBytes) {
+  int dev = 0, sms = 0, per = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (push)
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_list_two_fp64<true>, kPairThreads, two_smem<true>(recordBytes));
+  else
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_list_two_fp64<false>, kPairThreads,
+                                                  two_smem<false>(recordBytes));
+  return sms * per;
+}
+void list_two_fp64(const ListArgs& a, const PairArgs<3>& p, const Trt<double>& t, bool push, uint32_t recordBytes,
+                   cudaStream_t s) {
+  const uint32_t words = two_record_words(recordBytes);
+  if (push)
+    launch_chained(k_list_two_fp64<true>, p.nItems, kPairThreads, two_smem<true>(recordBytes), s, a, p, t, words);
+  else
+    launch_chained(k_list_two_fp64<false>, p.nItems, kPairThreads, two_smem<false>(recordBytes), s, a, p, t, words);
 }
 void list_pull_fp64(const ListArgs& a, const Trt<double>& t, cudaStream_t s) {
   // no adjacency prefetch: with the full adjacency it slowed this kernel by

@@ -80,7 +80,7 @@ template <int R, int kWords>
 struct PairShared {
   alignas(128) uint32_t run[kWords];
   alignas(16) PairRec<R> item;
-  alignas(8) uint64_t named;  // the item is here
+  alignas(8) uint64_t named;  // the item is here (and the first tile's run record)
   alignas(8) uint64_t go;     // the odd step may start: dependencies met, staged data here
   alignas(8) uint64_t even;   // every compute warp has stored its even nodes
 };
@@ -125,9 +125,12 @@ __device__ __forceinline__ bool pair_ready(const PairRec<R>& it, const PairArgs<
 
 // The service warp of block k (see above); runs: the array that the items'
 // staged data lies in.
+// first: where the run record of the item's first tile goes (two-grid lists),
+// or null.
 template <int R, int kWords>
 __device__ __forceinline__ void pair_service(PairShared<R, kWords>* sh, const PairArgs<R>& p, const void* runs,
-                                             int* err, uint32_t k) {
+                                             int* err, uint32_t k, uint32_t* second = nullptr,
+                                             uint32_t* first = nullptr) {
   constexpr int kItemWords = static_cast<int>(sizeof(PairRec<R>) / 4);
   static_assert(kItemWords <= 32, "one item word per lane");
   const int lane = threadIdx.x - kListTile;
@@ -138,10 +141,14 @@ __device__ __forceinline__ void pair_service(PairShared<R, kWords>* sh, const Pa
   const PairRec<R>& it = sh->item;
   const char* const base = static_cast<const char*>(runs);
   if (lane == 0) {
+    if (first && it.firstRun16) {
+      mbar_expect_tx(&sh->named, it.firstRun16 * 16u);
+      bulk_g2s(first, base + static_cast<size_t>(it.firstRun) * 16, it.firstRun16 * 16u, &sh->named);
+    }
     mbar_arrive(&sh->named);
     if (it.tile != kPairNone && it.run16) {
       mbar_expect_tx(&sh->go, it.run16 * 16u);
-      bulk_g2s(sh->run, base + static_cast<size_t>(it.run) * 16, it.run16 * 16u, &sh->go);
+      bulk_g2s(second ? second : sh->run, base + static_cast<size_t>(it.run) * 16, it.run16 * 16u, &sh->go);
     }
     if (p.prefetch) {
       // the staged data and the item of blocks that have not started yet, into L2

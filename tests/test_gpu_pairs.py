@@ -171,3 +171,38 @@ def test_captured_steps_replay():
                 inst.deinit()
         m = lat.mask != 0
         assert np.array_equal(fields[0][m], fields[1][m])
+
+
+TWO_GRID_CASES = [
+    ("cuda-list-pull-soa", lambda: _spheres((140, 62, 60), 0.6)),
+    ("cuda-list-pull-split-nt-2s-soa", lambda: lbmb200.geometry("fluid", (131, 47, 46), (1, 0, 1))),
+    ("cuda-list-push-soa", lambda: _spheres((140, 62, 60), 0.6)),
+] + [(k, g) for k in ("cuda-push-soa", "cuda-pull-soa") for g in (
+    lambda: lbmb200.geometry("fluid", (60, 61, 59), (1, 1, 1)),
+    lambda: lbmb200.geometry("channel", (45, 70, 64), (1, 0, 0)),
+    lambda: lbmb200.geometry("channel", (70, 50, 49), (0, 0, 0)),
+    lambda: lbmb200.geometry("fluid", (30, 66, 67), (0, 1, 0)),
+    lambda: lbmb200.geometry("fluid", (7, 5, 300), (1, 0, 0)),
+    lambda: _spheres((60, 47, 53), 0.5),
+    lambda: lbmb200.geometry("channel", (10, 317, 331), (1, 0, 0)))]
+
+
+@pytest.mark.parametrize("kname,make", TWO_GRID_CASES)
+def test_two_grid_steps_in_one_launch(kname, make):
+    """Two steps per launch (and a single last one) against one launch per
+    step: one-step runs take the latter."""
+    lat = make()
+    init = random_pdfs(lat.mask.size, 73)
+    fields = []
+    for steps in ([7], [1] * 7):
+        inst = lbmb200.kernel(kname).init(lat, kernel_args=["-lambda", "3/16"])
+        try:
+            assert inst.launches_for(7) == 4 and inst.launches_for(1) == 1
+            inst.set_field(init)
+            for n in steps:
+                inst.run(lbmb200.case(omega=1.2, xforce=2e-4, iterations=n))
+            fields.append(inst.get_field())
+        finally:
+            inst.deinit()
+    m = lat.mask != 0
+    assert np.array_equal(fields[0][m], fields[1][m])
