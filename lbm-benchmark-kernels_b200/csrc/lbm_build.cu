@@ -322,6 +322,7 @@ void list_tile_reach(const uint32_t* adj, int nFluid, long long nCells, uint32_t
 
 double pair_schedule(const uint32_t* reach, const uint32_t* runOff, int nTiles, int margin, double maxLag,
                      std::vector<PairItem>& items) {
+  const int shift = pair_group_shift(static_cast<size_t>(nTiles));
   std::vector<PairItem> work(nTiles);
   std::vector<uint32_t> need(nTiles), home(nTiles);
   for (int t = 0; t < nTiles; ++t) {
@@ -334,8 +335,8 @@ double pair_schedule(const uint32_t* reach, const uint32_t* runOff, int nTiles, 
       const uint32_t lo = reach[6 * (size_t)t + 2 * c], hi = reach[6 * (size_t)t + 2 * c + 1];
       if (lo > hi) continue;
       need[t] = std::max(need[t], hi);
-      it.lo[c] = lo >> kPairGroupShift;
-      it.n[c] = (hi >> kPairGroupShift) - it.lo[c] + 1;
+      it.lo[c] = lo >> shift;
+      it.n[c] = (hi >> shift) - it.lo[c] + 1;
     }
   }
   const double late =

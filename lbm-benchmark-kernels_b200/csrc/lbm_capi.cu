@@ -373,6 +373,7 @@ lbm::PairArgs<R> pair_args(Gpu* g) {
   p.count = g->dPairCount;
   p.nItems = g->pairItems;
   p.nTiles = g->pairTiles;
+  p.shift = lbm::pair_group_shift(g->pairTiles);
   p.launches = g->dPairCount + g->pairGroups;
   p.prefetch = list_prefetch_enabled();
   return p;
@@ -708,16 +709,17 @@ void cb_kernel(LatticeDesc* ld, KernelData* kd, CaseData* cd) {
 //
 // Margin (items between an odd step and the last even tile it needs): shorter,
 // and blocks wait; longer, and the PDFs leave L2 before the odd step. Lists,
-// FP64, 256^3 packing, 444 resident blocks: 0.280 ms per step at 350, 0.275 at
-// 444, 0.276 at 520, 0.281 at 600. Reduced storage takes half the room or
-// less: FP32, 740 resident: 0.172 at 740, 0.165 at 1100, 0.171 at 1500.
+// FP64, 256^3 packing, 444 resident blocks: 0.259 ms per step at 355, 0.256 at
+// 444, 0.258 at 530, 0.262 at 620. Reduced storage takes half the room or
+// less: FP32, 740 resident: 0.151 at 890, 0.152 at 1110, 0.154 at 1330, 0.169
+// at 1890 (160^3: 0.0384, 0.0386, 0.0389, 0.0413).
 //
 // Where the pair pays: the PDFs written between a tile's even and odd step have
 // to stay in L2. Up to 2/5 of L2 (50 MB) it is faster (lists, FP64, 256^3
-// packing: 25 MB 0.275 ms per step, 50 MB 0.328, two launches 0.342); where
-// more than a tenth of the tiles come later than that (lists of large
-// cross-sections, numberings that put neighbours far apart) the two launches
-// stay. FP16 storage: the two launches' even step, staged for two nodes per
+// packing, groups of 8 tiles: 25 MB 0.275 ms per step, 50 MB 0.328, two
+// launches 0.342); where more than a tenth of the tiles come later than that
+// (lists of large cross-sections, numberings that put neighbours far apart)
+// the two launches stay. FP16 storage: the two launches' even step, staged for two nodes per
 // thread, is worth more than the traffic saved, so the pair is for domains of
 // at most 2048 tiles, where it is the launch that counts (96^3 packing, 1382
 // tiles: 0.0097 ms per step against 0.0104; 128^3, 3274 tiles: 0.0185 both;
@@ -751,7 +753,7 @@ template <int R>
 void pair_upload(Gpu* g, const std::vector<lbm::PairRec<R>>& items, size_t nTiles) {
   g->pairTiles = static_cast<uint32_t>(nTiles);
   g->pairItems = static_cast<uint32_t>(items.size());
-  g->pairGroups = static_cast<uint32_t>((nTiles + (1u << lbm::kPairGroupShift) - 1) >> lbm::kPairGroupShift);
+  g->pairGroups = static_cast<uint32_t>(((nTiles - 1) >> lbm::pair_group_shift(nTiles)) + 1);
   LBM_CK(lbm::dev_alloc(&g->dPairCount, sizeof(uint32_t) * (g->pairGroups + 2)));
   LBM_CK(cudaMemsetAsync(g->dPairCount, 0, sizeof(uint32_t) * (g->pairGroups + 2), g->stream));
   LBM_CK(lbm::dev_alloc(&g->dPairItems, sizeof(lbm::PairRec<R>) * items.size()));

@@ -165,8 +165,16 @@ int list_runs_device(const uint32_t* adj, int nFluid, cudaStream_t s, uint32_t**
 // step. Item k: the even step of the k-th tile in even order (k < nTiles), then
 // the odd step of the tile that the record names, once the even tiles that
 // its links reach are complete: up to R ranges [lo, lo + n) of groups of
-// 2^kPairGroupShift tiles consecutive in even order.
-constexpr int kPairGroupShift = 3;
+// 2^shift tiles consecutive in even order.
+//
+// Large groups make few counters to poll, small ones short waits for the rest
+// of a group. us per step at shift 3 / 4 / 5 / 6: lists FP64 1382 tiles 15.5 /
+// 15.3 / 15.1 / 15.3, 26210 tiles 268 / 261 / 257 / 256; FP32 770 tiles 5.8 / - /
+// 6.4 / 6.5, 1382 tiles 9.8 / 9.7 / 10.1 / 10.7, 6397 tiles 40.3 / 39.8 / 38.7 /
+// 39.6, 26210 tiles 164 / 157 / 154 / 152 (full arrays: no difference).
+inline int pair_group_shift(size_t nTiles) {
+  return nTiles < 1024 ? 3 : nTiles < 4096 ? 4 : nTiles < 16384 ? 5 : 6;
+}
 constexpr uint32_t kPairNone = 0xffffffffu;
 constexpr uint32_t kPairAhead = 512;  // about a wave of resident blocks
 template <int R>
@@ -187,6 +195,7 @@ struct PairArgs {
   uint32_t* launches;       // [0] launches completed, [1] blocks of this one that have read [0]
   uint32_t nItems;          // blocks of the launch
   uint32_t nTiles;
+  int shift;                // pair_group_shift(nTiles)
   int prefetch;             // as ListArgs::prefetch (0: none)
 };
 
@@ -202,13 +211,15 @@ double pair_schedule(const uint32_t* reach, const uint32_t* runOff, int nTiles, 
 // Host: the odd steps `work` (any order; need[i] = the last position in even
 // order that work[i] depends on, home[i] = its own tile's position) as item
 // records: each odd step follows the last even tile it needs by at least
-// `margin` items (or by all of them) and takes the first free item from there
-// on. Returns the share of the odd steps that come more than maxLag items
+// `margin` items (or by all of them; by two groups at least, so that every
+// tile of the groups it waits for is an earlier block's) and takes the first
+// free item from there on. Returns the share of the odd steps that come more than maxLag items
 // after their own tile's even step (whose PDFs may have left L2 by then).
 template <int R>
 double pair_order(const std::vector<PairRec<R>>& work, const std::vector<uint32_t>& need,
                   const std::vector<uint32_t>& home, size_t nTiles, size_t margin, double maxLag,
                   std::vector<PairRec<R>>& items) {
+  margin = std::max(margin, size_t{2} << pair_group_shift(nTiles));
   // counting sort by need, stable: nearly the tile order, except for tiles
   // that need far later ones (the first x plane of a periodic lattice)
   std::vector<uint32_t> first(nTiles + 1, 0), order(work.size());

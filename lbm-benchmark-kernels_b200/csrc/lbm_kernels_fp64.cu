@@ -683,6 +683,7 @@ AaPairGeom aa_pair_geom(const AaArgs& a) {
 
 void aa_pair_schedule(const AaArgs& a, const AaPairGeom& g, int margin, std::vector<AaPairItem>& items) {
   const uint32_t nTiles = g.nX * g.tpp, lastStrip = (g.tpp - 1) / g.J;
+  const int shift = pair_group_shift(nTiles);
   auto width = [&](uint32_t s) { return s == lastStrip ? g.tpp - s * g.J : g.J; };
   auto position = [&](uint32_t x, uint32_t j) {
     const uint32_t s = j / g.J;
@@ -724,7 +725,7 @@ void aa_pair_schedule(const AaArgs& a, const AaPairGeom& g, int margin, std::vec
       for (uint32_t dx = 0; dx < 3; ++dx) {
         const uint32_t px = (x + g.nX + dx - 1) % g.nX;
         for (const Range& v : reach) {
-          pos.push_back({position(px, v.lo) >> kPairGroupShift, position(px, v.hi) >> kPairGroupShift});
+          pos.push_back({position(px, v.lo) >> shift, position(px, v.hi) >> shift});
           need[t] = std::max(need[t], position(px, v.hi));
         }
       }
@@ -738,7 +739,7 @@ void aa_pair_schedule(const AaArgs& a, const AaPairGeom& g, int margin, std::vec
       }
       if (m > 9) {  // more pieces than a record holds: wait for every even tile
         m = 1;
-        pos[0] = {0, (nTiles - 1) >> kPairGroupShift};
+        pos[0] = {0, (nTiles - 1) >> shift};
         need[t] = nTiles - 1;
       }
       for (size_t r = 0; r < m; ++r) {

@@ -14,8 +14,8 @@
 // groups of even tiles its links reach are complete (counters in device
 // memory, release/acquire at GPU scope). The hardware starts the blocks of a
 // one-dimensional grid in index order, and item k only depends on the even
-// tiles of blocks at least `margin` below k, so the blocks that a waiting one
-// depends on have always started and, waiting for nothing before their even
+// tiles of blocks at least `margin` less one group below k, so the blocks that
+// a waiting one depends on have always started and, waiting for nothing before their even
 // tile is counted, always finish it. The wait is bounded all the same: it
 // gives up after kPairSpinLimit polls, or as soon as another block has, and
 // sets the error word.
@@ -43,8 +43,8 @@ constexpr uint32_t kResidentSpinLimit = 1u << 22;  // the same between resident 
 // Cache hints. A slot written by the even step is read back by the odd step
 // soon, one written by the odd step not before the next pair: even loads and
 // odd stores stream (evict first), so that finished tiles do not push waiting
-// ones out of L2, and FP64 even stores ask to be kept (256^3 packing, FP64:
-// 0.298 -> 0.275 ms per step; the reduced storage takes a third or less of the
+// ones out of L2, and FP64 even stores ask to be kept (256^3 packing, FP64,
+// groups of 8 tiles: 0.298 -> 0.275 ms per step; the reduced storage takes a third or less of the
 // room and does without the policy's registers).
 __device__ __forceinline__ uint64_t l2_keep_policy() {
   uint64_t p;
@@ -117,7 +117,7 @@ __device__ __forceinline__ bool pair_ready(const PairRec<R>& it, const PairArgs<
       }
       j -= it.n[r];
     }
-    const uint32_t size = min(p.nTiles - (g << kPairGroupShift), 1u << kPairGroupShift);
+    const uint32_t size = min(p.nTiles - (g << p.shift), 1u << p.shift);
     good = static_cast<int32_t>(ld_acquire(p.count + g) - launch * size) >= 0 && good;
   }
   return __all_sync(0xffffffffu, good);
@@ -164,7 +164,7 @@ __device__ __forceinline__ void pair_service(PairShared<R, kWords>* sh, const Pa
   if (ready && lane == 0) mbar_arrive(&sh->go);
   if (even) {
     if (!mbar_wait_bounded(&sh->even, 0)) atomicOr(err, 1);
-    if (lane == 0) red_release(p.count + (k >> kPairGroupShift), 1u);
+    if (lane == 0) red_release(p.count + (k >> p.shift), 1u);
   }
   // the last block to have read the launch number moves it on
   if (lane == 0 && atomicInc(p.launches + 1, p.nItems - 1u) == p.nItems - 1u) atomicAdd(p.launches, 1u);

@@ -113,6 +113,34 @@ def test_slab_steps_on_a_whole_lattice():
     assert np.array_equal(fields[0][m], fields[1][m])
 
 
+@pytest.mark.parametrize("kname,prec", [("cuda-list-aa-pv-soa", "fp64"), ("cuda-list-aa-pv-soa", "fp32"),
+                                        ("cuda-list-pull-soa", "fp64"), ("cuda-aa-soa", "fp64")])
+@pytest.mark.parametrize("dims", [(65, 64, 63), (128, 128, 64), (129, 127, 64), (256, 128, 128), (257, 128, 129)])
+def test_every_group_size(kname, prec, dims):
+    """Either side of the tile counts at which the groups grow, whole and
+    ragged last groups: the fused steps against separate ones."""
+    lat = lbmb200.geometry("fluid", dims, (1, 1, 1))
+    init = random_pdfs(lat.mask.size, 29)
+    cd = lbmb200.case(omega=1.2, xforce=2e-4, iterations=4)
+    kargs = ["-lambda", "3/16"] + (["-precision", prec] if "list" in kname else [])
+    inst = lbmb200.kernel(kname).init(lat, kernel_args=kargs)
+    try:
+        assert inst.launches_for(4) == 2
+        inst.set_field(init)
+        inst.run(cd)
+        whole = inst.get_field()
+        if "pull" in kname:
+            inst.set_field(init)
+            for _ in range(4):
+                inst.run(lbmb200.case(omega=1.2, xforce=2e-4, iterations=1))
+            apart = inst.get_field()
+    finally:
+        inst.deinit()
+    if "pull" not in kname:
+        apart = _run_slabs(lat, 2, init, cd, 2, layout="list" if "list" in kname else "full", kargs=kargs)
+    assert np.array_equal(apart, whole)
+
+
 @pytest.mark.parametrize("prec", ["fp64", "fp32", "fp16"])
 @pytest.mark.parametrize("dims,steps", [((9, 8, 7), 2), ((30, 27, 29), 9), ((47, 44, 45), 6)])
 def test_small_domains_in_one_launch(prec, dims, steps):
