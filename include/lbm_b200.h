@@ -509,14 +509,18 @@ int lbm_batch_sync(void *batch);
 int lbm_batch_moments(void *batch, double *out);
 int lbm_batch_get_field(void *batch, int slot, double *out);
 int lbm_batch_set_field(void *batch, int slot, const double *in);
-/* which: 0 even, 1 odd, 2 both; threads 64/128/256 (nodes per thread =
+/* Launch shape of the even and odd steps where each step is a launch of its
+ * own: in batches whose PDFs fit into half of L2, and in every batch from this
+ * call on (larger ones otherwise take both steps of a pair in one launch).
+ * which: 0 even, 1 odd, 2 both; threads 64/128/256 (nodes per thread =
  * 256 / threads); blocks = persistent grid size, 0 = one block per tile. */
 int lbm_batch_set_launch(void *batch, int which, int threads, int blocks);
 void lbm_batch_get_launch(void *batch, int *out6);
 int lbm_batch_time_steps(void *batch, int nsteps, double *ms);
 /* Autotuner over block size x nodes per thread x grid (2..6 persistent
  * blocks per SM, or 0 = one block per tile); rows of {which, threads,
- * nodesPerThread, blocks, ms}; keeps the fastest. */
+ * nodesPerThread, blocks, ms}; keeps the fastest for steps that are launches
+ * of their own. */
 int lbm_batch_tune(void *batch, int trialSteps, double *results, int maxRows);
 /* Checkpoint / restart of one resident domain: its PDFs in the batch's
  * storage format plus its lattice size and relaxation parameters. _load

@@ -45,6 +45,8 @@ struct DomainSlot {
   void* pdfs = nullptr;
   uint32_t* runs = nullptr;    // run-compressed adjacency
   uint32_t* runOff = nullptr;
+  lbm::BatchOdd* odd = nullptr;
+  uint32_t ahead = 0;          // batch_odd_order
   int nTiles = 0;
   size_t bytes = 0;
   int dims[3] = {0, 0, 0};
@@ -73,6 +75,12 @@ struct Batch {
   int* dDomTileCount = nullptr;
   double* dMoments = nullptr;
   lbm::BatchLaunch evenL{256, 1, 0}, oddL{256, 1, 0};
+  bool separate = false;             // launches of their own for even and odd steps were asked for
+  lbm::PairArgs<3> pair{};           // fused pairs (nItems 0: none), as uploaded to dPair
+  lbm::PairArgs<3>* dPair = nullptr;
+  lbm::PairItem* dItems = nullptr;   // capacity itemCap
+  uint32_t* dCount = nullptr;        // capacity tileCap tiles
+  uint32_t itemCap = 0, gridItems = 0;
   std::map<int, cudaGraphExec_t> graphs;  // steps -> instantiated graph
   long long launches = 0;
   int numSMs = 148;
@@ -96,18 +104,74 @@ void drop_graphs(Batch* b) {
   b->graphs.clear();
 }
 
+// Fused pairs (two steps in one launch) for the tables just published, where
+// they are the faster way.
+//
+// The lead of the even steps: the blocks that run at once beyond what the
+// domain that needs it most needs its even tiles ahead; all tiles in a smaller
+// batch (FP32, 73905 / 17191 tiles, us per step: 459 / 105.1 at 740 resident
+// blocks, 470 / 105.9 at 925, 478 / 106.2 at 1110, 507 / 111 at 1400). The PDFs
+// in between have to stay in 2/5 of L2 as for one lattice.
+//
+// Worth it once the PDFs outgrow half of L2; below, both launches find them
+// there. us per step, a launch per step / fused: FP32 49 MB 14.9 / 16.3, 85 MB
+// 33.2 / 29.5, 104 MB 41.8 / 35.4, 334 MB 128.5 / 107.6; FP16 24 MB 13.6 / 14.9,
+// 43 MB 23.7 / 24.7, 52 MB 31.1 / 30.7, 167 MB 101.1 / 93.4.
+int publish_pairs(Batch* b, uint32_t ahead) {
+  const uint32_t n = static_cast<uint32_t>(b->nTiles);
+  const uint32_t margin = std::max<uint32_t>(lbm::batch_pair_resident(b->storage), 2u << lbm::pair_group_shift(n));
+  const uint32_t lead = std::min(n, margin + ahead);
+  int dev = 0, l2 = 0;
+  BCK(cudaGetDevice(&dev));
+  BCK(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev));
+  const bool fused = (double)n * lbm::kBatchTileNodes * Q * b->elemBytes > 0.5 * l2 &&
+                     (double)lead * lbm::kBatchTileNodes * Q * b->elemBytes <= 0.4 * l2;
+  if (fused != (b->pair.nItems > 0)) drop_graphs(b);
+  b->pair.nItems = 0;
+  if (!fused) return 0;
+  const uint32_t nItems = n + lead;
+  if (nItems > b->itemCap) {
+    BCK(cudaStreamSynchronize(b->stream));
+    lbm::dev_free(b->dItems);
+    b->dItems = nullptr;
+    b->itemCap = 0;
+    BCK(lbm::dev_alloc(&b->dItems, sizeof(lbm::PairItem) * (size_t)(nItems + nItems / 2)));
+    b->itemCap = nItems + nItems / 2;
+  }
+  if (nItems > b->gridItems || nItems < b->gridItems / 2) {
+    drop_graphs(b);
+    b->gridItems = nItems + nItems / 8;
+  }
+  const int shift = lbm::pair_group_shift(n);
+  const size_t groups = ((n - 1) >> shift) + 1;
+  b->pair.items = b->dItems;
+  b->pair.count = b->dCount;
+  b->pair.launches = b->dCount + groups;
+  b->pair.nTiles = n;
+  b->pair.shift = shift;
+  b->pair.prefetch = 0;
+  b->pair.nItems = nItems;
+  BCK(cudaMemsetAsync(b->dCount, 0, sizeof(uint32_t) * (groups + 2), b->stream));
+  BCK(cudaMemcpyAsync(b->dPair, &b->pair, sizeof(b->pair), cudaMemcpyHostToDevice, b->stream));
+  lbm::batch_build_items(b->dDoms, b->dTileDom, b->nTiles, lead, b->dItems, b->stream);
+  BCK(cudaGetLastError());
+  return 0;
+}
+
 // Rebuilds the tile table, the per-domain tile ranges and the tile records
 // after a change of membership (stream-ordered uploads, then a device pass
 // that fills the records).
 int publish(Batch* b) {
   b->tileDomHost.clear();
   std::vector<int> start(b->maxSlots, 0), count(b->maxSlots, 0);
+  uint32_t ahead = 0;
   for (int s = 0; s < b->maxSlots; ++s) {
     DomainSlot& d = b->slots[s];
     if (!d.active) continue;
     d.dev.tileStart = (int)b->tileDomHost.size();
     start[s] = d.dev.tileStart;
     count[s] = d.nTiles;
+    ahead = std::max(ahead, d.ahead);
     for (int t = 0; t < d.nTiles; ++t) b->tileDomHost.push_back(s);
     BCK(cudaMemcpyAsync(b->dDoms + s, &d.dev, sizeof(lbm::BatchDomain), cudaMemcpyHostToDevice, b->stream));
   }
@@ -121,10 +185,13 @@ int publish(Batch* b) {
     BCK(cudaStreamSynchronize(b->stream));
     drop_graphs(b);
     lbm::dev_free(b->dTiles);
+    lbm::dev_free(b->dCount);
     b->dTiles = nullptr;
+    b->dCount = nullptr;
     b->tileCap = 0;
     const int cap = std::min(b->maxTiles, std::max(b->nTiles + b->nTiles / 2, 1024));
     BCK(lbm::dev_alloc(&b->dTiles, sizeof(lbm::BatchTile) * (size_t)cap));
+    BCK(lbm::dev_alloc(&b->dCount, sizeof(uint32_t) * ((size_t)cap / 8 + 4)));  // groups of 8 tiles or more
     b->tileCap = cap;
   }
   // the grid of one-block-per-tile launches keeps some headroom, so that
@@ -142,13 +209,26 @@ int publish(Batch* b) {
   BCK(cudaMemcpyAsync(b->dDomTileCount, count.data(), sizeof(int) * b->maxSlots, cudaMemcpyHostToDevice, b->stream));
   lbm::batch_build_tiles(b->dDoms, b->dTileDom, b->nTiles, b->dTiles, b->stream);
   BCK(cudaGetLastError());
+  const int rc = publish_pairs(b, ahead);
+  if (rc) return rc;
   // the host vectors above are read by the copies: wait before they go away
   BCK(cudaStreamSynchronize(b->stream));
   return 0;
 }
 
+bool fused(const Batch* b) { return b->pair.nItems > 0 && !b->separate; }
+
 int enqueue(Batch* b, int nsteps) {
   if (b->nTiles == 0) return 0;
+  if (fused(b)) {
+    const lbm::BatchPairArgs a{b->dTiles, b->dPair, b->dErr, b->storage};
+    for (int it = 0; it < nsteps; it += 2) {
+      lbm::batch_pair_lp(a, (int)b->gridItems, b->stream);
+      ++b->launches;
+    }
+    BCK(cudaGetLastError());
+    return 0;
+  }
   const lbm::BatchArgs ae = args_of(b, b->evenL), ao = args_of(b, b->oddL);
   for (int it = 0; it < nsteps; it += 2) {
     lbm::batch_even_lp(ae, b->evenL, b->evenL.blocks ? b->evenL.blocks : b->gridTiles, b->stream);
@@ -240,6 +320,7 @@ void* lbm_batch_create(int storage, double budgetGB, int maxDomains) {
             lbm::dev_alloc(&b->dTileDom, sizeof(int) * b->maxTiles) == cudaSuccess &&
             lbm::dev_alloc(&b->dNTiles, sizeof(int)) == cudaSuccess &&
             lbm::dev_alloc(&b->dErr, sizeof(int)) == cudaSuccess &&
+            lbm::dev_alloc(&b->dPair, sizeof(lbm::PairArgs<3>)) == cudaSuccess &&
             lbm::dev_alloc(&b->dPartials, sizeof(double) * 4 * (size_t)b->maxTiles) == cudaSuccess &&
             lbm::dev_alloc(&b->dDomTileStart, sizeof(int) * b->maxSlots) == cudaSuccess &&
             lbm::dev_alloc(&b->dDomTileCount, sizeof(int) * b->maxSlots) == cudaSuccess &&
@@ -264,7 +345,11 @@ void lbm_batch_destroy(void* h) {
     lbm::dev_free(s.pdfs);
     lbm::dev_free(s.runs);
     lbm::dev_free(s.runOff);
+    lbm::dev_free(s.odd);
   }
+  lbm::dev_free(b->dPair);
+  lbm::dev_free(b->dItems);
+  lbm::dev_free(b->dCount);
   lbm::dev_free(b->dDoms);
   lbm::dev_free(b->dTileDom);
   lbm::dev_free(b->dTiles);
@@ -324,8 +409,20 @@ int lbm_batch_add(void* h, const LatticeDesc* ld, double omega, double lambda, d
   BCK(built);
   int rrc = 0;
   size_t runBytes = 0;
+  const int nTiles = (int)(nCells / lbm::kBatchTileNodes);
+  std::vector<uint32_t> reach;
+  uint32_t* dReach = nullptr;
+  if (nf == nFluid) {
+    for (int t = 0; t < 3 * nTiles; ++t) reach.insert(reach.end(), {1u, 0u});  // no node: reaches nothing
+    if (nFluid > 0) {
+      BCK(lbm::dev_alloc(&dReach, sizeof(uint32_t) * reach.size()));
+      lbm::list_tile_reach(adj, nFluid, nCells, dReach, b->stream);
+      BCK(cudaMemcpyAsync(reach.data(), dReach, sizeof(uint32_t) * reach.size(), cudaMemcpyDeviceToHost, b->stream));
+    }
+  }
   if (nf == nFluid) rrc = lbm::list_runs_device(adj, (int)nCells, b->stream, &d.runs, &d.runOff, &runBytes);
   lbm::dev_free(adj);
+  lbm::dev_free(dReach);
   if (nf != nFluid || rrc) {
     g_batchError = rrc ? "building the run-compressed adjacency failed"
                        : (nf < 0 ? berr : "the mask's fluid cell count differs from the lattice's");
@@ -333,9 +430,13 @@ int lbm_batch_add(void* h, const LatticeDesc* ld, double omega, double lambda, d
     d = DomainSlot();
     return -6;
   }
+  std::vector<lbm::BatchOdd> odd;
+  d.ahead = lbm::batch_odd_order(reach.data(), nTiles, odd);
+  BCK(lbm::dev_alloc(&d.odd, sizeof(lbm::BatchOdd) * odd.size()));
+  BCK(cudaMemcpyAsync(d.odd, odd.data(), sizeof(lbm::BatchOdd) * odd.size(), cudaMemcpyHostToDevice, b->stream));
   d.active = true;
   d.bytes = bytes;
-  d.nTiles = (int)(nCells / lbm::kBatchTileNodes);
+  d.nTiles = nTiles;
   for (int i = 0; i < 3; ++i) d.dims[i] = ld->Dims[i];
   d.omega = omega;
   d.lambda = lambda;
@@ -346,6 +447,7 @@ int lbm_batch_add(void* h, const LatticeDesc* ld, double omega, double lambda, d
   d.dev.nCells = nCells;
   d.dev.nFluid = nFluid;
   d.dev.trt = trt_of(omega, lambda, xforce);
+  d.dev.odd = d.odd;
   b->used += bytes;
   int rc = lbm_batch_reset(h, slot);
   if (rc) return rc;
@@ -361,6 +463,7 @@ int lbm_batch_remove(void* h, int slot) {
   lbm::dev_free(d.pdfs);
   lbm::dev_free(d.runs);
   lbm::dev_free(d.runOff);
+  lbm::dev_free(d.odd);
   b->used -= d.bytes;
   d = DomainSlot();
   return publish(b);
@@ -399,7 +502,7 @@ int lbm_batch_step(void* h, int nsteps, int use_graph) {
     it = b->graphs.emplace(nsteps, ge).first;
   }
   BCK(cudaGraphLaunch(it->second, b->stream));
-  b->launches += nsteps;
+  b->launches += fused(b) ? nsteps / 2 : nsteps;
   return 0;
 }
 
@@ -490,6 +593,7 @@ int lbm_batch_set_launch(void* h, int which, int threads, int blocks) {
   lbm::BatchLaunch l{threads, lbm::kBatchTileNodes / threads, blocks};
   if (which == 0 || which == 2) b->evenL = l;
   if (which == 1 || which == 2) b->oddL = l;
+  b->separate = true;
   drop_graphs(b);
   return 0;
 }
@@ -536,6 +640,8 @@ int lbm_batch_tune(void* h, int trialSteps, double* results, int maxRows) {
   const int threadsC[3] = {256, 128, 64};
   const int perSM[6] = {0, 2, 3, 4, 5, 6};  // 0: one block per tile
   int rows = 0;
+  const bool asked = b->separate;
+  b->separate = true;
   for (int which = 0; which < 2; ++which) {
     double bestMs = 1e300;
     lbm::BatchLaunch best = which == 0 ? b->evenL : b->oddL;
@@ -555,6 +661,7 @@ int lbm_batch_tune(void* h, int trialSteps, double* results, int maxRows) {
       }
     if (which == 0) b->evenL = best; else b->oddL = best;
   }
+  b->separate = asked;
   drop_graphs(b);
   return std::min(rows, maxRows);
 }

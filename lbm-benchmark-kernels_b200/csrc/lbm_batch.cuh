@@ -1,6 +1,7 @@
 // lbm_batch.cuh -- device side of the batched list AA form: many independent
-// porous domains of uneven size advanced by one launch per time step (a
-// persistent grid, or one block per tile) (no counterpart in the reference, which runs one domain per process).
+// porous domains of uneven size advanced together, by one launch per pair of
+// time steps or one per time step (a persistent grid, or one block per tile)
+// (no counterpart in the reference, which runs one domain per process).
 //
 // Each domain keeps its own list layout (fluid nodes numbered as the
 // reference's list kernels, adjacency with 32-bit PDF indices relative to the
@@ -11,12 +12,19 @@
 // stays valid when domains are admitted or retired.
 #pragma once
 #include <cstdint>
+#include <vector>
 
 #include "lbm_kernels.cuh"
 
 namespace lbm {
 
 constexpr int kBatchTileNodes = 256;  // node granularity of a domain's tiles
+
+// Odd step of one tile of a domain (tile numbers within the domain): the even
+// tiles it needs, by links with c_x = -1, 0, +1 (lowest > highest: none).
+struct BatchOdd {
+  uint32_t tile, lo[3], hi[3];
+};
 
 struct BatchDomain {
   void* f;                // PDFs, storage format of the batch, f[d * nCells + n]
@@ -26,6 +34,7 @@ struct BatchDomain {
   int nFluid;
   int tileStart;          // first tile of this domain in the tile table
   TrtW trt;               // relaxation rates and body force of this domain
+  const BatchOdd* odd;    // its tiles in the order of their odd steps in a fused pair
 };
 
 // Everything a block needs to update one tile, built on the device from the
@@ -55,6 +64,17 @@ struct BatchArgs {
   int nodesPerThread;
 };
 
+// Fused even/odd pairs of the whole batch (lbm_pair.cuh): item k is the even
+// step of tile k and the odd step number k - lead, domain after domain in the
+// order of BatchDomain::odd. The PairArgs lie in device memory, so that a
+// captured launch stays valid as domains come and go.
+struct BatchPairArgs {
+  const BatchTile* tiles;
+  const PairArgs<3>* pair;
+  int* err;
+  int storage;
+};
+
 // Launch configuration picked by the autotuner.
 struct BatchLaunch {
   int threads;         // block size
@@ -70,6 +90,17 @@ void batch_pad_adjacency(uint32_t* adj, int nFluid, long long nCells, cudaStream
 
 // Builds the tile records of tiles [0, nTiles).
 void batch_build_tiles(const BatchDomain* doms, const int* tileDom, int nTiles, BatchTile* out, cudaStream_t s);
+
+// Host: a domain's odd steps in order, from list_tile_reach (nTiles tiles);
+// returns the most that a step's last even tile is ahead of the step's number.
+uint32_t batch_odd_order(const uint32_t* reach, int nTiles, std::vector<BatchOdd>& odd);
+// The nTiles + lead items of the pairs (device), after batch_build_tiles.
+void batch_build_items(const BatchDomain* doms, const int* tileDom, int nTiles, uint32_t lead, PairItem* items,
+                       cudaStream_t s);
+// Blocks of the fused kernel that run at once.
+int batch_pair_resident(int storage);
+// grid: at least the pair's nItems.
+void batch_pair_lp(const BatchPairArgs& a, int grid, cudaStream_t s);
 
 // grid: the launch's block count (l.blocks, or the tile-grid size when
 // l.blocks is 0).

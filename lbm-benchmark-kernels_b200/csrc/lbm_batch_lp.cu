@@ -10,6 +10,7 @@
 #include "lbm_batch.cuh"
 #include "lbm_bulk.cuh"
 #include "lbm_chain.cuh"
+#include "lbm_pair.cuh"
 #include "lbm_store.cuh"
 
 namespace lbm {
@@ -210,6 +211,125 @@ __global__ void __launch_bounds__(kBatchTileNodes / NPT, 6 * NPT) k_batch_odd_ti
     const int local = threadIdx.x + k * (kBatchTileNodes / NPT);
     if (local < st.nValid) batch_odd_node<St>(st, srun, local);
   }
+}
+
+// The fused pair (lbm_pair.cuh) of all domains, with the tile records of the
+// other kernels: each thread reads the even tile's, the service warp stages the
+// odd tile's. What bounds it: as the list's pair, L2 and its latency, with the
+// tile records' on top (5 blocks per SM, 40 registers; packed arithmetic
+// spills: 0.478 -> 0.514 ms per step at 73905 tiles; records fetched ahead
+// into L2 0.469 -> 0.478). FP32, 48 domains of edge 32 to 128, 73905 tiles:
+// 0.559 -> 0.459 ms per step (41 GFLUP/s), FP16 0.432 -> 0.407.
+template <class St>
+__global__ void __launch_bounds__(kPairThreads, 5) k_batch_pair(const BatchPairArgs a) {
+  __shared__ ListPairShared sh;
+  __shared__ __align__(16) BatchTile odd;
+  pair_init(&sh);
+  const uint32_t k = blockIdx.x;
+  if (k >= a.pair->nItems) {
+    chain_wait();
+    return;
+  }
+  if (threadIdx.x >= kListTile) {
+    const PairArgs<3> p = *a.pair;
+    const int lane = threadIdx.x - kListTile;
+    pair_serve(&sh, p, [&](const PairItem& it) -> const void* {
+      if (it.tile == kPairNone) return nullptr;
+      if (lane < kTileWords)
+        reinterpret_cast<uint32_t*>(&odd)[lane] =
+            __ldg(reinterpret_cast<const uint32_t*>(a.tiles + it.tile) + lane);
+      __syncwarp();
+      return odd.run;
+    }, a.err, k);
+    return;
+  }
+  using T = typename St::T;
+  const bool even = k < a.pair->nTiles;
+  BatchTile et;
+  if (even) et = a.tiles[k];
+  chain_wait();
+  if (even) {
+    if (static_cast<int>(threadIdx.x) < et.nValid)
+      lp_even_node<St, false, PairAccess>(static_cast<T*>(et.f), et.nCells, et.n0 + threadIdx.x, TrtDev<St>(et.trt));
+    pair_even_done(&sh);
+  }
+  if (!pair_odd_turn(&sh, a.err)) return;
+  if (sh.item.run16 == 0) {
+    if (threadIdx.x == 0) atomicOr(a.err, 4);
+    return;
+  }
+  if (static_cast<int>(threadIdx.x) >= odd.nValid) return;
+  uint32_t off;
+  const uint32_t* e = run_row(sh.run, threadIdx.x, off);
+  lp_odd_node<St, false, PairAccess>(static_cast<T*>(odd.f), static_cast<uint32_t>(odd.nCells), odd.n0 + threadIdx.x, e,
+                                     off, TrtDev<St>(odd.trt));
+}
+
+int batch_pair_resident(int storage) {
+  static std::atomic<int> n32{0}, n16{0};
+  if (storage == kStoreF16) return prefetch_distance(n16, k_batch_pair<StoreF16>, kPairThreads, true);
+  return prefetch_distance(n32, k_batch_pair<StoreF32>, kPairThreads, true);
+}
+
+void batch_pair_lp(const BatchPairArgs& a, int grid, cudaStream_t s) {
+  if (a.storage == kStoreF16)
+    launch_chained(k_batch_pair<StoreF16>, grid, kPairThreads, 0, s, a);
+  else
+    launch_chained(k_batch_pair<StoreF32>, grid, kPairThreads, 0, s, a);
+}
+
+uint32_t batch_odd_order(const uint32_t* reach, int nTiles, std::vector<BatchOdd>& odd) {
+  std::vector<uint32_t> need(nTiles), first(nTiles + 1, 0);
+  for (int t = 0; t < nTiles; ++t) {
+    need[t] = static_cast<uint32_t>(t);
+    for (int c = 0; c < 3; ++c)
+      if (reach[6 * (size_t)t + 2 * c] <= reach[6 * (size_t)t + 2 * c + 1])
+        need[t] = std::max(need[t], reach[6 * (size_t)t + 2 * c + 1]);
+    ++first[need[t] + 1];
+  }
+  for (int t = 0; t < nTiles; ++t) first[t + 1] += first[t];
+  odd.resize(nTiles);
+  uint32_t ahead = 0;
+  for (int t = 0; t < nTiles; ++t) {
+    const uint32_t i = first[need[t]]++;
+    BatchOdd& o = odd[i];
+    o.tile = static_cast<uint32_t>(t);
+    for (int c = 0; c < 3; ++c) {
+      o.lo[c] = reach[6 * (size_t)t + 2 * c];
+      o.hi[c] = reach[6 * (size_t)t + 2 * c + 1];
+    }
+    ahead = std::max(ahead, need[t] > i ? need[t] - i : 0u);
+  }
+  return ahead;
+}
+
+__global__ void k_batch_items(const BatchDomain* doms, const int* tileDom, uint32_t nTiles, uint32_t lead, int shift,
+                              PairItem* items) {
+  const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= nTiles + lead) return;
+  PairItem it = {};
+  it.tile = kPairNone;
+  if (k >= lead) {
+    const BatchDomain& D = doms[tileDom[k - lead]];
+    const uint32_t start = static_cast<uint32_t>(D.tileStart);
+    const BatchOdd o = D.odd[k - lead - start];
+    it.tile = start + o.tile;
+    const uint32_t r16 = D.runOff[o.tile + 1] - D.runOff[o.tile];
+    it.run16 = run_bytes_ok(r16 * 16u) ? r16 : 0u;
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+      if (o.lo[c] <= o.hi[c]) {
+        it.lo[c] = (start + o.lo[c]) >> shift;
+        it.n[c] = ((start + o.hi[c]) >> shift) - it.lo[c] + 1u;
+      }
+  }
+  items[k] = it;
+}
+
+void batch_build_items(const BatchDomain* doms, const int* tileDom, int nTiles, uint32_t lead, PairItem* items,
+                       cudaStream_t s) {
+  const uint32_t n = static_cast<uint32_t>(nTiles);
+  k_batch_items<<<(n + lead + 255) / 256, 256, 0, s>>>(doms, tileDom, n, lead, pair_group_shift(n), items);
 }
 
 template <class St>

@@ -123,14 +123,13 @@ __device__ __forceinline__ bool pair_ready(const PairRec<R>& it, const PairArgs<
   return __all_sync(0xffffffffu, good);
 }
 
-// The service warp of block k (see above); runs: the array that the items'
-// staged data lies in.
+// The service warp of block k (see above); runs(item), called by the whole warp:
+// the array that the item's staged data lies in.
 // first: where the run record of the item's first tile goes (two-grid lists),
 // or null.
-template <int R, int kWords>
-__device__ __forceinline__ void pair_service(PairShared<R, kWords>* sh, const PairArgs<R>& p, const void* runs,
-                                             int* err, uint32_t k, uint32_t* second = nullptr,
-                                             uint32_t* first = nullptr) {
+template <int R, int kWords, class Runs>
+__device__ __forceinline__ void pair_serve(PairShared<R, kWords>* sh, const PairArgs<R>& p, Runs runs, int* err,
+                                           uint32_t k, uint32_t* second = nullptr, uint32_t* first = nullptr) {
   constexpr int kItemWords = static_cast<int>(sizeof(PairRec<R>) / 4);
   static_assert(kItemWords <= 32, "one item word per lane");
   const int lane = threadIdx.x - kListTile;
@@ -139,7 +138,7 @@ __device__ __forceinline__ void pair_service(PairShared<R, kWords>* sh, const Pa
     reinterpret_cast<uint32_t*>(&sh->item)[lane] = __ldg(reinterpret_cast<const uint32_t*>(p.items + k) + lane);
   __syncwarp();
   const PairRec<R>& it = sh->item;
-  const char* const base = static_cast<const char*>(runs);
+  const char* const base = static_cast<const char*>(runs(it));
   if (lane == 0) {
     if (first && it.firstRun16) {
       mbar_expect_tx(&sh->named, it.firstRun16 * 16u);
@@ -178,6 +177,13 @@ __device__ __forceinline__ void pair_service(PairShared<R, kWords>* sh, const Pa
     }
     if (lane == 0) mbar_arrive(&sh->go);
   }
+}
+
+template <int R, int kWords>
+__device__ __forceinline__ void pair_service(PairShared<R, kWords>* sh, const PairArgs<R>& p, const void* runs,
+                                             int* err, uint32_t k, uint32_t* second = nullptr,
+                                             uint32_t* first = nullptr) {
+  pair_serve(sh, p, [&](const PairRec<R>&) { return runs; }, err, k, second, first);
 }
 
 // Compute warps: their even nodes are stored.

@@ -169,3 +169,39 @@ def test_autotuner_picks_a_candidate():
         b.sync()
     finally:
         b.close()
+
+
+@pytest.mark.parametrize("prec", ["fp32", "fp16"])
+@pytest.mark.parametrize("graph", [False, True])
+def test_fused_pairs_equal_separate_launches(prec, graph):
+    """Both steps of a pair in one launch against a launch per step, for domains
+    of less than a tile up to more tiles than the even steps lead by, while
+    domains come and go."""
+    lats = [lbmb200.spheres((96, 120, 88), 3, 0.7, 3.0, 8.0)[0], lbmb200.geometry("fluid", (5, 4, 6), (1, 1, 1)),
+            lbmb200.geometry("channel", (61, 33, 47), (1, 0, 0)), lbmb200.geometry("box", (16, 16, 18), (0, 0, 0)),
+            lbmb200.spheres((150, 61, 64), 4, 0.6, 3.0, 8.0)[0], lbmb200.geometry("fluid", (700, 9, 7), (1, 1, 1)),
+            lbmb200.geometry("fluid", (128, 64, 65), (1, 1, 1))]
+    inits = [random_pdfs(lat.mask.size, 11 + k, amp=0.02) for k, lat in enumerate(lats)]
+    fields = []
+    for separate in (False, True):
+        b = lbmb200.Batch(prec, budget_gb=8.0, max_domains=8)
+        try:
+            if separate:
+                b.set_launch("both", 256, 0)
+            slots = {}
+            for k in (0, 4, 5, 6, 1):
+                slots[k] = b.add(lats[k], omega=1.0 + 0.1 * k, xforce=1e-4)
+                b.set_field(slots[k], inits[k])
+            b.step(10, graph=graph)
+            b.remove(slots.pop(5))
+            for k in (2, 3):
+                slots[k] = b.add(lats[k], omega=1.0 + 0.1 * k, xforce=1e-4)
+                b.set_field(slots[k], inits[k])
+            b.step(10, graph=graph)
+            b.step(6, graph=graph)
+            b.sync()
+            fields.append([b.get_field(slots[k])[lats[k].mask != 0] for k in sorted(slots)])
+        finally:
+            b.close()
+    for one, two in zip(*fields):
+        assert np.array_equal(one, two)
