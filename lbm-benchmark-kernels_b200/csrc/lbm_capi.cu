@@ -84,7 +84,6 @@ struct Gpu {
   int* dOddItems;          // odd step: nOddItems interior work items (aa_interior_items)
   int* dOddCells;          // odd step: the general cells of the items, in chunks of 128
   int nOddItems;
-  bool oddItemsBuilt;
   // x-slab of a larger lattice (lbm_aa_slab_init): halo/cross flags of the two x faces
   int halo[2], cross[2];
   int* sliceMask;          // the slab's own mask (owned)
@@ -811,10 +810,11 @@ void schedule_aa_pairs(Gpu* g, const LatticeDesc* ld) {
   pair_upload(g, items, nTiles);
 }
 
-// The interior work items of the AA odd step by itself (slabs), from the link
-// words.
+// The interior work items of the AA odd step by itself, from the link words:
+// for slabs, and for whole lattices too, which the slab entry points step half
+// by half on any stream, captured or not (256^3: 24 ms of the 4.5 s that the
+// links take).
 void build_odd_items(Gpu* g, const uint32_t* link) {
-  g->oddItemsBuilt = true;
   const lbm::AaArgs aa = aa_args(g);
   if (lbm::aa_interior_block_count(aa) <= 0) return;
   std::vector<int> items, cells;
@@ -828,15 +828,6 @@ void build_odd_items(Gpu* g, const uint32_t* link) {
     LBM_CK(lbm::dev_alloc(&g->dOddCells, sizeof(int) * cells.size()));
     LBM_CK(cudaMemcpyAsync(g->dOddCells, cells.data(), sizeof(int) * cells.size(), cudaMemcpyHostToDevice, g->stream));
   }
-}
-
-// The slab entry points also step a whole full-array AA instance half by half;
-// it gets its work items on the first such call.
-void need_odd_items(Gpu* g) {
-  if (g->kind != kAa || g->oddItemsBuilt) return;
-  std::vector<uint32_t> link((size_t)g->dstride);
-  LBM_CK(cudaMemcpyAsync(link.data(), g->dLink, sizeof(uint32_t) * link.size(), cudaMemcpyDeviceToHost));
-  build_odd_items(g, link.data());
 }
 
 // --- Init / Deinit ----------------------------------------------------------------
@@ -934,7 +925,7 @@ Gpu* gpu_new(Kind kind, LatticeDesc* ld, Parameters* params, const SlabSpec* sla
       LBM_CK(cudaMemsetAsync(g->dG, 0, sizeof(double) * g->mirrorElems, g->stream));
     }
     if (!slab) schedule_aa_pairs(g, ld);
-    if (kind == kAa && slab) build_odd_items(g, link);
+    if (kind == kAa) build_odd_items(g, link);
     std::free(link);
   } else {
     const bool pull = kind == kListPull || kind == kListPullPlain;
@@ -1564,7 +1555,6 @@ int lbm_aa_slab_step(KernelData* kd, CaseData* cd, int half, void* stream) {
     }
     return (int)cudaGetLastError();
   }
-  need_odd_items(g);
   const lbm::AaArgs a = aa_args(g);
   if (half == 0) {
     lbm::aa_even_fp64(a, t, s);
@@ -1652,7 +1642,6 @@ int lbm_aa_slab_odd_part(KernelData* kd, CaseData* cd, int part, void* stream) {
         lbm::list_odd_fp64_tiles(list_args(g), t, t0, t1, s);
     }
   } else {
-    need_odd_items(g);
     const lbm::AaArgs a = aa_args(g);
     if (part == 0) {
       // the interior blocks read and write only the slab's own planes

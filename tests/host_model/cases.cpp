@@ -1,0 +1,158 @@
+// Cases of the host layer on the model of fake_runtime.hpp: `cases NAME` runs
+// one and returns 0 if everything held. The step launchers are stand-ins that
+// look, when their stream runs, at what the kernels would read.
+#include "fake_runtime.hpp"
+
+#include <string>
+
+#include "../../include/lbm_b200.h"
+#include "../../lbm-benchmark-kernels_b200/csrc/lbm_batch.cuh"
+#include "../../lbm-benchmark-kernels_b200/csrc/lbm_kernels.cuh"
+
+namespace {
+
+int g_bad = 0;
+void check(bool ok, const char* what) {
+  if (ok) return;
+  std::printf("not so: %s\n", what);
+  ++g_bad;
+}
+
+// The interior work items of the AA odd step that aa_interior_items gives out.
+std::vector<int> odd_items() { return {0, 3, ~0, 5, ~1}; }
+std::vector<int> odd_cells() {
+  std::vector<int> c(256);
+  for (int k = 0; k < 256; ++k) c[k] = 7 * k + 1;
+  return c;
+}
+
+struct Lattice {
+  LatticeDesc ld{};
+  std::vector<int> mask;
+  Lattice(int nx, int ny, int nz) : mask((size_t)nx * ny * nz, LAT_CELL_FLUID) {
+    ld.Dims[0] = nx;
+    ld.Dims[1] = ny;
+    ld.Dims[2] = nz;
+    ld.Lattice = mask.data();
+    ld.nCells = ld.nFluid = nx * ny * nz;
+    ld.PeriodicX = ld.PeriodicY = ld.PeriodicZ = 1;
+    ld.Name = "fluid";
+  }
+};
+
+KernelData* full_array(Lattice& lat) {
+  Parameters p{};
+  KernelData* kd = nullptr;
+  D3Q19CudaAaInit_AaSoA(&lat.ld, &kd, &p);
+  return kd;
+}
+
+CaseData a_case() {
+  CaseData cd{};
+  cd.Omega = 1.2;
+  cd.MaxIterations = 2;
+  return cd;
+}
+
+}  // namespace
+
+namespace lbm {
+
+long long aa_interior_block_count(const AaArgs&) { return 8; }
+bool aa_shell_needed(const AaArgs&) { return false; }
+void aa_interior_items(const AaArgs&, const uint32_t*, std::vector<int>& items, std::vector<int>& cells) {
+  items = odd_items();
+  cells = odd_cells();
+}
+AaPairGeom aa_pair_geom(const AaArgs& a) {
+  AaPairGeom g{};
+  g.tpp = 1;
+  g.nX = (uint32_t)a.nX;
+  return g;
+}
+int aa_resident_tiles() { return 0; }
+int aa_pair_resident() { return 4; }
+void aa_pair_schedule(const AaArgs&, const AaPairGeom& g, int, std::vector<AaPairItem>& items) {
+  items.assign(g.nX + 2, AaPairItem{});
+  for (size_t k = 0; k < items.size(); ++k) items[k].tile = (uint32_t)k;
+}
+void aa_pair_fp64(const AaArgs& a, const AaPairArgs& q, const Trt<double>&, cudaStream_t s) {
+  fake::launch(s, [=] {
+    for (uint32_t k = 0; k < q.p.nItems; ++k) check(q.p.items[k].tile == k, "the fused pair reads its items");
+    check(*q.p.count == 0, "the counters start at zero");
+    a.f[0] += 1.0;
+  });
+}
+void aa_even_fp64(const AaArgs& a, const Trt<double>&, cudaStream_t s) {
+  fake::launch(s, [=] { a.f[0] += 1.0; });
+}
+void aa_odd_interior_fp64(const AaArgs&, const Trt<double>&, const int* items, int nItems, const int* cells,
+                          cudaStream_t s) {
+  fake::launch(s, [=] {
+    check(std::vector<int>(items, items + nItems) == odd_items(), "the odd step reads its work items");
+    const std::vector<int> want = odd_cells();
+    check(std::vector<int>(cells, cells + want.size()) == want, "the odd step reads its cell lists");
+  });
+}
+
+}  // namespace lbm
+
+namespace {
+
+// The first half step of a whole-lattice instance on the caller's own stream.
+void first_slab_step(int how) {
+  Lattice lat(6, 5, 4);
+  KernelData* kd = full_array(lat);
+  cudaStream_t mine;
+  cudaStreamCreateWithFlags(&mine, cudaStreamNonBlocking);
+  CaseData cd = a_case();
+  int rc = 0;
+  if (how == 0) rc = lbm_aa_slab_odd_part(kd, &cd, 0, mine);
+  if (how == 1) rc = lbm_aa_slab_step(kd, &cd, 1, mine);
+  if (how == 2) rc = lbm_aa_slab_step(kd, &cd, 0, mine) | lbm_aa_slab_step(kd, &cd, 1, mine);
+  check(rc == 0, "the step is accepted");
+  cudaStreamSynchronize(mine);
+  D3Q19CudaAaDeinit_AaSoA(&lat.ld, &kd);
+}
+
+// The same captured into a graph: nothing is allocated, copied or waited for.
+void first_slab_step_captured() {
+  Lattice lat(6, 5, 4);
+  KernelData* kd = full_array(lat);
+  cudaStream_t mine;
+  cudaStreamCreateWithFlags(&mine, cudaStreamNonBlocking);
+  CaseData cd = a_case();
+  const size_t blocks = fake::blocks.size();
+  cudaStreamBeginCapture(mine, cudaStreamCaptureModeGlobal);
+  fake::calls = 0;
+  check(lbm_aa_slab_step(kd, &cd, 0, mine) == 0 && lbm_aa_slab_step(kd, &cd, 1, mine) == 0, "the steps are accepted");
+  check(fake::calls == 0 && fake::blocks.size() == blocks, "a step is a launch and nothing else");
+  cudaGraph_t g;
+  cudaGraphExec_t e;
+  cudaStreamEndCapture(mine, &g);
+  cudaGraphInstantiate(&e, g, 0);
+  cudaGraphLaunch(e, mine);
+  cudaStreamSynchronize(mine);
+  cudaGraphExecDestroy(e);
+  cudaGraphDestroy(g);
+  D3Q19CudaAaDeinit_AaSoA(&lat.ld, &kd);
+}
+
+const std::map<std::string, std::function<void()>> kCases = {
+    {"first_odd_part", [] { first_slab_step(0); }},
+    {"first_odd_half", [] { first_slab_step(1); }},
+    {"first_even_half", [] { first_slab_step(2); }},
+    {"first_slab_step_captured", first_slab_step_captured},
+};
+
+}  // namespace
+
+int main(int argc, char** argv) {
+  const auto it = kCases.find(argc > 1 ? argv[1] : "");
+  if (it == kCases.end()) {
+    std::printf("unknown case\n");
+    return 2;
+  }
+  it->second();
+  return g_bad != 0;
+}

@@ -234,3 +234,38 @@ def test_two_grid_steps_in_one_launch(kname, make):
             inst.deinit()
     m = lat.mask != 0
     assert np.array_equal(fields[0][m], fields[1][m])
+
+
+@pytest.mark.parametrize("parts", [False, True])
+def test_first_half_steps_on_a_callers_stream(parts):
+    """The first half steps of a whole-lattice instance may go to any stream."""
+    import ctypes
+
+    import torch
+    lat = lbmb200.geometry("blocks-4", (30, 26, 25), (1, 1, 1))
+    init = random_pdfs(lat.mask.size, 79)
+    cd = lbmb200.case(omega=1.1, xforce=2e-4, iterations=4)
+    L = lbmb200.lib()
+    fields = []
+    for apart in (False, True):
+        inst = lbmb200.kernel("cuda-aa-soa").init(lat, kernel_args=["-lambda", "3/16"])
+        try:
+            inst.set_field(init)
+            if apart:
+                mine = torch.cuda.Stream()
+                st = ctypes.c_void_p(mine.cuda_stream)
+                for half in (0, 1, 0, 1):
+                    if parts:
+                        step = L.lbm_aa_slab_odd_part if half else L.lbm_aa_slab_even_part
+                        assert all(step(inst.kdp, ctypes.byref(cd), k, st) == 0 for k in (0, 1))
+                    else:
+                        assert L.lbm_aa_slab_step(inst.kdp, ctypes.byref(cd), half, st) == 0
+                mine.synchronize()
+                inst.sync_mirror()
+            else:
+                inst.run(cd)
+            fields.append(inst.get_field())
+        finally:
+            inst.deinit()
+    m = lat.mask != 0
+    assert np.array_equal(fields[0][m], fields[1][m])

@@ -1,0 +1,49 @@
+"""The host layer (csrc/lbm_capi.cu, lbm_batch.cu, lbm_mem.cu) on a model of
+the CUDA runtime (tests/host_model): order between streams, lifetimes of host
+and device memory, and failed allocations, which a GPU that happens to be quick
+enough does not show."""
+import os
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CSRC = os.path.join(ROOT, "lbm-benchmark-kernels_b200", "csrc")
+CUDA = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+MODEL = os.path.join(ROOT, "tests", "host_model")
+
+
+@pytest.fixture(scope="module")
+def cases(tmp_path_factory):
+    if not os.path.exists(os.path.join(CUDA, "include", "cuda_runtime.h")):
+        pytest.skip("no CUDA headers")
+    d = tmp_path_factory.mktemp("host_model")
+    flags = ["-g", "-O0", "-fsanitize=address", "-fno-omit-frame-pointer", "-fno-pie", "-I" + CUDA + "/include"]
+    jobs = [["g++", "-std=c++17", "-x", "c++", *flags, "-c", os.path.join(CSRC, f + ".cu"), "-o", str(d / (f + ".o"))]
+            for f in ("lbm_capi", "lbm_batch", "lbm_mem")]
+    jobs.append(["gcc", "-std=c99", "-D_POSIX_C_SOURCE=200112L", *flags, "-c", os.path.join(CSRC, "lbm_host.c"), "-o",
+                 str(d / "lbm_host.o")])
+    jobs.append(["g++", "-std=c++17", *flags, "-c", os.path.join(MODEL, "cases.cpp"), "-o", str(d / "cases.o")])
+    running = [subprocess.Popen(j, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True) for j in jobs]
+    for p in running:
+        out = p.communicate()[0]
+        assert p.returncode == 0, out
+    # launchers that no case reaches stay undefined
+    exe = str(d / "cases")
+    subprocess.run(["g++", "-fsanitize=address", "-no-pie", "-Wl,--unresolved-symbols=ignore-all",
+                    *[str(d / (f + ".o")) for f in ("lbm_capi", "lbm_batch", "lbm_mem", "lbm_host", "cases")],
+                    "-o", exe], check=True)
+    return exe
+
+
+def _run(exe, name):
+    p = subprocess.run([exe, name], capture_output=True, text=True, timeout=60,
+                       env={**os.environ, "ASAN_OPTIONS": "detect_leaks=0"})
+    assert p.returncode == 0, p.stdout + p.stderr[-4000:]
+
+
+@pytest.mark.parametrize("name", ["first_odd_part", "first_odd_half", "first_even_half", "first_slab_step_captured"])
+def test_first_slab_step_on_a_callers_stream(cases, name):
+    """The work items of the odd step are there before any half step that a
+    caller's stream takes, captured or not."""
+    _run(cases, name)
