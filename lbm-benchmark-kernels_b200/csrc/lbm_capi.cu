@@ -60,6 +60,8 @@ struct Gpu {
   size_t elemBytes;  // bytes per stored PDF
   void* rawStage;    // pinned staging buffer of the device format (reduced storage)
 
+  int device;  // current at Init; the memory and the stream are its
+
   // device memory
   double* dF;
   double* dG;
@@ -860,6 +862,7 @@ Gpu* gpu_new(Kind kind, LatticeDesc* ld, Parameters* params, const SlabSpec* sla
   g->per[0] = ld->PeriodicX;
   g->per[1] = ld->PeriodicY;
   g->per[2] = ld->PeriodicZ;
+  LBM_CK(cudaGetDevice(&g->device));
   LBM_CK(cudaStreamCreateWithFlags(&g->stream, cudaStreamNonBlocking));
   LBM_CK(cudaEventCreate(&g->ev0));
   LBM_CK(cudaEventCreate(&g->ev1));
@@ -1035,8 +1038,12 @@ Gpu* gpu_new(Kind kind, LatticeDesc* ld, Parameters* params, const SlabSpec* sla
 void gpu_free(KernelData** kernelData) {
   if (kernelData == nullptr || *kernelData == nullptr) return;
   Gpu* g = reinterpret_cast<Gpu*>(*kernelData);
-  // all streams: slab steps, or a caller that reads the device state, may
-  // still use the memory on another one
+  // all streams of the instance's device, whichever is current: slab steps, or
+  // a caller that reads the device state, may still use the memory on one of
+  // its own, and dev_free does not wait
+  int current = g->device;
+  cudaGetDevice(&current);
+  if (current != g->device) cudaSetDevice(g->device);
   cudaDeviceSynchronize();
   lbm::dev_free(g->dF);
   lbm::dev_free(g->dG);
@@ -1062,6 +1069,7 @@ void gpu_free(KernelData** kernelData) {
   cudaEventDestroy(g->ev0);
   cudaEventDestroy(g->ev1);
   cudaStreamDestroy(g->stream);
+  if (current != g->device) cudaSetDevice(current);
   std::free(g->grid);
   std::free(g->adjHost);
   std::free(g);

@@ -138,11 +138,25 @@ void first_slab_step_captured() {
   D3Q19CudaAaDeinit_AaSoA(&lat.ld, &kd);
 }
 
+// Deinit of an instance whose steps are under way, with another device current.
+void deinit_from_another_device() {
+  Lattice lat(6, 5, 4);
+  KernelData* kd = full_array(lat);
+  CaseData cd = a_case();
+  check(lbm_b200_step_device(kd, &cd, 4) == 0, "the steps are accepted");
+  cudaSetDevice(1);
+  D3Q19CudaAaDeinit_AaSoA(&lat.ld, &kd);
+  check(fake::device == 1, "the caller's device stays current");
+  check(fake::blocks.empty(), "the instance's memory is given back");
+  fake::run_device(0);  // what the free did not wait for uses the memory now
+}
+
 const std::map<std::string, std::function<void()>> kCases = {
     {"first_odd_part", [] { first_slab_step(0); }},
     {"first_odd_half", [] { first_slab_step(1); }},
     {"first_even_half", [] { first_slab_step(2); }},
     {"first_slab_step_captured", first_slab_step_captured},
+    {"deinit_from_another_device", deinit_from_another_device},
 };
 
 }  // namespace

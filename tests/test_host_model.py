@@ -47,3 +47,9 @@ def test_first_slab_step_on_a_callers_stream(cases, name):
     """The work items of the odd step are there before any half step that a
     caller's stream takes, captured or not."""
     _run(cases, name)
+
+
+def test_deinit_waits_for_the_instances_own_device(cases):
+    """Deinit may be called with another device current (a finaliser thread,
+    one process with several devices) while steps are still queued."""
+    _run(cases, "deinit_from_another_device")
