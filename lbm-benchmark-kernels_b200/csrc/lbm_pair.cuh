@@ -160,6 +160,7 @@ __device__ __forceinline__ void pair_serve(PairShared<R, kWords>* sh, const Pair
   // launch can be replayed
   const uint32_t launch = ld_relaxed(p.launches) + 1u;
   const bool ready = it.tile == kPairNone || pair_ready(it, p, launch);
+  __syncwarp();  // the vote orders nothing: what every lane acquired comes before lane 0's arrival
   if (ready && lane == 0) mbar_arrive(&sh->go);
   if (even) {
     if (!mbar_wait_bounded(&sh->even, 0)) atomicOr(err, 1);
@@ -175,6 +176,7 @@ __device__ __forceinline__ void pair_serve(PairShared<R, kWords>* sh, const Pair
         break;
       }
     }
+    __syncwarp();  // as above
     if (lane == 0) mbar_arrive(&sh->go);
   }
 }

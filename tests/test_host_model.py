@@ -53,3 +53,46 @@ def test_deinit_waits_for_the_instances_own_device(cases):
     """Deinit may be called with another device current (a finaliser thread,
     one process with several devices) while steps are still queued."""
     _run(cases, "deinit_from_another_device")
+
+
+def _extract(path, *starts):
+    """The definitions of a source file that begin with the given lines."""
+    text = open(path).read()
+    out = []
+    for start in starts:
+        a = text.index(start)
+        assert text.find(start, a + 1) < 0, start
+        a = max(text.rfind("\n\n", 0, a), text.rfind("\n}\n", 0, a))
+        k = text.index("{", text.index(start))
+        depth = 0
+        for i in range(k, len(text)):
+            depth += {"{": 1, "}": -1}.get(text[i], 0)
+            if depth == 0:
+                break
+        out.append(text[a:i + 1].lstrip("}\n") + (";" if text[i + 1] == ";" else ""))
+    return "\n".join(out)
+
+
+@pytest.fixture(scope="module")
+def service_warp(tmp_path_factory):
+    if not os.path.exists(os.path.join(CUDA, "include", "cuda_runtime.h")):
+        pytest.skip("no CUDA headers")
+    d = tmp_path_factory.mktemp("service_warp")
+    (d / "extracted.inc").write_text(_extract(os.path.join(CSRC, "lbm_pair.cuh"), "struct PairShared",
+                                              "__device__ __forceinline__ bool pair_ready",
+                                              "__device__ __forceinline__ void pair_serve"))
+    exe = str(d / "service_warp")
+    p = subprocess.run(["g++", "-std=c++20", "-O1", "-w", "-pthread", "-I" + CUDA + "/include", "-I" + str(d),
+                        os.path.join(MODEL, "service_warp.cpp"), "-o", exe], capture_output=True, text=True)
+    assert p.returncode == 0, p.stderr
+    return exe
+
+
+@pytest.mark.parametrize("ranges", [(1, 1, 1), (2, 0, 3), (12, 12, 12)])
+@pytest.mark.parametrize("polls", [0, 300])
+def test_the_odd_step_is_ordered_after_every_group_it_needs(service_warp, ranges, polls):
+    """The even tiles that any lane of the service warp polled are ordered
+    before the compute warps' odd step, ready at once or after waiting; fewer
+    and more groups than lanes."""
+    p = subprocess.run([service_warp, *map(str, ranges), str(polls)], capture_output=True, text=True, timeout=60)
+    assert p.returncode == 0, p.stdout + p.stderr
