@@ -1298,8 +1298,9 @@ __global__ void __launch_bounds__(kPairThreads, 3)
   }
   if (k < p.nTiles) {
     const int n = static_cast<int>(k) * kListTile + threadIdx.x;
-    pair_odd_named(&sh, a.err);  // the first tile's run record
+    const bool named = pair_named(&sh, a.err);  // the first tile's run record
     chain_wait();
+    if (!named) return;
     if (n < a.nFluid) {
       uint32_t off;
       const uint32_t* e = run_row(records, threadIdx.x, off);

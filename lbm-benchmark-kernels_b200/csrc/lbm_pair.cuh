@@ -195,14 +195,19 @@ __device__ __forceinline__ void pair_even_done(Sh* sh) {
   if ((threadIdx.x & 31) == 0) mbar_arrive(&sh->even);
 }
 
+// Compute warps: waits for the item and the run record of its first tile;
+// false if they did not come.
+template <class Sh>
+__device__ __forceinline__ bool pair_named(Sh* sh, int* err) {
+  if (mbar_wait_bounded(&sh->named, 0)) return true;
+  atomicOr(err, 1);
+  return false;
+}
+
 // Compute warps: waits for the item; false if it names no odd step.
 template <class Sh>
 __device__ __forceinline__ bool pair_odd_named(Sh* sh, int* err) {
-  if (!mbar_wait_bounded(&sh->named, 0)) {
-    atomicOr(err, 1);
-    return false;
-  }
-  return sh->item.tile != kPairNone;
+  return pair_named(sh, err) && sh->item.tile != kPairNone;
 }
 
 // Compute warps: waits for the odd step's turn; false if there is none.

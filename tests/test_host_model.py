@@ -73,19 +73,25 @@ def _extract(path, *starts):
     return "\n".join(out)
 
 
-@pytest.fixture(scope="module")
-def service_warp(tmp_path_factory):
+def _device_model(tmp_path_factory, name, source):
+    """Device code on the host: tests/host_model/NAME.cpp around `source`."""
     if not os.path.exists(os.path.join(CUDA, "include", "cuda_runtime.h")):
         pytest.skip("no CUDA headers")
-    d = tmp_path_factory.mktemp("service_warp")
-    (d / "extracted.inc").write_text(_extract(os.path.join(CSRC, "lbm_pair.cuh"), "struct PairShared",
-                                              "__device__ __forceinline__ bool pair_ready",
-                                              "__device__ __forceinline__ void pair_serve"))
-    exe = str(d / "service_warp")
+    d = tmp_path_factory.mktemp(name)
+    (d / "extracted.inc").write_text(source)
+    exe = str(d / name)
     p = subprocess.run(["g++", "-std=c++20", "-O1", "-w", "-pthread", "-I" + CUDA + "/include", "-I" + str(d),
-                        os.path.join(MODEL, "service_warp.cpp"), "-o", exe], capture_output=True, text=True)
+                        os.path.join(MODEL, name + ".cpp"), "-o", exe], capture_output=True, text=True)
     assert p.returncode == 0, p.stderr
     return exe
+
+
+@pytest.fixture(scope="module")
+def service_warp(tmp_path_factory):
+    return _device_model(tmp_path_factory, "service_warp",
+                         _extract(os.path.join(CSRC, "lbm_pair.cuh"), "struct PairShared",
+                                  "__device__ __forceinline__ bool pair_ready",
+                                  "__device__ __forceinline__ void pair_serve"))
 
 
 @pytest.mark.parametrize("ranges", [(1, 1, 1), (2, 0, 3), (12, 12, 12)])
@@ -95,4 +101,19 @@ def test_the_odd_step_is_ordered_after_every_group_it_needs(service_warp, ranges
     before the compute warps' odd step, ready at once or after waiting; fewer
     and more groups than lanes."""
     p = subprocess.run([service_warp, *map(str, ranges), str(polls)], capture_output=True, text=True, timeout=60)
+    assert p.returncode == 0, p.stdout + p.stderr
+
+
+@pytest.fixture(scope="module")
+def compute_warps(tmp_path_factory):
+    pair = open(os.path.join(CSRC, "lbm_pair.cuh")).read()
+    waits = pair[pair.index("// Compute warps: their even nodes"):pair.index("// Small domains:")]
+    return _device_model(tmp_path_factory, "compute_warps",
+                         waits + "\n" + _extract(os.path.join(CSRC, "lbm_kernels_fp64.cu"), "    k_list_two_fp64("))
+
+
+@pytest.mark.parametrize("push", [0, 1])
+@pytest.mark.parametrize("named,go", [(1, 1), (0, 1), (1, 0), (0, 0)])
+def test_no_run_record_is_followed_whose_wait_ran_out(compute_warps, push, named, go):
+    p = subprocess.run([compute_warps, str(push), str(named), str(go)], capture_output=True, text=True, timeout=60)
     assert p.returncode == 0, p.stdout + p.stderr
