@@ -504,6 +504,9 @@ int lbm_batch_reset(void *batch, int slot);
 /* Enqueues nsteps (rounded up to even) steps of every active domain; with
  * use_graph the sequence is replayed from a captured CUDA graph. */
 int lbm_batch_step(void *batch, int nsteps, int use_graph);
+/* Waits for the steps. -7: a wait inside one of them gave up, and the PDFs are
+ * no state of the update; lbm_batch_moments, lbm_batch_get_field and
+ * lbm_batch_checkpoint_save return that too. */
 int lbm_batch_sync(void *batch);
 /* FP64 {rho, jx, jy, jz} sums of every slot: out has maxDomains * 4 doubles. */
 int lbm_batch_moments(void *batch, double *out);

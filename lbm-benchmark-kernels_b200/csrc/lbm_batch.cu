@@ -81,6 +81,7 @@ struct Batch {
   lbm::PairItem* dItems = nullptr;   // capacity itemCap
   uint32_t* dCount = nullptr;        // capacity tileCap tiles
   uint32_t itemCap = 0, gridItems = 0;
+  int* errHost = nullptr;            // page-locked copy of the device error word
   std::map<int, cudaGraphExec_t> graphs;  // steps -> instantiated graph
   long long launches = 0;
   int numSMs = 148;
@@ -239,6 +240,17 @@ int enqueue(Batch* b, int nsteps) {
   return 0;
 }
 
+// Waits for the stream; -7 if a wait inside a step gave up before this (the
+// steps' blocks wait for one another), so that what was copied back on the
+// stream is no state of the update.
+int finish(Batch* b) {
+  BCK(cudaMemcpyAsync(b->errHost, b->dErr, sizeof(int), cudaMemcpyDeviceToHost, b->stream));
+  BCK(cudaStreamSynchronize(b->stream));
+  if (*b->errHost == 0) return 0;
+  g_batchError = "a device wait exceeded its limit";
+  return -7;
+}
+
 // Bound on a domain's device bytes: PDFs plus the adjacency (full rows
 // while the run-compressed form is built from them; the runs never exceed
 // the full rows plus a 48-byte header per tile).
@@ -320,6 +332,7 @@ void* lbm_batch_create(int storage, double budgetGB, int maxDomains) {
             lbm::dev_alloc(&b->dTileDom, sizeof(int) * b->maxTiles) == cudaSuccess &&
             lbm::dev_alloc(&b->dNTiles, sizeof(int)) == cudaSuccess &&
             lbm::dev_alloc(&b->dErr, sizeof(int)) == cudaSuccess &&
+            cudaMallocHost(reinterpret_cast<void**>(&b->errHost), sizeof(int)) == cudaSuccess &&
             lbm::dev_alloc(&b->dPair, sizeof(lbm::PairArgs<3>)) == cudaSuccess &&
             lbm::dev_alloc(&b->dPartials, sizeof(double) * 4 * (size_t)b->maxTiles) == cudaSuccess &&
             lbm::dev_alloc(&b->dDomTileStart, sizeof(int) * b->maxSlots) == cudaSuccess &&
@@ -355,6 +368,7 @@ void lbm_batch_destroy(void* h) {
   lbm::dev_free(b->dTiles);
   lbm::dev_free(b->dNTiles);
   lbm::dev_free(b->dErr);
+  cudaFreeHost(b->errHost);
   lbm::dev_free(b->dPartials);
   lbm::dev_free(b->dDomTileStart);
   lbm::dev_free(b->dDomTileCount);
@@ -507,15 +521,7 @@ int lbm_batch_step(void* h, int nsteps, int use_graph) {
 }
 
 int lbm_batch_sync(void* h) {
-  Batch* b = static_cast<Batch*>(h);
-  BCK(cudaStreamSynchronize(b->stream));
-  int err = 0;
-  BCK(cudaMemcpy(&err, b->dErr, sizeof(int), cudaMemcpyDeviceToHost));
-  if (err) {
-    g_batchError = "a device wait exceeded its limit";
-    return -7;
-  }
-  return 0;
+  return finish(static_cast<Batch*>(h));
 }
 
 // FP64 sums {rho, jx, jy, jz} of every slot into out (maxDomains x 4,
@@ -529,8 +535,7 @@ int lbm_batch_moments(void* h, double* out) {
                        b->stream);
   BCK(cudaGetLastError());
   BCK(cudaMemcpyAsync(out, b->dMoments, sizeof(double) * 4 * b->maxSlots, cudaMemcpyDeviceToHost, b->stream));
-  BCK(cudaStreamSynchronize(b->stream));
-  return 0;
+  return finish(b);
 }
 
 // Logical PDFs of a slot (cells x fastest, 19 per cell, obstacles untouched)
@@ -542,7 +547,8 @@ int lbm_batch_get_field(void* h, int slot, double* out) {
   const size_t nc = (size_t)d.dev.nCells;
   std::vector<unsigned char> raw(nc * Q * b->elemBytes);
   BCK(cudaMemcpyAsync(raw.data(), d.pdfs, raw.size(), cudaMemcpyDeviceToHost, b->stream));
-  BCK(cudaStreamSynchronize(b->stream));
+  const int rc = finish(b);
+  if (rc) return rc;
   const long ncell = (long)d.dims[0] * d.dims[1] * d.dims[2];
   for (long c = 0; c < ncell; ++c) {
     const uint32_t n = d.grid[c];
@@ -672,7 +678,8 @@ int lbm_batch_checkpoint_save(void* h, int slot, const char* path) {
   DomainSlot& d = b->slots[slot];
   std::vector<unsigned char> raw((size_t)d.dev.nCells * Q * b->elemBytes);
   BCK(cudaMemcpyAsync(raw.data(), d.pdfs, raw.size(), cudaMemcpyDeviceToHost, b->stream));
-  BCK(cudaStreamSynchronize(b->stream));
+  const int rc = finish(b);
+  if (rc) return rc;
   DomCkpt c = dom_header_of(b, d);
   c.checksum = dom_fnv1a64(raw.data(), raw.size());
   FILE* fh = std::fopen(path, "wb");

@@ -459,7 +459,8 @@ class Batch:
         lat = self.lattices[slot]
         out = np.full(lat.mask.size * Q, np.nan)
         rc = self.L.lbm_batch_get_field(self.h, slot, out.ctypes.data_as(ctypes.POINTER(ctypes.c_double)))
-        assert rc == 0
+        if rc:
+            raise RuntimeError("batch get_field failed (%d): %s" % (rc, self.L.lbm_batch_last_error().decode()))
         return out.reshape(-1, Q)
 
     def set_field(self, slot, pdfs):

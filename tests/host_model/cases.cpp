@@ -8,10 +8,12 @@
 #include "../../include/lbm_b200.h"
 #include "../../lbm-benchmark-kernels_b200/csrc/lbm_batch.cuh"
 #include "../../lbm-benchmark-kernels_b200/csrc/lbm_kernels.cuh"
+#include "../../lbm-benchmark-kernels_b200/csrc/lbm_mem.cuh"
 
 namespace {
 
 int g_bad = 0;
+bool g_waitRunsOut = false;  // the next steps set the error word
 void check(bool ok, const char* what) {
   if (ok) return;
   std::printf("not so: %s\n", what);
@@ -95,6 +97,54 @@ void aa_odd_interior_fp64(const AaArgs&, const Trt<double>&, const int* items, i
   });
 }
 
+// The list layout of a lattice of fluid cells, and the tables of a batch.
+long long list_build_device(const int*, const int dims[3], const int*, int, const int*, int, uint32_t* grid, uint32_t*,
+                            long long, cudaStream_t s, const char**) {
+  const int n = dims[0] * dims[1] * dims[2];
+  fake::launch(s, [=] {
+    for (int k = 0; k < n; ++k) grid[k] = (uint32_t)k;
+  });
+  return n;
+}
+int list_runs_device(const uint32_t*, int nFluid, cudaStream_t s, uint32_t** runs, uint32_t** runOff, size_t* runBytes) {
+  cudaStreamSynchronize(s);
+  const int tiles = (nFluid + kListTile - 1) / kListTile;
+  *runBytes = 64 * (size_t)tiles;
+  const cudaError_t e = dev_alloc(runs, *runBytes);
+  if (e != cudaSuccess) return (int)e;
+  return (int)dev_alloc(runOff, sizeof(uint32_t) * (tiles + 1));
+}
+void list_tile_reach(const uint32_t*, int nFluid, long long, uint32_t* reach, cudaStream_t s) {
+  fake::launch(s, [=] {
+    for (int t = 0; t < (nFluid + kListTile - 1) / kListTile; ++t)
+      for (int c = 0; c < 6; ++c) reach[6 * t + c] = (uint32_t)t;
+  });
+}
+void batch_pad_adjacency(uint32_t*, int, long long, cudaStream_t) {}
+void batch_build_tiles(const BatchDomain*, const int*, int nTiles, BatchTile* out, cudaStream_t s) {
+  fake::launch(s, [=] { std::memset((void*)out, 0, sizeof(BatchTile) * nTiles); });
+}
+uint32_t batch_odd_order(const uint32_t*, int nTiles, std::vector<BatchOdd>& odd) {
+  odd.resize(nTiles);
+  return 0;
+}
+void batch_build_items(const BatchDomain*, const int*, int nTiles, uint32_t lead, PairItem* items, cudaStream_t s) {
+  fake::launch(s, [=] { std::memset((void*)items, 0, sizeof(PairItem) * (nTiles + lead)); });
+}
+int batch_pair_resident(int) { return 16; }
+void batch_even_lp(const BatchArgs& a, const BatchLaunch&, int, cudaStream_t s) {
+  fake::launch(s, [=] {
+    if (g_waitRunsOut) *a.err |= 1;
+    for (int t = 0; t < *a.nTiles; ++t) check(a.tiles[t].nCells == 0, "the step reads its tile records");
+  });
+}
+void batch_odd_lp(const BatchArgs& a, const BatchLaunch& l, int grid, cudaStream_t s) { batch_even_lp(a, l, grid, s); }
+void batch_moments(const BatchArgs&, int, double*, const int*, const int*, int slots, double* out, cudaStream_t s) {
+  fake::launch(s, [=] {
+    for (int k = 0; k < 4 * slots; ++k) out[k] = 1.0;
+  });
+}
+
 }  // namespace lbm
 
 namespace {
@@ -151,12 +201,36 @@ void deinit_from_another_device() {
   fake::run_device(0);  // what the free did not wait for uses the memory now
 }
 
+// A wait inside a step runs out: what is read back afterwards says so.
+void batch_results_of_a_lost_state() {
+  Lattice lat(6, 5, 4);
+  void* b = lbm_batch_create(1, 1.0, 4);
+  const int slot = lbm_batch_add(b, &lat.ld, 1.2, 0.1875, 1e-5);
+  check(slot == 0, "the domain is admitted");
+  std::vector<double> sums(16), field(19 * 6 * 5 * 4);
+  const char* path = "/dev/null";
+  for (int graph = 0; graph < 2; ++graph) {
+    check(lbm_batch_step(b, 2, graph) == 0, "the steps are accepted");
+    check(lbm_batch_moments(b, sums.data()) == 0 && sums[0] == 1.0, "the sums of a good state");
+    check(lbm_batch_get_field(b, slot, field.data()) == 0, "the field of a good state");
+    check(lbm_batch_checkpoint_save(b, slot, path) == 0, "the checkpoint of a good state");
+  }
+  g_waitRunsOut = true;
+  check(lbm_batch_step(b, 2, 1) == 0, "the steps are accepted");
+  check(lbm_batch_moments(b, sums.data()) == -7, "no sums of a lost state");
+  check(lbm_batch_get_field(b, slot, field.data()) == -7, "no field of a lost state");
+  check(lbm_batch_checkpoint_save(b, slot, path) == -7, "no checkpoint of a lost state");
+  check(lbm_batch_sync(b) == -7, "sync reports it too");
+  lbm_batch_destroy(b);
+}
+
 const std::map<std::string, std::function<void()>> kCases = {
     {"first_odd_part", [] { first_slab_step(0); }},
     {"first_odd_half", [] { first_slab_step(1); }},
     {"first_even_half", [] { first_slab_step(2); }},
     {"first_slab_step_captured", first_slab_step_captured},
     {"deinit_from_another_device", deinit_from_another_device},
+    {"batch_results_of_a_lost_state", batch_results_of_a_lost_state},
 };
 
 }  // namespace

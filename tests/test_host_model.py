@@ -55,6 +55,11 @@ def test_deinit_waits_for_the_instances_own_device(cases):
     _run(cases, "deinit_from_another_device")
 
 
+def test_batch_results_of_a_lost_state_are_refused(cases):
+    """Sums, fields and checkpoints read after a step whose wait ran out."""
+    _run(cases, "batch_results_of_a_lost_state")
+
+
 def _extract(path, *starts):
     """The definitions of a source file that begin with the given lines."""
     text = open(path).read()
