@@ -28,6 +28,7 @@ const char* g_batchError = "";
     cudaError_t e_ = (call);                                               \
     if (e_ != cudaSuccess) {                                               \
       g_batchError = cudaGetErrorString(e_);                               \
+      cudaGetLastError(); /* reported here, not by the next launch check */ \
       std::fprintf(stderr, "lbm batch: %s: %s\n", #call, g_batchError);   \
       return -(int)e_ - 1000;                                              \
     }                                                                      \
@@ -79,7 +80,7 @@ struct Batch {
   lbm::PairArgs<3> pair{};           // fused pairs (nItems 0: none), as uploaded to dPair
   lbm::PairArgs<3>* dPair = nullptr;
   lbm::PairItem* dItems = nullptr;   // capacity itemCap
-  uint32_t* dCount = nullptr;        // capacity tileCap tiles
+  uint32_t* dCount = nullptr;        // as many groups as itemCap items can have
   uint32_t itemCap = 0, gridItems = 0;
   int* errHost = nullptr;            // page-locked copy of the device error word
   std::map<int, cudaGraphExec_t> graphs;  // steps -> instantiated graph
@@ -105,6 +106,27 @@ void drop_graphs(Batch* b) {
   b->graphs.clear();
 }
 
+// Tables of fused pairs of nItems items. False without memory for them, which is
+// no reason to refuse a domain: the steps are launches of their own then.
+bool reserve_pairs(Batch* b, uint32_t nItems) {
+  if (nItems <= b->itemCap) return true;
+  lbm::dev_free(b->dItems);  // the caller has waited for the steps
+  lbm::dev_free(b->dCount);
+  b->dItems = nullptr;
+  b->dCount = nullptr;
+  b->itemCap = 0;
+  const uint32_t cap = nItems + nItems / 2;
+  if (lbm::dev_alloc(&b->dItems, sizeof(lbm::PairItem) * (size_t)cap) != cudaSuccess ||
+      lbm::dev_alloc(&b->dCount, sizeof(uint32_t) * ((size_t)cap / 8 + 4)) != cudaSuccess) {  // groups of 8 or more
+    cudaGetLastError();
+    lbm::dev_free(b->dItems);
+    b->dItems = nullptr;
+    return false;
+  }
+  b->itemCap = cap;
+  return true;
+}
+
 // Fused pairs (two steps in one launch) for the tables just published, where
 // they are the faster way.
 //
@@ -125,20 +147,12 @@ int publish_pairs(Batch* b, uint32_t ahead) {
   int dev = 0, l2 = 0;
   BCK(cudaGetDevice(&dev));
   BCK(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev));
+  const uint32_t nItems = n + lead;
   const bool fused = (double)n * lbm::kBatchTileNodes * Q * b->elemBytes > 0.5 * l2 &&
-                     (double)lead * lbm::kBatchTileNodes * Q * b->elemBytes <= 0.4 * l2;
+                     (double)lead * lbm::kBatchTileNodes * Q * b->elemBytes <= 0.4 * l2 && reserve_pairs(b, nItems);
   if (fused != (b->pair.nItems > 0)) drop_graphs(b);
   b->pair.nItems = 0;
   if (!fused) return 0;
-  const uint32_t nItems = n + lead;
-  if (nItems > b->itemCap) {
-    BCK(cudaStreamSynchronize(b->stream));
-    lbm::dev_free(b->dItems);
-    b->dItems = nullptr;
-    b->itemCap = 0;
-    BCK(lbm::dev_alloc(&b->dItems, sizeof(lbm::PairItem) * (size_t)(nItems + nItems / 2)));
-    b->itemCap = nItems + nItems / 2;
-  }
   if (nItems > b->gridItems || nItems < b->gridItems / 2) {
     drop_graphs(b);
     b->gridItems = nItems + nItems / 8;
@@ -161,40 +175,44 @@ int publish_pairs(Batch* b, uint32_t ahead) {
 
 // Rebuilds the tile table, the per-domain tile ranges and the tile records
 // after a change of membership (stream-ordered uploads, then a device pass
-// that fills the records).
+// that fills the records). What can fail for want of memory comes first and
+// leaves the tables published before as they are.
 int publish(Batch* b) {
-  b->tileDomHost.clear();
   std::vector<int> start(b->maxSlots, 0), count(b->maxSlots, 0);
   uint32_t ahead = 0;
+  int n = 0;
+  for (int s = 0; s < b->maxSlots; ++s) {
+    const DomainSlot& d = b->slots[s];
+    if (!d.active) continue;
+    start[s] = n;
+    count[s] = d.nTiles;
+    ahead = std::max(ahead, d.ahead);
+    n += d.nTiles;
+  }
+  if (n > b->maxTiles) return -3;
+  BCK(cudaStreamSynchronize(b->stream));
+  if (n > b->tileCap) {
+    const int cap = std::min(b->maxTiles, std::max(n + n / 2, 1024));
+    lbm::BatchTile* tiles = nullptr;
+    BCK(lbm::dev_alloc(&tiles, sizeof(lbm::BatchTile) * (size_t)cap));
+    // graphs captured with the old records go
+    drop_graphs(b);
+    lbm::dev_free(b->dTiles);
+    b->dTiles = tiles;
+    b->tileCap = cap;
+  }
+  b->nTiles = n;
+  b->tileDomHost.clear();
   for (int s = 0; s < b->maxSlots; ++s) {
     DomainSlot& d = b->slots[s];
     if (!d.active) continue;
-    d.dev.tileStart = (int)b->tileDomHost.size();
-    start[s] = d.dev.tileStart;
-    count[s] = d.nTiles;
-    ahead = std::max(ahead, d.ahead);
-    for (int t = 0; t < d.nTiles; ++t) b->tileDomHost.push_back(s);
+    d.dev.tileStart = start[s];
+    b->tileDomHost.insert(b->tileDomHost.end(), d.nTiles, s);
     BCK(cudaMemcpyAsync(b->dDoms + s, &d.dev, sizeof(lbm::BatchDomain), cudaMemcpyHostToDevice, b->stream));
   }
-  b->nTiles = (int)b->tileDomHost.size();
-  if (b->nTiles > b->maxTiles) return -3;
   if (b->nTiles)
     BCK(cudaMemcpyAsync(b->dTileDom, b->tileDomHost.data(), sizeof(int) * b->nTiles, cudaMemcpyHostToDevice,
                         b->stream));
-  if (b->nTiles > b->tileCap) {
-    // records are reallocated: graphs captured with the old table go
-    BCK(cudaStreamSynchronize(b->stream));
-    drop_graphs(b);
-    lbm::dev_free(b->dTiles);
-    lbm::dev_free(b->dCount);
-    b->dTiles = nullptr;
-    b->dCount = nullptr;
-    b->tileCap = 0;
-    const int cap = std::min(b->maxTiles, std::max(b->nTiles + b->nTiles / 2, 1024));
-    BCK(lbm::dev_alloc(&b->dTiles, sizeof(lbm::BatchTile) * (size_t)cap));
-    BCK(lbm::dev_alloc(&b->dCount, sizeof(uint32_t) * ((size_t)cap / 8 + 4)));  // groups of 8 tiles or more
-    b->tileCap = cap;
-  }
   // the grid of one-block-per-tile launches keeps some headroom, so that
   // graphs survive admissions; it is resized (and graphs dropped) when the
   // table outgrows it or shrinks below half of it
@@ -215,6 +233,14 @@ int publish(Batch* b) {
   // the host vectors above are read by the copies: wait before they go away
   BCK(cudaStreamSynchronize(b->stream));
   return 0;
+}
+
+void free_domain(DomainSlot& d) {
+  lbm::dev_free(d.pdfs);
+  lbm::dev_free(d.runs);
+  lbm::dev_free(d.runOff);
+  lbm::dev_free(d.odd);
+  d = DomainSlot();
 }
 
 bool fused(const Batch* b) { return b->pair.nItems > 0 && !b->separate; }
@@ -266,6 +292,75 @@ lbm::TrtW trt_of(double omega, double lambda, double xforce) {
   t.fx1 = (float)(3.0 * (1.0 / 18.0) * xforce);
   t.fx2 = (float)(3.0 * (1.0 / 36.0) * xforce);
   return t;
+}
+
+// The device arrays of a domain of lattice `ld`, into slot d (on failure the
+// caller frees what is there).
+int build_domain(Batch* b, const LatticeDesc* ld, long long nCells, DomainSlot& d) {
+  // what is needed while building; goes when the stream has finished with it
+  struct Scratch {
+    cudaStream_t s;
+    uint32_t *adj = nullptr, *grid = nullptr, *reach = nullptr;
+    int* mask = nullptr;
+    ~Scratch() {
+      cudaStreamSynchronize(s);
+      lbm::dev_free(adj);
+      lbm::dev_free(grid);
+      lbm::dev_free(reach);
+      lbm::dev_free(mask);
+    }
+  };
+  const int nFluid = ld->nFluid, nTiles = (int)(nCells / lbm::kBatchTileNodes);
+  const long ncell = (long)ld->Dims[0] * ld->Dims[1] * ld->Dims[2];
+  std::vector<uint32_t> reach;
+  std::vector<lbm::BatchOdd> odd;
+  d = DomainSlot();
+  d.grid.resize(ncell);
+  Scratch tmp{b->stream};
+  BCK(lbm::dev_alloc(&d.pdfs, (size_t)nCells * Q * b->elemBytes));
+  // numbering and adjacency built on the device (lbm_build.cu); padding
+  // nodes then point at their own slots so that every entry is in range;
+  // the steps read the run-compressed form, built from it
+  BCK(lbm::dev_alloc(&tmp.adj, (size_t)nCells * QM * 4));
+  BCK(lbm::dev_alloc(&tmp.mask, sizeof(int) * ncell));
+  BCK(lbm::dev_alloc(&tmp.grid, sizeof(uint32_t) * ncell));
+  BCK(cudaMemcpyAsync(tmp.mask, ld->Lattice, sizeof(int) * ncell, cudaMemcpyHostToDevice, b->stream));
+  const int blk[3] = {0, 0, 0}, per[3] = {ld->PeriodicX, ld->PeriodicY, ld->PeriodicZ};
+  const char* berr = "";
+  const long long nf = lbm::list_build_device(tmp.mask, ld->Dims, per, 0, blk, (int)nCells, tmp.grid, tmp.adj, nCells,
+                                              b->stream, &berr);
+  if (nf != nFluid) {
+    g_batchError = nf < 0 ? berr : "the mask's fluid cell count differs from the lattice's";
+    cudaGetLastError();
+    return -6;
+  }
+  lbm::batch_pad_adjacency(tmp.adj, nFluid, nCells, b->stream);
+  BCK(cudaMemcpyAsync(d.grid.data(), tmp.grid, sizeof(uint32_t) * ncell, cudaMemcpyDeviceToHost, b->stream));
+  for (int t = 0; t < 3 * nTiles; ++t) reach.insert(reach.end(), {1u, 0u});  // no node: reaches nothing
+  if (nFluid > 0) {
+    BCK(lbm::dev_alloc(&tmp.reach, sizeof(uint32_t) * reach.size()));
+    lbm::list_tile_reach(tmp.adj, nFluid, nCells, tmp.reach, b->stream);
+    BCK(cudaMemcpyAsync(reach.data(), tmp.reach, sizeof(uint32_t) * reach.size(), cudaMemcpyDeviceToHost, b->stream));
+  }
+  size_t runBytes = 0;
+  if (lbm::list_runs_device(tmp.adj, (int)nCells, b->stream, &d.runs, &d.runOff, &runBytes)) {
+    g_batchError = "building the run-compressed adjacency failed";
+    cudaGetLastError();
+    return -6;
+  }
+  BCK(cudaStreamSynchronize(b->stream));
+  d.ahead = lbm::batch_odd_order(reach.data(), nTiles, odd);
+  BCK(lbm::dev_alloc(&d.odd, sizeof(lbm::BatchOdd) * odd.size()));
+  BCK(cudaMemcpyAsync(d.odd, odd.data(), sizeof(lbm::BatchOdd) * odd.size(), cudaMemcpyHostToDevice, b->stream));
+  d.nTiles = nTiles;
+  for (int i = 0; i < 3; ++i) d.dims[i] = ld->Dims[i];
+  d.dev.f = d.pdfs;
+  d.dev.runs = d.runs;
+  d.dev.runOff = d.runOff;
+  d.dev.nCells = nCells;
+  d.dev.nFluid = nFluid;
+  d.dev.odd = d.odd;
+  return 0;
 }
 
 // Domain checkpoint: header (host byte order), then the slot's PDF array as
@@ -354,12 +449,7 @@ void lbm_batch_destroy(void* h) {
   if (!b) return;
   cudaStreamSynchronize(b->stream);
   drop_graphs(b);
-  for (auto& s : b->slots) {
-    lbm::dev_free(s.pdfs);
-    lbm::dev_free(s.runs);
-    lbm::dev_free(s.runOff);
-    lbm::dev_free(s.odd);
-  }
+  for (auto& s : b->slots) free_domain(s);
   lbm::dev_free(b->dPair);
   lbm::dev_free(b->dItems);
   lbm::dev_free(b->dCount);
@@ -395,91 +485,31 @@ int lbm_batch_add(void* h, const LatticeDesc* ld, double omega, double lambda, d
   if ((uint64_t)nCells * Q >= (1ull << 32)) return -5;
 
   DomainSlot& d = b->slots[slot];
-  d = DomainSlot();
-  const long ncell = (long)ld->Dims[0] * ld->Dims[1] * ld->Dims[2];
-  d.grid.resize(ncell);
-  BCK(lbm::dev_alloc(&d.pdfs, (size_t)nCells * Q * b->elemBytes));
-  uint32_t* adj = nullptr;
-  BCK(lbm::dev_alloc(&adj, (size_t)nCells * QM * 4));
-  // numbering and adjacency built on the device (lbm_build.cu); padding
-  // nodes then point at their own slots so that every entry is in range;
-  // the steps read the run-compressed form, built from it
-  int* dMask = nullptr;
-  uint32_t* dGrid = nullptr;
-  BCK(lbm::dev_alloc(&dMask, sizeof(int) * ncell));
-  BCK(lbm::dev_alloc(&dGrid, sizeof(uint32_t) * ncell));
-  BCK(cudaMemcpyAsync(dMask, ld->Lattice, sizeof(int) * ncell, cudaMemcpyHostToDevice, b->stream));
-  const int blk[3] = {0, 0, 0}, per[3] = {ld->PeriodicX, ld->PeriodicY, ld->PeriodicZ};
-  const char* berr = "";
-  const long long nf = lbm::list_build_device(dMask, ld->Dims, per, 0, blk, (int)nCells, dGrid, adj, nCells,
-                                              b->stream, &berr);
-  if (nf == nFluid) {
-    lbm::batch_pad_adjacency(adj, nFluid, nCells, b->stream);
-    BCK(cudaMemcpyAsync(d.grid.data(), dGrid, sizeof(uint32_t) * ncell, cudaMemcpyDeviceToHost, b->stream));
+  int rc = build_domain(b, ld, nCells, d);
+  if (rc == 0) {
+    d.active = true;
+    d.bytes = bytes;
+    d.omega = omega;
+    d.lambda = lambda;
+    d.xforce = xforce;
+    d.dev.trt = trt_of(omega, lambda, xforce);
+    b->used += bytes;
+    rc = lbm_batch_reset(h, slot);
+    if (rc == 0) rc = publish(b);
+    if (rc == 0) return slot;
+    b->used -= bytes;
   }
-  const cudaError_t built = cudaStreamSynchronize(b->stream);
-  lbm::dev_free(dGrid);
-  lbm::dev_free(dMask);
-  BCK(built);
-  int rrc = 0;
-  size_t runBytes = 0;
-  const int nTiles = (int)(nCells / lbm::kBatchTileNodes);
-  std::vector<uint32_t> reach;
-  uint32_t* dReach = nullptr;
-  if (nf == nFluid) {
-    for (int t = 0; t < 3 * nTiles; ++t) reach.insert(reach.end(), {1u, 0u});  // no node: reaches nothing
-    if (nFluid > 0) {
-      BCK(lbm::dev_alloc(&dReach, sizeof(uint32_t) * reach.size()));
-      lbm::list_tile_reach(adj, nFluid, nCells, dReach, b->stream);
-      BCK(cudaMemcpyAsync(reach.data(), dReach, sizeof(uint32_t) * reach.size(), cudaMemcpyDeviceToHost, b->stream));
-    }
-  }
-  if (nf == nFluid) rrc = lbm::list_runs_device(adj, (int)nCells, b->stream, &d.runs, &d.runOff, &runBytes);
-  lbm::dev_free(adj);
-  lbm::dev_free(dReach);
-  if (nf != nFluid || rrc) {
-    g_batchError = rrc ? "building the run-compressed adjacency failed"
-                       : (nf < 0 ? berr : "the mask's fluid cell count differs from the lattice's");
-    lbm::dev_free(d.pdfs);
-    d = DomainSlot();
-    return -6;
-  }
-  std::vector<lbm::BatchOdd> odd;
-  d.ahead = lbm::batch_odd_order(reach.data(), nTiles, odd);
-  BCK(lbm::dev_alloc(&d.odd, sizeof(lbm::BatchOdd) * odd.size()));
-  BCK(cudaMemcpyAsync(d.odd, odd.data(), sizeof(lbm::BatchOdd) * odd.size(), cudaMemcpyHostToDevice, b->stream));
-  d.active = true;
-  d.bytes = bytes;
-  d.nTiles = nTiles;
-  for (int i = 0; i < 3; ++i) d.dims[i] = ld->Dims[i];
-  d.omega = omega;
-  d.lambda = lambda;
-  d.xforce = xforce;
-  d.dev.f = d.pdfs;
-  d.dev.runs = d.runs;
-  d.dev.runOff = d.runOff;
-  d.dev.nCells = nCells;
-  d.dev.nFluid = nFluid;
-  d.dev.trt = trt_of(omega, lambda, xforce);
-  d.dev.odd = d.odd;
-  b->used += bytes;
-  int rc = lbm_batch_reset(h, slot);
-  if (rc) return rc;
-  rc = publish(b);  // synchronises: the host adjacency may go
-  return rc ? rc : slot;
+  cudaStreamSynchronize(b->stream);
+  free_domain(d);
+  return rc;
 }
 
 int lbm_batch_remove(void* h, int slot) {
   Batch* b = static_cast<Batch*>(h);
   if (slot < 0 || slot >= b->maxSlots || !b->slots[slot].active) return -1;
   BCK(cudaStreamSynchronize(b->stream));
-  DomainSlot& d = b->slots[slot];
-  lbm::dev_free(d.pdfs);
-  lbm::dev_free(d.runs);
-  lbm::dev_free(d.runOff);
-  lbm::dev_free(d.odd);
-  b->used -= d.bytes;
-  d = DomainSlot();
+  b->used -= b->slots[slot].bytes;
+  free_domain(b->slots[slot]);
   return publish(b);
 }
 

@@ -13,6 +13,7 @@
 namespace {
 
 int g_bad = 0;
+int g_pairs = 0;             // fused launches of batches that have run
 bool g_waitRunsOut = false;  // the next steps set the error word
 void check(bool ok, const char* what) {
   if (ok) return;
@@ -138,6 +139,16 @@ void batch_even_lp(const BatchArgs& a, const BatchLaunch&, int, cudaStream_t s) 
     for (int t = 0; t < *a.nTiles; ++t) check(a.tiles[t].nCells == 0, "the step reads its tile records");
   });
 }
+void batch_pair_lp(const BatchPairArgs& a, int grid, cudaStream_t s) {
+  fake::launch(s, [=] {
+    const PairArgs<3> p = *a.pair;
+    check((uint32_t)grid >= p.nItems, "the grid covers the items");
+    for (uint32_t k = 0; k < p.nItems; ++k) check(p.items[k].tile == 0, "the pair reads its items");
+    for (uint32_t k = 0; k < p.nTiles; ++k) check(a.tiles[k].nCells == 0, "the pair reads its tile records");
+    for (uint32_t k = 0; k < ((p.nTiles - 1) >> p.shift) + 3; ++k) check(p.count[k] == 0, "the counters start at zero");
+    ++g_pairs;
+  });
+}
 void batch_odd_lp(const BatchArgs& a, const BatchLaunch& l, int grid, cudaStream_t s) { batch_even_lp(a, l, grid, s); }
 void batch_moments(const BatchArgs&, int, double*, const int*, const int*, int slots, double* out, cudaStream_t s) {
   fake::launch(s, [=] {
@@ -224,6 +235,41 @@ void batch_results_of_a_lost_state() {
   lbm_batch_destroy(b);
 }
 
+// A domain is admitted to a running batch, or leaves it, with memory for k more
+// allocations. The others go on, and nothing of a refused one stays.
+void batch_without_memory() {
+  Lattice first(32, 32, 32), next(72, 71, 70);
+  auto steps = [](void* b, const char* what) {
+    for (int graph = 0; graph < 2; ++graph)
+      check(lbm_batch_step(b, 2, graph) == 0 && lbm_batch_sync(b) == 0, what);
+  };
+  for (int k = 0; k == 0 || fake::failed; ++k) {
+    void* b = lbm_batch_create(1, 1.0, 4);
+    check(lbm_batch_add(b, &first.ld, 1.2, 0.1875, 1e-5) == 0, "the first domain is admitted");
+    g_pairs = 0;
+    steps(b, "it steps");
+    check(g_pairs == 2, "in fused pairs");
+    const size_t used = lbm_batch_bytes_used(b), blocks = fake::blocks.size();
+    fake::failed = false;
+    fake::failAfter = k;
+    const int slot = lbm_batch_add(b, &next.ld, 1.2, 0.1875, 1e-5);
+    fake::failAfter = -1;
+    if (slot < 0) {
+      check(lbm_batch_active_domains(b) == 1 && lbm_batch_bytes_used(b) == used, "the refused domain does not count");
+      check(fake::blocks.size() <= blocks, "its memory is given back");
+      steps(b, "the steps go on");
+      check(lbm_batch_add(b, &next.ld, 1.2, 0.1875, 1e-5) == 1, "it is admitted later");
+    }
+    steps(b, "the steps go on with it");
+    fake::failAfter = 0;
+    check(lbm_batch_remove(b, 0) == 0, "a domain may leave without memory");
+    fake::failAfter = -1;
+    steps(b, "the steps go on without it");
+    lbm_batch_destroy(b);
+    check(fake::blocks.empty(), "the batch's memory is given back");
+  }
+}
+
 const std::map<std::string, std::function<void()>> kCases = {
     {"first_odd_part", [] { first_slab_step(0); }},
     {"first_odd_half", [] { first_slab_step(1); }},
@@ -231,6 +277,7 @@ const std::map<std::string, std::function<void()>> kCases = {
     {"first_slab_step_captured", first_slab_step_captured},
     {"deinit_from_another_device", deinit_from_another_device},
     {"batch_results_of_a_lost_state", batch_results_of_a_lost_state},
+    {"batch_without_memory", batch_without_memory},
 };
 
 }  // namespace

@@ -44,7 +44,9 @@ struct Block {
 inline int device = 0;
 inline std::set<cudaStream_t> streams;
 inline std::map<void*, Block> blocks;
-inline int failAlloc = -1;  // the allocation that fails, counted down; -1: none
+inline int failAfter = -1;  // device allocations that succeed before all fail; -1: all succeed
+inline bool failed = false; // one has failed
+inline cudaError_t last = cudaSuccess;
 inline bool staged = true;  // copies from the host read their source at the call; false: when the stream runs
 inline int calls = 0;       // copies, clears, waits and allocations so far
 
@@ -76,7 +78,11 @@ inline void enqueue(cudaStream_t s, std::function<void()> op) {
 inline cudaError_t allocate(void** p, size_t bytes, bool pool) {
   *p = nullptr;
   ++calls;
-  if (failAlloc >= 0 && failAlloc-- == 0) return cudaErrorMemoryAllocation;
+  if (failAfter == 0) {
+    failed = true;
+    return last = cudaErrorMemoryAllocation;
+  }
+  if (failAfter > 0) --failAfter;
   if (bytes == 0) return cudaSuccess;
   *p = std::malloc(bytes);
   std::memset(*p, 0xCD, bytes);
@@ -89,7 +95,11 @@ inline cudaError_t allocate(void** p, size_t bytes, bool pool) {
 extern "C" {
 cudaError_t cudaGetDevice(int* d) { *d = fake::device; return cudaSuccess; }
 cudaError_t cudaSetDevice(int d) { fake::device = d; return cudaSuccess; }
-cudaError_t cudaGetLastError() { return cudaSuccess; }
+cudaError_t cudaGetLastError() {
+  const cudaError_t e = fake::last;
+  fake::last = cudaSuccess;
+  return e;
+}
 const char* cudaGetErrorString(cudaError_t e) { return e == cudaErrorMemoryAllocation ? "out of memory" : "error"; }
 cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr a, int) {
   *v = a == cudaDevAttrL2CacheSize ? 4 << 20 : a == cudaDevAttrMultiProcessorCount ? 148 : 1;

@@ -60,6 +60,12 @@ def test_batch_results_of_a_lost_state_are_refused(cases):
     _run(cases, "batch_results_of_a_lost_state")
 
 
+def test_batch_goes_on_when_memory_runs_out(cases):
+    """Every allocation of an admission may fail, those of the fused steps'
+    tables among them: no step uses tables that were given back."""
+    _run(cases, "batch_without_memory")
+
+
 def _extract(path, *starts):
     """The definitions of a source file that begin with the given lines."""
     text = open(path).read()
