@@ -531,6 +531,7 @@ int lbm_batch_step(void* h, int nsteps, int use_graph) {
   Batch* b = static_cast<Batch*>(h);
   nsteps += nsteps & 1;
   if (nsteps <= 0) return 0;
+  if (b->nTiles == 0) return 0;  // nothing to capture that would hold for later domains
   if (!use_graph) return enqueue(b, nsteps);
   auto it = b->graphs.find(nsteps);
   if (it == b->graphs.end()) {

@@ -13,6 +13,7 @@
 namespace {
 
 int g_bad = 0;
+int g_steps = 0;             // launches of one step of batches that have run
 int g_pairs = 0;             // fused launches of batches that have run
 bool g_waitRunsOut = false;  // the next steps set the error word
 void check(bool ok, const char* what) {
@@ -136,6 +137,7 @@ int batch_pair_resident(int) { return 16; }
 void batch_even_lp(const BatchArgs& a, const BatchLaunch&, int, cudaStream_t s) {
   fake::launch(s, [=] {
     if (g_waitRunsOut) *a.err |= 1;
+    g_steps += *a.nTiles > 0;
     for (int t = 0; t < *a.nTiles; ++t) check(a.tiles[t].nCells == 0, "the step reads its tile records");
   });
 }
@@ -270,6 +272,25 @@ void batch_without_memory() {
   }
 }
 
+// Steps of an empty batch do nothing; those of the domain that comes next do.
+void batch_steps_while_empty() {
+  Lattice lat(6, 5, 4);
+  void* b = lbm_batch_create(1, 1.0, 4);
+  for (int round = 0; round < 2; ++round) {
+    check(lbm_batch_step(b, 2, 1) == 0 && lbm_batch_sync(b) == 0, "an empty batch steps");
+    check(lbm_batch_add(b, &lat.ld, 1.2, 0.1875, 1e-5) == 0, "the domain is admitted");
+    g_steps = 0;
+    check(lbm_batch_step(b, 2, 1) == 0 && lbm_batch_sync(b) == 0 && g_steps == 2, "the domain steps");
+    check(lbm_batch_remove(b, 0) == 0, "the domain leaves");
+    check(lbm_batch_step(b, 4, 1) == 0 && lbm_batch_sync(b) == 0, "an empty batch steps");
+    check(lbm_batch_add(b, &lat.ld, 1.2, 0.1875, 1e-5) == 0, "the domain is admitted");
+    g_steps = 0;
+    check(lbm_batch_step(b, 4, 1) == 0 && lbm_batch_sync(b) == 0 && g_steps == 4, "the domain steps");
+    check(lbm_batch_remove(b, 0) == 0, "the domain leaves");
+  }
+  lbm_batch_destroy(b);
+}
+
 const std::map<std::string, std::function<void()>> kCases = {
     {"first_odd_part", [] { first_slab_step(0); }},
     {"first_odd_half", [] { first_slab_step(1); }},
@@ -278,6 +299,7 @@ const std::map<std::string, std::function<void()>> kCases = {
     {"deinit_from_another_device", deinit_from_another_device},
     {"batch_results_of_a_lost_state", batch_results_of_a_lost_state},
     {"batch_without_memory", batch_without_memory},
+    {"batch_steps_while_empty", batch_steps_while_empty},
 };
 
 }  // namespace

@@ -66,6 +66,11 @@ def test_batch_goes_on_when_memory_runs_out(cases):
     _run(cases, "batch_without_memory")
 
 
+def test_batch_steps_after_it_was_empty(cases):
+    """A step count first asked for while no domain was there."""
+    _run(cases, "batch_steps_while_empty")
+
+
 def _extract(path, *starts):
     """The definitions of a source file that begin with the given lines."""
     text = open(path).read()
