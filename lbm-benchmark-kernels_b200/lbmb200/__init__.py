@@ -286,7 +286,7 @@ class Instance:
         return out.reshape(-1, Q)
 
     def set_field(self, pdfs):
-        if getattr(pdfs, "shape", None) == (self.lattice.mask.size, Q) and pdfs.strides[0] == 0:
+        if isinstance(pdfs, np.ndarray) and pdfs.shape == (self.lattice.mask.size, Q) and pdfs.strides[0] == 0:
             # one row repeated (np.broadcast_to): no need to write it out
             row = np.ascontiguousarray(pdfs[0], dtype=np.float64)
             lib().lbm_b200_set_uniform(self.kdp, ctypes.byref(self.lattice.desc),

@@ -160,3 +160,41 @@ def test_packing_256_layout_matches_reference_fixture(pull):
     assert (nf, nc) == (lay["n_fluid"], lay["n_cells"])
     assert hashlib.sha256(g.tobytes()).hexdigest() == lay["grid_sha256"]
     assert hashlib.sha256(a.tobytes()).hexdigest() == lay["adj_sha256"]
+
+
+def _field_inputs():
+    import pandas
+    import torch
+    row = np.arange(19.0) / 7
+    full = np.arange(12 * 19.0).reshape(12, 19)
+    rows = np.broadcast_to(row, (12, 19))
+    return {
+        "array": full, "flat": full.reshape(-1), "float32": full.astype(np.float32), "transposed": full.T.copy().T,
+        "nested list": full.tolist(), "tensor": torch.from_numpy(full), "tensor float32": torch.from_numpy(full).float(),
+        "tensor repeated row": torch.from_numpy(row).expand(12, 19), "data frame": pandas.DataFrame(full),
+        "memory view": memoryview(full), "memory view of a repeated row": memoryview(rows), "repeated row": rows,
+        "repeated float32 row": np.broadcast_to(row.astype(np.float32), (12, 19)),
+        "repeated number": np.broadcast_to(np.float64(0.5), (12, 19)),
+    }
+
+
+@pytest.mark.parametrize("name", [
+    "array", "flat", "float32", "transposed", "nested list", "tensor", "tensor float32", "tensor repeated row",
+    "data frame", "memory view", "memory view of a repeated row", "repeated row", "repeated float32 row",
+    "repeated number"])
+def test_set_field_takes_what_numpy_takes(name, monkeypatch):
+    """Instance.set_field hands the library the cells' PDFs, whatever kind of
+    array they come in; a repeated row may go by itself."""
+    import ctypes
+    import types
+    pdfs = _field_inputs()[name]
+    got = []
+
+    def taken(n):
+        return lambda kdp, ld, p: got.append(np.broadcast_to(np.ctypeslib.as_array(p, shape=(n, 19)), (12, 19)).copy())
+
+    fake = types.SimpleNamespace(lbm_b200_set_field=taken(12), lbm_b200_set_uniform=taken(1))
+    monkeypatch.setattr(lbmb200, "lib", lambda: fake)
+    lattice = types.SimpleNamespace(mask=np.ones(12, np.int32), desc=ctypes.c_int(0))
+    lbmb200.Instance(None, lattice, None).set_field(pdfs)
+    assert len(got) == 1 and np.array_equal(got[0], np.ascontiguousarray(pdfs, dtype=np.float64).reshape(12, 19))
