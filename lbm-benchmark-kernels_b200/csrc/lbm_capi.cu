@@ -759,6 +759,7 @@ void pair_upload(Gpu* g, const std::vector<lbm::PairRec<R>>& items, size_t nTile
   LBM_CK(cudaMemsetAsync(g->dPairCount, 0, sizeof(uint32_t) * (g->pairGroups + 2), g->stream));
   LBM_CK(lbm::dev_alloc(&g->dPairItems, sizeof(lbm::PairRec<R>) * items.size()));
   LBM_CK(cudaMemcpyAsync(g->dPairItems, items.data(), sizeof(lbm::PairRec<R>) * items.size(), cudaMemcpyHostToDevice, g->stream));
+  LBM_CK(cudaStreamSynchronize(g->stream));  // the caller's records go
 }
 
 void schedule_list_pairs(Gpu* g) {
@@ -830,6 +831,7 @@ void build_odd_items(Gpu* g, const uint32_t* link) {
     LBM_CK(lbm::dev_alloc(&g->dOddCells, sizeof(int) * cells.size()));
     LBM_CK(cudaMemcpyAsync(g->dOddCells, cells.data(), sizeof(int) * cells.size(), cudaMemcpyHostToDevice, g->stream));
   }
+  LBM_CK(cudaStreamSynchronize(g->stream));  // the vectors go
 }
 
 // --- Init / Deinit ----------------------------------------------------------------
@@ -929,6 +931,7 @@ Gpu* gpu_new(Kind kind, LatticeDesc* ld, Parameters* params, const SlabSpec* sla
     }
     if (!slab) schedule_aa_pairs(g, ld);
     if (kind == kAa) build_odd_items(g, link);
+    LBM_CK(cudaStreamSynchronize(g->stream));  // the link words are up
     std::free(link);
   } else {
     const bool pull = kind == kListPull || kind == kListPullPlain;

@@ -106,6 +106,7 @@ long long list_build_device(const int*, const int dims[3], const int*, int, cons
   fake::launch(s, [=] {
     for (int k = 0; k < n; ++k) grid[k] = (uint32_t)k;
   });
+  cudaStreamSynchronize(s);
   return n;
 }
 int list_runs_device(const uint32_t*, int nFluid, cudaStream_t s, uint32_t** runs, uint32_t** runOff, size_t* runBytes) {
@@ -115,6 +116,19 @@ int list_runs_device(const uint32_t*, int nFluid, cudaStream_t s, uint32_t** run
   const cudaError_t e = dev_alloc(runs, *runBytes);
   if (e != cudaSuccess) return (int)e;
   return (int)dev_alloc(runOff, sizeof(uint32_t) * (tiles + 1));
+}
+int list_resident_tiles(int) { return 0; }
+int list_pair_resident(int) { return 4; }
+double pair_schedule(const uint32_t*, const uint32_t*, int nTiles, int, double, std::vector<PairItem>& items) {
+  items.assign(nTiles + 2, PairItem{});
+  for (size_t k = 0; k < items.size(); ++k) items[k].tile = (uint32_t)k;
+  return 0.0;
+}
+void list_pair_fp64(const ListArgs& a, const PairArgs<3>& p, const Trt<double>&, cudaStream_t s) {
+  fake::launch(s, [=] {
+    for (uint32_t k = 0; k < p.nItems; ++k) check(p.items[k].tile == k, "the fused pair reads its items");
+    a.f[0] += 1.0;
+  });
 }
 void list_tile_reach(const uint32_t*, int nFluid, long long, uint32_t* reach, cudaStream_t s) {
   fake::launch(s, [=] {
@@ -291,12 +305,44 @@ void batch_steps_while_empty() {
   lbm_batch_destroy(b);
 }
 
+// Copies from pageable memory may read it as late as the stream gets to them:
+// what they read has to be there until then.
+void uploads_outlive_the_call(const char* what) {
+  fake::staged = false;
+  const std::string kind = what;
+  Lattice lat(16, 10, 8);
+  Parameters p{};
+  CaseData cd = a_case();
+  KernelData* kd = nullptr;
+  if (kind == "batch") {
+    void* b = lbm_batch_create(1, 1.0, 4);
+    check(lbm_batch_add(b, &lat.ld, 1.2, 0.1875, 1e-5) == 0 && lbm_batch_step(b, 2, 1) == 0 && lbm_batch_sync(b) == 0,
+          "a domain steps");
+    lbm_batch_destroy(b);
+    return;
+  }
+  if (kind == "full") D3Q19CudaAaInit_AaSoA(&lat.ld, &kd, &p);
+  if (kind == "list") D3Q19CudaListAaPvInit_PushSoA(&lat.ld, &kd, &p);
+  if (kind == "slab") kd = lbm_aa_slab_init(&lat.ld, 0, 8, 1, 1, &p);
+  if (kind == "list slab") kd = lbm_aa_list_slab_init(&lat.ld, 0, 8, 1, 1, &p);
+  check(kd != nullptr, "the instance is there");
+  if (kind == "full" || kind == "list") check(lbm_b200_step_device(kd, &cd, 4) == 0, "the steps are accepted");
+  if (kind == "slab") check(lbm_aa_slab_step(kd, &cd, 1, nullptr) == 0, "the step is accepted");
+  fake::run_device(0);
+  lbm_aa_slab_deinit(kd);
+}
+
 const std::map<std::string, std::function<void()>> kCases = {
     {"first_odd_part", [] { first_slab_step(0); }},
     {"first_odd_half", [] { first_slab_step(1); }},
     {"first_even_half", [] { first_slab_step(2); }},
     {"first_slab_step_captured", first_slab_step_captured},
     {"deinit_from_another_device", deinit_from_another_device},
+    {"uploads_full", [] { uploads_outlive_the_call("full"); }},
+    {"uploads_list", [] { uploads_outlive_the_call("list"); }},
+    {"uploads_slab", [] { uploads_outlive_the_call("slab"); }},
+    {"uploads_list_slab", [] { uploads_outlive_the_call("list slab"); }},
+    {"uploads_batch", [] { uploads_outlive_the_call("batch"); }},
     {"batch_results_of_a_lost_state", batch_results_of_a_lost_state},
     {"batch_without_memory", batch_without_memory},
     {"batch_steps_while_empty", batch_steps_while_empty},

@@ -71,6 +71,12 @@ def test_batch_steps_after_it_was_empty(cases):
     _run(cases, "batch_steps_while_empty")
 
 
+@pytest.mark.parametrize("kind", ["full", "list", "slab", "list_slab", "batch"])
+def test_uploads_outlive_the_call(cases, kind):
+    """Init and admission keep the host tables until their copies are done."""
+    _run(cases, "uploads_" + kind)
+
+
 def _extract(path, *starts):
     """The definitions of a source file that begin with the given lines."""
     text = open(path).read()
