@@ -1004,10 +1004,11 @@ Gpu* gpu_new(Kind kind, LatticeDesc* ld, Parameters* params, const SlabSpec* sla
     }
     if (!g->listSlab) schedule_list_pairs(g);
     g->mirrorElems = (size_t)Q * nCells;
-    LBM_CK(lbm::dev_alloc(&g->dF, g->elemBytes * g->mirrorElems));
+    // lbm_b200_device_state gives out their pointers
+    LBM_CK(lbm::dev_alloc_block(&g->dF, g->elemBytes * g->mirrorElems));
     LBM_CK(cudaMemsetAsync(g->dF, 0, g->elemBytes * g->mirrorElems, g->stream));
     if (two_grid(kind)) {
-      LBM_CK(lbm::dev_alloc(&g->dG, sizeof(double) * g->mirrorElems));
+      LBM_CK(lbm::dev_alloc_block(&g->dG, sizeof(double) * g->mirrorElems));
       LBM_CK(cudaMemsetAsync(g->dG, 0, sizeof(double) * g->mirrorElems, g->stream));
     }
     kd->GlobalDims[0] = ld->Dims[0];

@@ -7,7 +7,7 @@
 #include <cstdint>
 #include <mutex>
 #include <unordered_map>
-#include <unordered_set>
+#include <vector>
 
 #include "../../include/lbm_b200.h"
 
@@ -26,7 +26,18 @@ struct HostBlock {
 
 std::mutex g_lock;
 Pool g_pools[kMaxDevices];
-std::unordered_set<void*> g_direct;  // device blocks from cudaMalloc
+struct Block {
+  size_t bytes;
+  int dev;
+  bool keep;  // worth keeping for the next one when it is freed
+};
+std::unordered_map<void*, Block> g_direct;  // device blocks from cudaMalloc
+struct Kept {
+  void* p;
+  size_t bytes;
+  int dev;
+};
+std::vector<Kept> g_kept;  // freed blocks, oldest first
 std::unordered_map<void*, HostBlock> g_host;
 
 // The pool of device `dev`, made on first use; null where it has none.
@@ -59,9 +70,52 @@ Pool* pool_of(int dev) {
   return &p;
 }
 
+// Frees kept blocks of device `dev`, oldest first, until `room` bytes fit beside
+// the others; keeps block p of that size, if there is one.
+void make_room(int dev, size_t room, void* p) {
+  std::vector<void*> out;
+  {
+    std::lock_guard<std::mutex> hold(g_lock);
+    size_t sum = room;
+    for (const Kept& k : g_kept) sum += k.dev == dev ? k.bytes : 0;
+    for (size_t i = 0; i < g_kept.size() && sum > lbm::kBlockKeep;) {
+      if (g_kept[i].dev != dev) {
+        ++i;
+        continue;
+      }
+      sum -= g_kept[i].bytes;
+      out.push_back(g_kept[i].p);
+      g_kept.erase(g_kept.begin() + i);
+    }
+    if (p) g_kept.push_back(Kept{p, room, dev});
+  }
+  for (void* q : out) cudaFree(q);
+}
+
+// Gives back what is kept on device `dev`.
+void release(int dev, Pool* pool) {
+  make_room(dev, lbm::kBlockKeep, nullptr);
+  if (pool) cudaMemPoolTrimTo(pool->pool, 0);
+}
+
 }  // namespace
 
 namespace lbm {
+
+// From cudaMalloc, once more without what is kept if there is no memory.
+static cudaError_t dev_alloc_direct(void** p, size_t bytes, int dev, bool keep) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    release(dev, pool_of(dev));
+    e = cudaMalloc(p, bytes);
+  }
+  if (e == cudaSuccess && *p) {
+    std::lock_guard<std::mutex> hold(g_lock);
+    g_direct[*p] = Block{bytes, dev, keep};
+  }
+  return e;
+}
 
 cudaError_t dev_alloc(void** p, size_t bytes) {
   *p = nullptr;
@@ -73,30 +127,52 @@ cudaError_t dev_alloc(void** p, size_t bytes) {
     e = cudaMallocFromPoolAsync(p, bytes, pool->pool, pool->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(pool->stream);
     if (e == cudaSuccess) return e;
-    // out of memory with freed blocks kept: give those back and try without
+    // out of memory with freed blocks kept: try without the pool
     *p = nullptr;
     cudaGetLastError();
-    cudaMemPoolTrimTo(pool->pool, 0);
   }
-  e = cudaMalloc(p, bytes);
-  if (e == cudaErrorMemoryAllocation && !pool && (pool = pool_of(dev))) {
-    cudaGetLastError();
-    cudaMemPoolTrimTo(pool->pool, 0);
-    e = cudaMalloc(p, bytes);
-  }
-  if (e == cudaSuccess && *p) {
+  return dev_alloc_direct(p, bytes, dev, false);
+}
+
+cudaError_t dev_alloc_block(void** p, size_t bytes) {
+  *p = nullptr;
+  int dev = 0;
+  const cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  {
+    // the tightest of the kept blocks, at most a quarter larger
     std::lock_guard<std::mutex> hold(g_lock);
-    g_direct.insert(*p);
+    size_t best = g_kept.size();
+    for (size_t i = 0; i < g_kept.size(); ++i)
+      if (g_kept[i].dev == dev && g_kept[i].bytes >= bytes && g_kept[i].bytes <= bytes + bytes / 4 &&
+          (best == g_kept.size() || g_kept[i].bytes < g_kept[best].bytes))
+        best = i;
+    if (best < g_kept.size()) {
+      *p = g_kept[best].p;
+      g_direct[*p] = Block{g_kept[best].bytes, dev, true};
+      g_kept.erase(g_kept.begin() + best);
+      return cudaSuccess;
+    }
   }
-  return e;
+  return dev_alloc_direct(p, bytes, dev, bytes <= kBlockKeep);
 }
 
 void dev_free(void* p) {
   if (!p) return;
-  bool direct;
+  Block b{0, 0, false};
+  bool direct = false;
   {
     std::lock_guard<std::mutex> hold(g_lock);
-    direct = g_direct.erase(p) != 0;
+    auto it = g_direct.find(p);
+    if (it != g_direct.end()) {
+      direct = true;
+      b = it->second;
+      g_direct.erase(it);
+    }
+  }
+  if (b.keep) {
+    make_room(b.dev, b.bytes, p);
+    return;
   }
   if (direct) {
     cudaFree(p);
@@ -160,9 +236,8 @@ int lbm_b200_release_memory(void) {
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return (int)e;
   Pool* pool = pool_of(dev);
-  if (!pool) return 0;
-  e = cudaStreamSynchronize(pool->stream);
-  if (e == cudaSuccess) e = cudaMemPoolTrimTo(pool->pool, 0);
+  if (pool) e = cudaStreamSynchronize(pool->stream);
+  if (e == cudaSuccess) release(dev, pool);
   return (int)e;
 }
 

@@ -130,6 +130,9 @@ void list_pair_fp64(const ListArgs& a, const PairArgs<3>& p, const Trt<double>&,
     a.f[0] += 1.0;
   });
 }
+void list_pull_fp64(const ListArgs& a, const Trt<double>&, cudaStream_t s) {
+  fake::launch(s, [=] { a.g[0] = a.f[0] + 1.0; });
+}
 void list_tile_reach(const uint32_t*, int nFluid, long long, uint32_t* reach, cudaStream_t s) {
   fake::launch(s, [=] {
     for (int t = 0; t < (nFluid + kListTile - 1) / kListTile; ++t)
@@ -332,12 +335,82 @@ void uploads_outlive_the_call(const char* what) {
   lbm_aa_slab_deinit(kd);
 }
 
+// The PDF arrays whose pointers the library gives out are blocks of their own:
+// memory of a pool has no IPC handle and is not mapped to peers.
+void state_pointer_is_a_block() {
+  Lattice lat(6, 5, 4);
+  Parameters p{};
+  for (int row = 0; row < 2; ++row) {
+    KernelData* kd = nullptr;
+    if (row == 0) D3Q19CudaListAaPvInit_PushSoA(&lat.ld, &kd, &p);
+    if (row == 1) D3Q19CudaListInit_PullSoA(&lat.ld, &kd, &p);
+    CaseData cd = a_case();
+    for (int k = 0; k < 2; ++k) {  // both grids of the two-grid row
+      double* pdfs = nullptr;
+      check(lbm_b200_device_state(kd, &pdfs, nullptr, nullptr, nullptr) == 0, "the state has a pointer");
+      const auto it = fake::blocks.find(pdfs);
+      check(it != fake::blocks.end() && !it->second.pool, "it is a block from cudaMalloc");
+      check(lbm_b200_step_device(kd, &cd, 1) == 0, "the step is accepted");
+    }
+    D3Q19CudaListAaPvDeinit_PushSoA(&lat.ld, &kd);
+    check(lbm_b200_release_memory() == 0 && fake::blocks.empty(), "the instance's memory is given back");
+  }
+}
+
+// Freed blocks are kept for the next of about their size, up to a bound, per
+// device, and go when memory is short.
+void kept_blocks() {
+  const size_t MB = 1 << 20;
+  auto kept = [] {
+    size_t n = 0;
+    for (const auto& b : fake::blocks) n += b.second.bytes;
+    return n;
+  };
+  void *a, *b, *c;
+  lbm::dev_alloc_block(&a, 8 * MB);
+  lbm::dev_free(a);
+  lbm::dev_alloc_block(&b, 7 * MB);
+  check(b == a, "a block is used again");
+  lbm::dev_free(b);
+  lbm::dev_alloc_block(&b, 6 * MB);
+  check(b != a, "not for a much smaller one");
+  lbm::dev_alloc_block(&c, 9 * MB);
+  check(c != a, "not for a larger one");
+  fake::device = 1;
+  void* d;
+  lbm::dev_alloc_block(&d, 8 * MB);
+  check(d != a, "not on another device");
+  lbm::dev_free(d);
+  lbm::dev_free(c);
+  lbm::dev_free(b);
+  check(lbm_b200_release_memory() == 0 && kept() == 23 * MB, "the current device's are given back");
+  fake::device = 0;
+  check(lbm_b200_release_memory() == 0 && kept() == 0, "and the other's");
+  std::vector<void*> many(30);
+  for (void*& p : many) lbm::dev_alloc_block(&p, 5 * MB);
+  for (void* p : many) lbm::dev_free(p);
+  check(kept() <= 64 * MB && kept() > 50 * MB, "what is kept is bounded");
+  lbm::dev_alloc_block(&a, 65 * MB);
+  lbm::dev_free(a);
+  check(kept() <= 64 * MB, "a larger block is not kept");
+  fake::capacity = 70 * MB;
+  check(lbm::dev_alloc_block(&a, 66 * MB) == cudaSuccess && kept() == 66 * MB, "what is kept makes room");
+  lbm::dev_free(a);
+  lbm::dev_alloc_block(&a, 40 * MB);
+  lbm::dev_free(a);
+  check(lbm::dev_alloc(&b, 60 * MB) == cudaSuccess && kept() == 60 * MB, "for the pool's too");
+  check(lbm::dev_alloc(&c, 60 * MB) == cudaErrorMemoryAllocation && !c, "no memory is an error");
+  lbm::dev_free(b);
+}
+
 const std::map<std::string, std::function<void()>> kCases = {
     {"first_odd_part", [] { first_slab_step(0); }},
     {"first_odd_half", [] { first_slab_step(1); }},
     {"first_even_half", [] { first_slab_step(2); }},
     {"first_slab_step_captured", first_slab_step_captured},
     {"deinit_from_another_device", deinit_from_another_device},
+    {"state_pointer_is_a_block", state_pointer_is_a_block},
+    {"kept_blocks", kept_blocks},
     {"uploads_full", [] { uploads_outlive_the_call("full"); }},
     {"uploads_list", [] { uploads_outlive_the_call("list"); }},
     {"uploads_slab", [] { uploads_outlive_the_call("slab"); }},

@@ -45,6 +45,7 @@ inline int device = 0;
 inline std::set<cudaStream_t> streams;
 inline std::map<void*, Block> blocks;
 inline int failAfter = -1;  // device allocations that succeed before all fail; -1: all succeed
+inline size_t capacity = SIZE_MAX;  // device memory there is
 inline bool failed = false; // one has failed
 inline cudaError_t last = cudaSuccess;
 inline bool staged = true;  // copies from the host read their source at the call; false: when the stream runs
@@ -78,7 +79,9 @@ inline void enqueue(cudaStream_t s, std::function<void()> op) {
 inline cudaError_t allocate(void** p, size_t bytes, bool pool) {
   *p = nullptr;
   ++calls;
-  if (failAfter == 0) {
+  size_t used = 0;
+  for (const auto& b : blocks) used += b.second.bytes;
+  if (failAfter == 0 || (capacity != SIZE_MAX && used + bytes > capacity)) {
     failed = true;
     return last = cudaErrorMemoryAllocation;
   }

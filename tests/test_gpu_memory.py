@@ -60,3 +60,20 @@ def test_instances_from_several_threads():
     for t in threads:
         t.join()
     assert all(np.array_equal(g, want) for g in got)
+
+
+@pytest.mark.parametrize("kname", ["cuda-list-aa-pv-soa", "cuda-list-pull-soa"])
+@pytest.mark.parametrize("edge", [12, 40])
+def test_state_pointers_have_an_ipc_handle(kname, edge):
+    """Other processes may open the PDFs that lbm_b200_device_state points to."""
+    import ctypes
+    rt = pytest.importorskip("cuda.bindings.runtime")
+    inst = lbmb200.kernel(kname).init(lbmb200.geometry("fluid", (edge,) * 3, (1, 1, 1)))
+    try:
+        for _ in range(2):
+            p = ctypes.c_void_p()
+            assert lbmb200.lib().lbm_b200_device_state(inst.kdp, ctypes.byref(p), None, None, None) == 0
+            assert rt.cudaIpcGetMemHandle(p.value)[0] == rt.cudaError_t.cudaSuccess
+            inst.step_device(lbmb200.case(omega=1.2, xforce=0.0, iterations=1), 1)
+    finally:
+        inst.deinit()

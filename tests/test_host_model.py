@@ -77,6 +77,13 @@ def test_uploads_outlive_the_call(cases, kind):
     _run(cases, "uploads_" + kind)
 
 
+def test_state_pointers_are_blocks_of_their_own(cases):
+    """lbm_b200_device_state gives out pointers that cudaIpcGetMemHandle and
+    peer access take."""
+    _run(cases, "state_pointer_is_a_block")
+    _run(cases, "kept_blocks")
+
+
 def _extract(path, *starts):
     """The definitions of a source file that begin with the given lines."""
     text = open(path).read()
