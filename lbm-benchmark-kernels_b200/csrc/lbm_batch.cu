@@ -74,7 +74,7 @@ struct Batch {
   double* dPartials = nullptr;
   int* dDomTileStart = nullptr;
   int* dDomTileCount = nullptr;
-  double* dMoments = nullptr;
+  double* dMoments = nullptr;  // 4 per slot, then the error word
   lbm::BatchLaunch evenL{256, 1, 0}, oddL{256, 1, 0};
   bool separate = false;             // launches of their own for even and odd steps were asked for
   lbm::PairArgs<3> pair{};           // fused pairs (nItems 0: none), as uploaded to dPair
@@ -82,7 +82,7 @@ struct Batch {
   lbm::PairItem* dItems = nullptr;   // capacity itemCap
   uint32_t* dCount = nullptr;        // as many groups as itemCap items can have
   uint32_t itemCap = 0, gridItems = 0;
-  int* errHost = nullptr;            // page-locked copy of the device error word
+  std::vector<double> sums;          // dMoments on the host
   std::map<int, cudaGraphExec_t> graphs;  // steps -> instantiated graph
   long long launches = 0;
   int numSMs = 148;
@@ -266,15 +266,20 @@ int enqueue(Batch* b, int nsteps) {
   return 0;
 }
 
-// Waits for the stream; -7 if a wait inside a step gave up before this (the
-// steps' blocks wait for one another), so that what was copied back on the
-// stream is no state of the update.
-int finish(Batch* b) {
-  BCK(cudaMemcpyAsync(b->errHost, b->dErr, sizeof(int), cudaMemcpyDeviceToHost, b->stream));
-  BCK(cudaStreamSynchronize(b->stream));
-  if (*b->errHost == 0) return 0;
+// -7 if a wait inside a step gave up (the steps' blocks wait for one another):
+// the PDFs, and what was copied from them, are no state of the update.
+int lost_state(int err) {
+  if (err == 0) return 0;
   g_batchError = "a device wait exceeded its limit";
   return -7;
+}
+
+// Waits for what the stream holds; lost_state of the device error word.
+int finish(Batch* b) {
+  int err = 0;
+  BCK(cudaMemcpyAsync(&err, b->dErr, sizeof(int), cudaMemcpyDeviceToHost, b->stream));
+  BCK(cudaStreamSynchronize(b->stream));
+  return lost_state(err);
 }
 
 // Bound on a domain's device bytes: PDFs plus the adjacency (full rows
@@ -427,12 +432,11 @@ void* lbm_batch_create(int storage, double budgetGB, int maxDomains) {
             lbm::dev_alloc(&b->dTileDom, sizeof(int) * b->maxTiles) == cudaSuccess &&
             lbm::dev_alloc(&b->dNTiles, sizeof(int)) == cudaSuccess &&
             lbm::dev_alloc(&b->dErr, sizeof(int)) == cudaSuccess &&
-            cudaMallocHost(reinterpret_cast<void**>(&b->errHost), sizeof(int)) == cudaSuccess &&
             lbm::dev_alloc(&b->dPair, sizeof(lbm::PairArgs<3>)) == cudaSuccess &&
             lbm::dev_alloc(&b->dPartials, sizeof(double) * 4 * (size_t)b->maxTiles) == cudaSuccess &&
             lbm::dev_alloc(&b->dDomTileStart, sizeof(int) * b->maxSlots) == cudaSuccess &&
             lbm::dev_alloc(&b->dDomTileCount, sizeof(int) * b->maxSlots) == cudaSuccess &&
-            lbm::dev_alloc(&b->dMoments, sizeof(double) * 4 * b->maxSlots) == cudaSuccess &&
+            lbm::dev_alloc(&b->dMoments, sizeof(double) * (4 * (size_t)b->maxSlots + 1)) == cudaSuccess &&
             cudaMemsetAsync(b->dErr, 0, sizeof(int), b->stream) == cudaSuccess &&
             cudaMemsetAsync(b->dNTiles, 0, sizeof(int), b->stream) == cudaSuccess;
   if (!ok) {
@@ -458,7 +462,6 @@ void lbm_batch_destroy(void* h) {
   lbm::dev_free(b->dTiles);
   lbm::dev_free(b->dNTiles);
   lbm::dev_free(b->dErr);
-  cudaFreeHost(b->errHost);
   lbm::dev_free(b->dPartials);
   lbm::dev_free(b->dDomTileStart);
   lbm::dev_free(b->dDomTileCount);
@@ -565,8 +568,17 @@ int lbm_batch_moments(void* h, double* out) {
     lbm::batch_moments(a, b->nTiles, b->dPartials, b->dDomTileStart, b->dDomTileCount, b->maxSlots, b->dMoments,
                        b->stream);
   BCK(cudaGetLastError());
-  BCK(cudaMemcpyAsync(out, b->dMoments, sizeof(double) * 4 * b->maxSlots, cudaMemcpyDeviceToHost, b->stream));
-  return finish(b);
+  // the error word in the same copy: one of its own costs 8 us more, and
+  // page-locked memory for it 2 to 5 ms when a batch is made
+  const size_t n = 4 * (size_t)b->maxSlots;
+  b->sums.resize(n + 1);
+  BCK(cudaMemcpyAsync(b->dMoments + n, b->dErr, sizeof(int), cudaMemcpyDeviceToDevice, b->stream));
+  BCK(cudaMemcpyAsync(b->sums.data(), b->dMoments, sizeof(double) * (n + 1), cudaMemcpyDeviceToHost, b->stream));
+  BCK(cudaStreamSynchronize(b->stream));
+  int err;
+  std::memcpy(&err, &b->sums[n], sizeof(int));
+  if (err == 0) std::memcpy(out, b->sums.data(), sizeof(double) * n);
+  return lost_state(err);
 }
 
 // Logical PDFs of a slot (cells x fastest, 19 per cell, obstacles untouched)
