@@ -400,7 +400,8 @@ int lbm_b200_release_memory(void);
 int lbm_b200_set_device(int device);
 
 /* Device state of a list-kernel instance: the current PDF array (list
- * layout, f[d * nCells + n]), its padded cell count and node count, and the
+ * layout, f[d * nCells + n]; a block from cudaMalloc, so that an IPC handle
+ * and peer access apply to it), its padded cell count and node count, and the
  * instance's CUDA stream. Returns -1 for the full-array kernel. */
 int lbm_b200_device_state(KernelData *kd, double **pdfs, long long *nCells, int *nFluid, void **stream);
 

@@ -708,6 +708,15 @@ void cb_kernel(LatticeDesc* ld, KernelData* kd, CaseData* cd) {
 // always take two steps per launch; lists do unless that is the slower way
 // (below), slabs do not (their halo messages travel between the steps).
 //
+// Full arrays have no such rule, because no shape was found where one launch per
+// step is the faster way, not even with rows so long that most tiles find their
+// PDFs gone from L2. us per step, one launch each / one for two, AA, push, pull
+// (share of AA tiles later than 2/5 of L2 allows): 256^3 820 / 592, 860 / 745,
+// 897 / 750 (0.4 %); 40 x 100 x 3000 575 / 448, 584 / 537, 592 / 526 (22 %); 100
+// x 30 x 4000 576 / 521, 583 / 565, 609 / 559 (56 %); 12 x 60 x 20000 694 / 649,
+// 704 / 689, 725 / 697 (96 %); 8000 x 40 x 44 903 / 515, 1104 / 670, 1349 / 785
+// (0 %). Lists gather through the adjacency instead and do lose.
+//
 // Margin (items between an odd step and the last even tile it needs): shorter,
 // and blocks wait; longer, and the PDFs leave L2 before the odd step. Lists,
 // FP64, 256^3 packing, 444 resident blocks: 0.259 ms per step at 355, 0.256 at

@@ -17,7 +17,7 @@ namespace lbm {
 
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-// Grids of fewer than about 4 blocks per SM leave it to the blocks' ends: the
+// Grids of fewer than about 4 blocks per SM (of 148) leave it to the blocks' ends: the
 // successor's blocks, placed beside theirs, would crowd on the SMs that free up
 // first. us per step, plain launches / from the start / at the ends: list pull
 // 172 tiles 6.2 / 5.4 / 4.1, 408 tiles 8.2 / 5.8 / 5.2, 3274 tiles 53.0 / 49.0 /

@@ -155,8 +155,8 @@ void slot_gather(const void* f, const uint32_t* idx, long long n, void* buf, int
 void slot_scatter(void* f, const uint32_t* idx, long long n, const void* buf, int elemBytes, cudaStream_t s);
 
 // Run-compressed adjacency of the nFluid nodes of adj (device, 18 entries
-// per node): allocates *runs (cudaMalloc, *runBytes bytes) and *runOff
-// (nTiles + 1 entries) and fills them; synchronises s. Returns 0 or a CUDA
+// per node): allocates *runs (*runBytes bytes) and *runOff (nTiles + 1 entries)
+// with dev_alloc (lbm_mem.cuh) and fills them; synchronises s. Returns 0 or a CUDA
 // error code.
 int list_runs_device(const uint32_t* adj, int nFluid, cudaStream_t s, uint32_t** runs, uint32_t** runOff,
                      size_t* runBytes);

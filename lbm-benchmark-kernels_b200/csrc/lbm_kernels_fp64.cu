@@ -478,8 +478,8 @@ __device__ __forceinline__ void aa_pair_odd_cell(const AaArgs& a, const Trt<doub
 // fluid (solid cells' slots exist; nothing is stored there): 0.310 against
 // 0.319 ms on that channel, 0.189 / 0.194 at 85 % fluid cells, 0.176 / 0.174
 // at 40 %.
-// Bound by L2 requests and their latency as the list pair: 256^3 fluid box
-// 0.818 -> 0.597 ms per step (28.1 GFLUP/s, half the HBM bytes), 64^3 channel
+// 72 registers spill 52 bytes, more in the open-face function. Bound by L2
+// requests and their latency as the list pair: 256^3 fluid box 0.818 -> 0.597 ms per step (28.1 GFLUP/s, half the HBM bytes), 64^3 channel
 // 0.0220 -> 0.0106, 128 x 112 x 120 blocks, periodic, 0.101 -> 0.064.
 __global__ void __launch_bounds__(kPairThreads, 3)
     k_aa_pair_fp64(const __grid_constant__ AaArgs a, const __grid_constant__ AaPairArgs q,
@@ -1144,9 +1144,9 @@ __device__ __forceinline__ void pair_odd_node(const ListArgs& a, const Trt<doubl
 }
 
 // The fused pair (lbm_pair.cuh). The parameters are read in place
-// (__grid_constant__), which leaves room for both steps under the 72 registers
-// of 3 blocks of 288 threads per SM. What bounds it: L2 and the fabric between
-// its halves (the odd step's gathers and scatters touch 1.2-1.5 sectors per
+// (__grid_constant__), which fits both steps into the 72 registers of 3 blocks of
+// 288 threads per SM but for 16 bytes of spills. What bounds it: L2 and the
+// fabric between its halves (the odd step's gathers and scatters touch 1.2-1.5 sectors per
 // sector of payload; without any waiting the 256^3 packing would take 0.247 ms
 // per step), then the waits.
 __global__ void __launch_bounds__(kPairThreads, 3)
@@ -1253,8 +1253,8 @@ __global__ void __launch_bounds__(kListTile, 3) k_list_push_fp64(const ListArgs 
 // wrote the slots of g it reads and have read the slots of f it writes). The
 // second step finds g in L2: per two steps HBM sees f read and written and g
 // written, 3/4 of two launches' traffic. ms per step, one launch each / one for
-// two: pull 256^3 packing 0.342 / 0.309, 160^3 0.0864 / 0.0768, 96^3 0.0197 /
-// 0.0178; push 0.401 / 0.396, 0.0988 / 0.0935, 0.0230 / 0.0210. Loads ask for
+// two: pull 256^3 packing 0.355 / 0.313, 160^3 0.0939 / 0.0770, 96^3 0.0268 /
+// 0.0210; push 0.407 / 0.377, 0.1034 / 0.0910, 0.0284 / 0.0240. Loads ask for
 // no early eviction: the second step overwrites the lines of f that the first
 // one read, and a push into lines that have left L2 reads them back for the
 // sectors it fills in part (push with streaming loads: 0.433 ms). Both tiles'

@@ -137,7 +137,8 @@ __global__ void __launch_bounds__(kListTile, LBM_LP_ODD_BLOCKS) k_list_odd_lp(co
 }
 
 // The fused pair (lbm_pair.cuh): the arithmetic of the per-node even kernel
-// and of the odd kernel above. 5 blocks of 288 threads per SM (40 registers);
+// and of the odd kernel above. 5 blocks of 288 threads per SM (40 registers,
+// which spill 20 bytes in FP16);
 // 4 blocks measured the same, 3 slower (FP32, 256^3 packing, groups of 8 tiles:
 // 0.165, 0.166 and 0.173 ms per step; groups of 64 0.152, two launches 0.185).
 template <class St>

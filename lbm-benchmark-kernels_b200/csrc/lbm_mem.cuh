@@ -11,7 +11,7 @@
 // ready for any stream when dev_alloc returns; dev_free wants the work on it
 // complete, as seen from the host. Safe from several threads.
 //
-// Host memory: page-locked, zeroed. 2 MiB pages make locking about three times
+// Host memory: page-locked, zeroed, in whole 2 MiB pages. These make locking about three times
 // as fast as cudaMallocHost (40 MB: 5.8 ms against 17 and 2.7 for clearing it;
 // freeing 1.0 against 4.2).
 #pragma once
