@@ -402,8 +402,9 @@ def _batch_domains(n, seed, edge_range=(32, 128), threads=16):
 
 def section_batched(args, dist, peak):
     """512 domains in one batch (FP32), 100-step CUDA graphs, against the same
-    kernel family run one domain at a time. The autotuner's pick is reported; it
-    holds for batches that take a launch per step."""
+    kernel family run one domain at a time. The autotuner chooses between fused
+    pairs and a launch per step; the launch shapes reported are its pick for the
+    latter."""
     import time
 
     import numpy as np

@@ -515,7 +515,8 @@ int lbm_batch_get_field(void *batch, int slot, double *out);
 int lbm_batch_set_field(void *batch, int slot, const double *in);
 /* Launch shape of the even and odd steps where each step is a launch of its
  * own: in batches whose PDFs fit into half of L2, and in every batch from this
- * call on (larger ones otherwise take both steps of a pair in one launch).
+ * call on (larger ones otherwise take both steps of a pair in one launch;
+ * lbm_batch_tune chooses again).
  * which: 0 even, 1 odd, 2 both; threads 64/128/256 (nodes per thread =
  * 256 / threads); blocks = persistent grid size, 0 = one block per tile. */
 int lbm_batch_set_launch(void *batch, int which, int threads, int blocks);
@@ -523,8 +524,9 @@ void lbm_batch_get_launch(void *batch, int *out6);
 int lbm_batch_time_steps(void *batch, int nsteps, double *ms);
 /* Autotuner over block size x nodes per thread x grid (2..6 persistent
  * blocks per SM, or 0 = one block per tile); rows of {which, threads,
- * nodesPerThread, blocks, ms}; keeps the fastest for steps that are launches
- * of their own. */
+ * nodesPerThread, blocks, ms}. Keeps the fastest for steps that are launches of
+ * their own, and from this call on steps the batch in that way or, where it has
+ * the choice, with both steps of a pair in one launch, whichever was faster. */
 int lbm_batch_tune(void *batch, int trialSteps, double *results, int maxRows);
 /* Checkpoint / restart of one resident domain: its PDFs in the batch's
  * storage format plus its lattice size and relaxation parameters. _load

@@ -680,8 +680,9 @@ int lbm_batch_time_steps(void* h, int nsteps, double* ms) {
 // Autotuner: times each (block size, nodes per thread, grid) candidate --
 // grids of 2..6 persistent blocks per SM, or one block per tile -- on the current batch for `trialSteps` steps, separately for the
 // even and the odd kernel (each candidate runs whole even/odd pairs with the
-// other kernel on its current setting), and keeps the fastest. Advances the
-// domains by the trial steps. results (optional): rows of
+// other kernel on its current setting), then fused pairs against the best of
+// these where the batch has them, and keeps the fastest. Advances the domains
+// by the trial steps. results (optional): rows of
 // {which, threads, nodesPerThread, blocks, ms} for every candidate; returns the
 // number of rows written (at most maxRows).
 int lbm_batch_tune(void* h, int trialSteps, double* results, int maxRows) {
@@ -711,6 +712,16 @@ int lbm_batch_tune(void* h, int trialSteps, double* results, int maxRows) {
     if (which == 0) b->evenL = best; else b->oddL = best;
   }
   b->separate = asked;
+  if (b->pair.nItems > 0) {
+    // both steps of a pair in one launch against the best launches apart
+    double apart = 0.0, fusedMs = 0.0;
+    b->separate = true;
+    bool timed = lbm_batch_time_steps(h, trialSteps, &apart) == 0;
+    b->separate = false;
+    timed = timed && lbm_batch_time_steps(h, 2, &fusedMs) == 0;  // warm
+    timed = timed && lbm_batch_time_steps(h, trialSteps, &fusedMs) == 0;
+    b->separate = timed ? apart < fusedMs : asked;
+  }
   drop_graphs(b);
   return std::min(rows, maxRows);
 }

@@ -14,6 +14,7 @@ namespace {
 
 int g_bad = 0;
 int g_steps = 0;             // launches of one step of batches that have run
+double g_pairMs = 1.5;       // what a fused launch takes; a step of its own: 1
 int g_pairs = 0;             // fused launches of batches that have run
 bool g_waitRunsOut = false;  // the next steps set the error word
 void check(bool ok, const char* what) {
@@ -155,6 +156,7 @@ void batch_even_lp(const BatchArgs& a, const BatchLaunch&, int, cudaStream_t s) 
   fake::launch(s, [=] {
     if (g_waitRunsOut) *a.err |= 1;
     g_steps += *a.nTiles > 0;
+    fake::now += 1.0;
     for (int t = 0; t < *a.nTiles; ++t) check(a.tiles[t].nCells == 0, "the step reads its tile records");
   });
 }
@@ -166,6 +168,7 @@ void batch_pair_lp(const BatchPairArgs& a, int grid, cudaStream_t s) {
     for (uint32_t k = 0; k < p.nTiles; ++k) check(a.tiles[k].nCells == 0, "the pair reads its tile records");
     for (uint32_t k = 0; k < ((p.nTiles - 1) >> p.shift) + 3; ++k) check(p.count[k] == 0, "the counters start at zero");
     ++g_pairs;
+    fake::now += g_pairMs;
   });
 }
 void batch_odd_lp(const BatchArgs& a, const BatchLaunch& l, int grid, cudaStream_t s) { batch_even_lp(a, l, grid, s); }
@@ -403,6 +406,40 @@ void kept_blocks() {
   lbm::dev_free(b);
 }
 
+// The tuner leaves the batch on the faster of fused pairs and the best steps
+// apart, whatever a launch shape asked for before it.
+void batch_tune_keeps_the_fastest() {
+  Lattice large(32, 32, 32), small(16, 10, 8);
+  for (double pairMs : {1.5, 2.5, 1.5})
+    for (int shaped = 0; shaped < 2; ++shaped) {
+      g_pairMs = pairMs;
+      void* b = lbm_batch_create(1, 1.0, 4);
+      check(lbm_batch_add(b, &large.ld, 1.2, 0.1875, 1e-5) == 0, "the domain is admitted");
+      if (shaped) check(lbm_batch_set_launch(b, 2, 128, 0) == 0, "a launch shape is taken");
+      for (int graph = 0; graph < 2; ++graph) {
+        g_pairs = g_steps = 0;
+        check(lbm_batch_step(b, 2, graph) == 0 && lbm_batch_sync(b) == 0, "the domain steps");
+        check(shaped ? g_steps == 2 && g_pairs == 0 : g_pairs == 1 && g_steps == 0, "in the shape asked for");
+      }
+      double rows[64 * 5];
+      check(lbm_batch_tune(b, 4, rows, 64) == 36, "every launch shape is timed");
+      for (int graph = 0; graph < 2; ++graph) {
+        g_pairs = g_steps = 0;
+        check(lbm_batch_step(b, 2, graph) == 0 && lbm_batch_sync(b) == 0, "the domain steps");
+        check(pairMs < 2 ? g_pairs == 1 && g_steps == 0 : g_steps == 2 && g_pairs == 0, "in the fastest way");
+      }
+      lbm_batch_destroy(b);
+    }
+  // a batch that has no fused form
+  void* b = lbm_batch_create(1, 1.0, 4);
+  check(lbm_batch_add(b, &small.ld, 1.2, 0.1875, 1e-5) == 0, "the domain is admitted");
+  check(lbm_batch_tune(b, 4, nullptr, 64) == 36, "every launch shape is timed");
+  check(lbm_batch_add(b, &large.ld, 1.2, 0.1875, 1e-5) == 1, "a large one joins");
+  g_pairs = g_steps = 0;
+  check(lbm_batch_step(b, 2, 1) == 0 && lbm_batch_sync(b) == 0 && g_pairs == 1 && g_steps == 0, "it steps fused");
+  lbm_batch_destroy(b);
+}
+
 const std::map<std::string, std::function<void()>> kCases = {
     {"first_odd_part", [] { first_slab_step(0); }},
     {"first_odd_half", [] { first_slab_step(1); }},
@@ -419,6 +456,7 @@ const std::map<std::string, std::function<void()>> kCases = {
     {"batch_results_of_a_lost_state", batch_results_of_a_lost_state},
     {"batch_without_memory", batch_without_memory},
     {"batch_steps_while_empty", batch_steps_while_empty},
+    {"batch_tune_keeps_the_fastest", batch_tune_keeps_the_fastest},
 };
 
 }  // namespace

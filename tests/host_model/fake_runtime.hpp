@@ -27,6 +27,9 @@ struct CUstream_st {
   std::deque<std::function<void()>> q;
   std::vector<std::function<void()>>* capture = nullptr;
 };
+struct CUevent_st {
+  double at = 0.0;
+};
 struct CUgraph_st {
   std::vector<std::function<void()>> ops;
 };
@@ -49,6 +52,7 @@ inline size_t capacity = SIZE_MAX;  // device memory there is
 inline bool failed = false; // one has failed
 inline cudaError_t last = cudaSuccess;
 inline bool staged = true;  // copies from the host read their source at the call; false: when the stream runs
+inline double now = 0.0;    // ms; moved on by what the cases' launches do
 inline int calls = 0;       // copies, clears, waits and allocations so far
 
 inline void run(cudaStream_t s) {
@@ -125,11 +129,24 @@ cudaError_t cudaStreamSynchronize(cudaStream_t s) {
   if (s) fake::run(s);
   return cudaSuccess;
 }
-cudaError_t cudaEventCreate(cudaEvent_t* e) { *e = nullptr; return cudaSuccess; }
-cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
-cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
-cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
-cudaError_t cudaEventElapsedTime(float* ms, cudaEvent_t, cudaEvent_t) { *ms = 1.f; return cudaSuccess; }
+cudaError_t cudaEventCreate(cudaEvent_t* e) { *e = new CUevent_st; return cudaSuccess; }
+cudaError_t cudaEventDestroy(cudaEvent_t e) {
+  for (cudaStream_t s : fake::streams) fake::run(s);
+  delete e;
+  return cudaSuccess;
+}
+cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) {
+  fake::launch(s, [=] { e->at = fake::now; });
+  return cudaSuccess;
+}
+cudaError_t cudaEventSynchronize(cudaEvent_t) {
+  for (cudaStream_t s : fake::streams) fake::run(s);
+  return cudaSuccess;
+}
+cudaError_t cudaEventElapsedTime(float* ms, cudaEvent_t a, cudaEvent_t b) {
+  *ms = (float)(b->at - a->at);
+  return cudaSuccess;
+}
 
 cudaError_t cudaMalloc(void** p, size_t n) { return fake::allocate(p, n, false); }
 cudaError_t cudaFree(void* p) {

@@ -84,6 +84,11 @@ def test_state_pointers_are_blocks_of_their_own(cases):
     _run(cases, "kept_blocks")
 
 
+def test_batch_tune_keeps_the_fastest(cases):
+    """Fused pairs are among what the tuner chooses from."""
+    _run(cases, "batch_tune_keeps_the_fastest")
+
+
 def _extract(path, *starts):
     """The definitions of a source file that begin with the given lines."""
     text = open(path).read()
