@@ -296,7 +296,7 @@ void batch_without_memory() {
 void batch_steps_while_empty() {
   Lattice lat(6, 5, 4);
   void* b = lbm_batch_create(1, 1.0, 4);
-  for (int round = 0; round < 2; ++round) {
+  for (int again = 0; again < 2; ++again) {
     check(lbm_batch_step(b, 2, 1) == 0 && lbm_batch_sync(b) == 0, "an empty batch steps");
     check(lbm_batch_add(b, &lat.ld, 1.2, 0.1875, 1e-5) == 0, "the domain is admitted");
     g_steps = 0;
